@@ -1,0 +1,787 @@
+// pair.cuh -- one particle on two lanes: the horizontal plane (x, px) on the
+// even lane, the vertical one (y, py) on the odd lane.
+//
+// Why.  A sub-partition of this GPU starts one FP64 warp instruction every
+// 64.6 cycles, whatever the active mask and however many independent chains
+// the warp holds (ufo_fp64_probe), so a warp's time is its number of FP64
+// instructions.  With a particle per lane every drift, kick and thick map
+// spends one instruction per plane; with a plane per lane one instruction does
+// both.  A warp then carries 16 particles and half the instructions: a launch
+// with fewer warps than sub-partitions (608) finishes in about half the time,
+// and at full occupancy the work is the same but comes in twice as many,
+// shorter warps, which spread more evenly.  What couples the planes (z = x+iy
+// of a kick, an aperture) goes through a warp shuffle.
+//
+// Results are those of the one-lane interpreter (one_turn) bit for bit (up to
+// the sign of an exact zero): every quantity is formed by the same IEEE
+// operations; a - b*c is evaluated as a + (-b)*c and the like, which only moves
+// signs, and a term that one plane lacks is added there as a zero.  The trimmed
+// expressions of the fast paths hold for finite coordinates, and a coordinate
+// that left the finite range never returns (x += px L keeps inf and NaN).  So
+// the list is cut into segments of 16 ops: a segment in which some particle
+// ends non-finite is run again from its entry state by the one-lane code on the
+// gathered state (`wide`).
+//
+// Latency.  FP64 results reach the next FP64 instruction of a chain in 64.6
+// cycles but any other instruction only after about 115 (measured: one integer
+// operation, shuffle, vote or select per step of a dependent DFMA chain takes
+// the step from 64.7 to 114-115 cycles).  The code therefore keeps selects and
+// sign changes on constants and off the chain, and tests once per segment.
+#pragma once
+
+namespace ufo {
+
+struct Half {
+  double u, pu;  // (x, px) on even lanes, (y, py) on odd lanes
+};
+
+// a lane's state besides its coordinates
+struct PairCtx {
+  double o;       // 1 / (1 + dp)
+  const double *tab;
+  int neg;        // sign bit on even lanes: a - b as a + (b ^ neg)
+  bool even;
+  bool dead;      // no particle, or all four coordinates are NaN (they stay NaN)
+  bool bad_o;     // o is not finite
+};
+
+// what only some ops read, kept out of the registers
+struct PairShared {
+  int64_t p[32];         // particle, -1: none (the lane runs along on zeros)
+  double *obs[32];       // this turn's first observation slot, or null
+  int64_t obs_left[32];  // observation slots left from there
+  int turn[32], target[32];
+  // the lane's state across the out-of-line calls
+  double u[32], pu[32], o[32];
+  const double *tab[32];
+  bool dead[32];
+};
+
+constexpr unsigned PAIR_ALL = 0xffffffffu;
+
+UFO_DEV double pair_other(double v) { return __shfl_xor_sync(PAIR_ALL, v, 1); }
+UFO_DEV double flip(double v, int bit) {
+  return __hiloint2double(__double2hiint(v) ^ bit, __double2loint(v));
+}
+UFO_DEV double pick(bool first, double a, double b) { return first ? a : b; }
+
+// ---- opcode words of this kernel, built on the host (decode_pair)
+//   head  bits 0-7 variant, 8-15 exponent shift of div_shift, PF_* flags
+//   toff  first constant in the table row
+//   a     slices; first field in the coefficient cache (-1: none); observation
+//         index; first op of a segment in the public list
+//   b     normal mask | skew mask << 16; end of the segment
+struct PairOp {
+  int head, toff, a, b;
+};
+enum : int {
+  PF_NEG = 1 << 16,    // div_shift subtracts
+  PF_ACHRO = 1 << 17, PF_SPLITO = 1 << 18,
+  PF_X = 1 << 19, PF_Y = 1 << 20,  // the plane has the term (align, edge)
+  PF_CONST = 1 << 21,
+  PF_DIV = 1 << 23,    // the table holds [A, d, 1/d, A/d] for the inner drift
+  PF_FILL = 1 << 24    // this op fills its cache fields
+};
+enum : int {
+  PV_SEGMENT = 0, PV_DRIFT, PV_DRIFT2, PV_DRIFT_DIV, PV_ALIGN, PV_EDGE, PV_EDGE_PSI, PV_THICKQ,
+  PV_THICKB, PV_CIRCLE, PV_OBSERVE, PV_LINEAR, PV_WIDE,
+  PV_KICK = 16,   // + pattern (0..3, see teapot in ops.cuh)
+  PV_TEAPOT = 20  // + pattern (0..3) + 4 * division form (0..2) + 12 * weak
+};
+constexpr int PAIR_SEGMENT = 16;
+// forms of the inner drift of a teapot: x += px L; x += (px A) / d with one
+// FMA (see div_shift); the same by Markstein's correction (divc)
+enum : int { DIV_NONE = 0, DIV_SHIFT = 1, DIV_GENERAL = 2, DIV_ANY = 3 };
+// cached fields of a thick element, per lane
+enum : int { TC_C = 0, TC_S, TC_K, TC_R, TC_Z, TC_D, TC_DP, TC_FIELDS };
+
+// Correctly rounded a / d for a small integer d with one FMA: q = RN(a r + u),
+// r = RN(1/d), u = +-a 2^-s (the exponent field moved, no FP64 instruction).
+// With r = 1/d - eps ulp(r) the exact quotient is a r + a eps ulp(r).  N/d for
+// an integer N is at least 1/(2 d') ulp away from every rounding boundary (d'
+// the odd part of d: 2N - (2i+1) d' is odd), so any u closer to a eps ulp(r)
+// than that gives the correctly rounded quotient; the host admits the form
+// when a power of two is (d' = 3: eps = 1/3, 1/4 serves; d' = 7: eps = 2/7,
+// 1/4 serves; d' = 5 has none and keeps the general form).  Zeros and
+// subnormal a take u = 0, which is as good there (the quotient is a multiple of
+// 2^-1074 off by far less than 1/(2 d') of it); `bad` collects operands whose
+// exponent the shift would take out of range.
+UFO_DEV double div_shift(double a, double r, int shift_hi, int sign, bool &bad) {
+  const int hi = __double2hiint(a);
+  const unsigned t = (static_cast<unsigned>(hi) & 0x7fffffffu) - 0x00100000u;
+  bad = bad || t < 0x07000000u;
+  const bool tiny = static_cast<int>(t) < 0;
+  const double u = __hiloint2double(tiny ? 0 : (hi - shift_hi) ^ sign,
+                                    tiny ? 0 : __double2loint(a));
+  return fma_(a, r, u);
+}
+
+// divc without its branch: operands outside its range set `bad`
+UFO_DEV double div_markstein(double a, double d, double r, bool &bad) {
+  const int hi = __double2hiint(a);
+  const unsigned e = static_cast<unsigned>(hi) & 0x7ff00000u;
+  const bool zero = ((hi & 0x7fffffff) | __double2loint(a)) == 0;
+  bad = bad || (!zero && e - 0x07700000u > 0x77f00000u - 0x07700000u);
+  const double q0 = mul(a, r);
+  return fma_(fma_(-q0, d, a), r, q0);
+}
+
+// a / order of the strict Horner scheme
+UFO_DEV double div_order_pair(double a, int order, bool &bad) {
+  if (order == 1) return a;
+  if (order == 2) return mul(a, 0.5);
+  if (order == 4) return mul(a, 0.25);
+  const double r = c_rcp_order[order];
+  if (order == 3) return div_shift(a, r, 56 << 20, 0, bad);
+  return div_markstein(a, static_cast<double>(order), r, bad);
+}
+
+// Correctly rounded a / d with r = RN(1/d) and z = RN((1 - d r)/d) prepared:
+// q1 = RN(a r + RN(a z)) is within an ulp of a/d, and Markstein's correction
+// with the exact remainder rounds it correctly.  The caller keeps a and d in
+// the range where nothing under- or overflows.
+UFO_DEV double div_prepared(double a, double d, double r, double z) {
+  const double q1 = fma_(a, r, mul(a, z));
+  return fma_(fma_(-q1, d, a), r, q1);
+}
+
+// ---------------------------------------------------------------- wide ops
+template <bool FMA>
+__device__ __noinline__ P4 wide_op(double x, double px, double y, double py, double z, double dp,
+                                   double o, int turn, const Op *raw, const double *c) {
+  State s{};
+  s.x = x; s.px = px; s.y = y; s.py = py; s.z = z; s.dp = dp; s.o = o;
+  s.opdp = add(1., dp);
+  s.turn = turn;
+  s.bad_o = nf(o);
+  const int4 w0 = __ldg(reinterpret_cast<const int4 *>(raw));
+  const int4 w1 = __ldg(reinterpret_cast<const int4 *>(raw) + 1);
+  apply_op<FMA, true>(s, Op{w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w}, c, [](int) {});
+  return {s.x, s.px, s.y, s.py};
+}
+
+// ---------------------------------------------------------------- kicks
+// One Horner pass of the strict mode (methods.kick, ufo/methods.py:45-76) over
+// a trimmed coefficient list, the pair form of horner_trim: the even lane
+// holds dpx, the odd lane dpy.  Normal: dpx = a, dpy = b; skew: dpx = b,
+// dpy = a.  Returns this lane's kick.
+template <bool SKEW>
+UFO_DEV double pair_horner(double u, double v, const PairCtx &x, uint32_t mask, const double *c,
+                           double o1, bool &bad) {
+  const int m = 31 - __clz(mask);
+  int k = __popc(mask) - 1;
+  const double top = mul(ld(c + k), o1);
+  --k;
+  // lane that carries `a` (the accumulator the coefficients enter)
+  const bool lane_a = SKEW ? !x.even : x.even;
+  if (m == 0) return lane_a ? top : 0.0;
+  double own;
+  for (int order = m; order > 0; --order) {
+    if (order == m) {  // b is an exact zero: na = a x, nb = +-a y
+      own = mul(top, SKEW ? flip(v, x.neg) : u);
+    } else {
+      const double oth = pair_other(own);
+      const double A = pick(lane_a, own, oth), B = pick(lane_a, oth, own);
+      own = add(mul(SKEW ? B : A, u), mul(flip(SKEW ? A : B, x.neg), v));
+    }
+    own = div_order_pair(own, order, bad);
+    if ((mask >> (order - 1)) & 1u) {
+      own = add(lane_a ? mul(ld(c + k), o1) : 0.0, own);
+      --k;
+    }
+  }
+  return own;
+}
+
+// General kick on finite coordinates: the new momentum.  Strict mode: the
+// normal, then the skew list.
+UFO_DEV double pair_kick_strict(const Half &h, const PairCtx &x, double o1, uint32_t masks,
+                                const double *c, bool &bad) {
+  const double v = pair_other(h.u);
+  const uint32_t mn = masks & 0xffffu, ms = masks >> 16;
+  double pu = h.pu;
+  if (mn) pu = add(pu, flip(pair_horner<false>(h.u, v, x, mn, c, o1, bad), x.neg));
+  if (ms) pu = add(pu, flip(pair_horner<true>(h.u, v, x, ms, c + __popc(mn), o1, bad), x.neg));
+  return pu;
+}
+
+// With FMA: one complex Horner pass over the dense series of M terms
+// (kick_pser_ool)
+UFO_DEV double pair_kick_series(const Half &h, const PairCtx &x, double o1, int M,
+                                const double *ps) {
+  const double v = pair_other(h.u);
+  const double *q = ps + (x.even ? 0 : M);
+  double own = ld(q + M - 1);
+  const double vs = flip(v, x.neg);
+#pragma unroll 1
+  for (int n = M - 2; n >= 0; --n) {
+    const double oth = pair_other(own);
+    own = fma_(pick(x.even, own, oth), h.u, fma_(pick(x.even, oth, own), vs, ld(q + n)));
+  }
+  return fma_(flip(o1, x.neg), own, h.pu);
+}
+
+// ---------------------------------------------------------------- teapot
+// one kick; t: the strength (with the plane's sign, pair_strength), or the
+// factor o of a general kick
+template <bool FMA, int PAT>
+UFO_DEV void pair_kick(Half &h, const PairCtx &x, uint32_t masks, const double *ck, double t,
+                       const double *ps, bool &bad) {
+  if (PAT == 0) {
+    h.pu = FMA ? pair_kick_series(h, x, t, pser_len(masks & 0xffffu, masks >> 16), ps)
+               : pair_kick_strict(h, x, t, masks, ck, bad);
+  } else if (PAT == 1) {
+    h.pu = FMA ? fma_(t, h.u, h.pu) : add(h.pu, mul(t, h.u));
+  } else if (PAT == 2) {
+    const double v = pair_other(h.u);
+    if (FMA) {  // px -= t (x^2 - y^2), py += 2t xy
+      const double m = mul(v, pick(x.even, flip(v, x.neg), h.u));  // -y^2 | xy
+      h.pu = fma_(t, fma_(pick(x.even, h.u, 0.0), h.u, m), h.pu);
+    } else {  // a = t x, b = t y; px -= a x - b y; py += a y + b x
+      const double own = mul(t, h.u);  // -a | b
+      const double oth = pair_other(own);
+      const double A = pick(x.even, own, flip(oth, static_cast<int>(0x80000000u)));
+      const double B = pick(x.even, oth, own);
+      h.pu = add(h.pu, add(mul(A, h.u), mul(B, v)));
+    }
+  }
+}
+
+template <bool FMA, int PAT>
+UFO_DEV double pair_strength(const PairCtx &x, double K, double o1) {
+  if (PAT == 0 || PAT == 3) return o1;
+  // constants carry the signs and the factor 1/2 (exact unless K is subnormal,
+  // which the host keeps from this path)
+  if (PAT == 1 || (FMA && !x.even)) return mul(flip(K, x.neg), o1);
+  return mul(mul(flip(K, x.neg), o1), 0.5);
+}
+
+template <bool FMA>
+UFO_DEV void pair_drift(Half &h, double L) {
+  h.u = FMA ? fma_(h.pu, L, h.u) : add(h.u, mul(h.pu, L));
+}
+
+// DIV = DIV_ANY, WEAK = 2: decided at run time (the general kicks, whose code
+// is long and is instantiated once)
+template <bool FMA, int PAT, int DIV, int WEAK>
+UFO_DEV void pair_teapot(Half &h, const PairCtx &x, const PairOp &op, double Lo, const double *c,
+                         bool &bad) {
+  const int N = op.a;
+  const uint32_t masks = static_cast<uint32_t>(op.b);
+  const double o1 = (op.head & PF_ACHRO) ? 1.0 : x.o;
+  const bool table_div = op.head & PF_DIV;
+  const int variant = (op.head & 0xff) - PV_TEAPOT;
+  const int form = DIV == DIV_ANY ? variant / 4 % 3 : DIV;
+  const bool weak = WEAK == 2 ? variant >= 12 : WEAK != 0;
+  const double *ck = c + 1 + (N > 1 ? (table_div ? 4 : 1) : 0);
+  double Li = 0.0, A = 0.0, d = 0.0, r = 0.0;
+  if (N <= 1) {
+    // a single slice has no inner drift
+  } else if (FMA || form == DIV_NONE) {
+    Li = ld(c + (table_div ? 4 : 1));
+  } else {
+    A = ld(c + 1);
+    d = ld(c + 2);
+    r = ld(c + 3);
+  }
+  const int nk = __popc(masks);
+  const double W = weak && x.even ? ld(ck + nk) : 0.0;
+  const double Lx = (op.head & PF_SPLITO) ? ld(ck + nk + (weak ? 1 : 0)) : Lo;
+  const double t = pair_strength<FMA, PAT>(x, PAT == 1 || PAT == 2 ? ld(ck) : 0.0, o1);
+  const double *ps =
+      FMA && PAT == 0 ? ck + nk + (weak ? 1 : 0) + ((op.head & PF_SPLITO) ? 1 : 0) : nullptr;
+  const int shift_hi = ((op.head >> 8) & 0xff) << 20;
+  const int sign = static_cast<int>(static_cast<unsigned>(op.head & PF_NEG) << 15);
+  pair_drift<FMA>(h, Lo);
+  for (int sl = 1;; ++sl) {
+    pair_kick<FMA, PAT>(h, x, masks, ck, t, ps, bad);
+    if (weak) h.pu = FMA ? fma_(-h.u, W, h.pu) : sub(h.pu, mul(h.u, W));
+    if (sl >= N) break;
+    if (FMA || form == DIV_NONE)
+      pair_drift<FMA>(h, Li);
+    else if (form == DIV_SHIFT)
+      h.u = add(h.u, div_shift(mul(h.pu, A), r, shift_hi, sign, bad));
+    else
+      h.u = add(h.u, div_markstein(mul(h.pu, A), d, r, bad));
+  }
+  pair_drift<FMA>(h, Lx);
+}
+
+// ---------------------------------------------------------------- thick
+// A thick map is linear in the plane's coordinates with coefficients that
+// depend on the particle's momentum alone (ufo/methods.py:99-196):
+//   u' = C u + S pu / k2 + D,   pu' = -+S u k2 + C pu + DP.
+// The coefficients are formed in a particle's first turn, by the operations of
+// thick_quad / thick_bend, and kept for the launch in a per-lane cache; the
+// later turns issue 11 to 13 FP64 instructions instead of a square root, a
+// sine, a cosine, two hyperbolic functions and the divisions.  k2 = 0 marks a
+// plane that is a drift (C = 1, S = length, pu unchanged); r = 0 one that
+// takes the one-lane code (k2 out of range, undefined strength).
+struct ThickHalf { double C, S, k, r, z, D, DP; };
+
+UFO_DEV void thick_put(const ThickHalf &t, double *out, int64_t n, bool bend) {
+  out[TC_C * n] = t.C;
+  out[TC_S * n] = t.S;
+  out[TC_K * n] = t.k;
+  out[TC_R * n] = t.r;
+  out[TC_Z * n] = t.z;
+  if (bend) {
+    out[TC_D * n] = t.D;
+    out[TC_DP * n] = t.DP;
+  }
+}
+
+UFO_DEV void thick_recip(ThickHalf &t, double k2) {
+  const unsigned e = static_cast<unsigned>(__double2hiint(k2)) & 0x7ff00000u;
+  if (e - 0x30000000u > 0x20000000u) {  // outside [2^-255, 2^257]: not prepared
+    t.r = 0.0;
+    t.z = 0.0;
+    return;
+  }
+  t.r = dvd(1.0, k2);
+  t.z = mul(fma_(-k2, t.r, 1.0), t.r);
+}
+
+__device__ __noinline__ void thick_quad_half(double o, int flags, const double *c, double *out,
+                                             int64_t n) {
+  const bool even = (threadIdx.x & 1) == 0;
+  const double k = ld(c), Lf = ld(c + 1);
+  const bool foc = even ? k > 0. : !(k > 0.);
+  ThickHalf t;
+  double k2;
+  if (flags & PF_CONST) {
+    k2 = ld(c + 2);
+    t.C = ld(c + (foc ? 3 : 5));
+    t.S = ld(c + (foc ? 4 : 6));
+  } else {
+    k2 = __dsqrt_rn(fabs((flags & PF_ACHRO) ? k : mul(k, o)));
+    const double k2l = mul(Lf, k2);
+    if (foc) {
+      sincos(k2l, &t.S, &t.C);
+    } else {
+      t.C = cosh(k2l);
+      t.S = sinh(k2l);
+    }
+  }
+  t.k = foc ? -k2 : k2;
+  thick_recip(t, k2);
+  thick_put(t, out, n, false);
+}
+
+__device__ __noinline__ void thick_bend_half(double o, double dp, int flags, const double *c,
+                                             double *out, int64_t n) {
+  const bool even = (threadIdx.x & 1) == 0;
+  const bool achro = flags & PF_ACHRO;
+  const double Lf = ld(c + 2);
+  const double curv = achro ? ld(c) : mul(ld(c), o);
+  const double *q = c + (even ? 9 : 3);  // folded constants of this plane
+  double k = (flags & PF_CONST) ? ld(q) : achro ? ld(c + 1) : mul(ld(c + 1), o);
+  if (even && !(flags & PF_CONST))
+    k = add(k, achro ? mul(curv, curv) : dvd(mul(curv, curv), o));
+  ThickHalf t;
+  t.D = t.DP = -0.0;
+  if (k == 0.) {  // a drift: u += Lf pu
+    t.C = 1.0;
+    t.S = Lf;
+    t.k = 0.0;
+    t.r = 1.0;
+    t.z = 0.0;
+    thick_put(t, out, n, true);
+    return;
+  }
+  const bool foc = even ? k > 0. : k < 0.;
+  const double k2 = (flags & PF_CONST) ? ld(q + 1) : __dsqrt_rn(fabs(k));
+  if (flags & PF_CONST) {
+    t.C = ld(q + (foc ? 2 : 4));
+    t.S = ld(q + (foc ? 3 : 5));
+  } else {
+    const double k2l = mul(Lf, k2);
+    if (foc) {
+      sincos(k2l, &t.S, &t.C);
+    } else {
+      t.C = cosh(k2l);
+      t.S = sinh(k2l);
+    }
+  }
+  t.k = foc ? -k2 : k2;
+  thick_recip(t, k2);
+  if (isnan(k)) t.r = 0.0;
+  if (even) {
+    const double ak = (flags & PF_CONST) ? ld(c + 15) : fabs(k);
+    const double dc = mul(dp, curv);
+    t.D = dvd(mul(dc, foc ? sub(1., t.C) : sub(t.C, 1.)), ak);
+    t.DP = dvd(mul(dc, t.S), k2);
+  }
+  thick_put(t, out, n, true);
+}
+
+UFO_DEV double *pair_cache(const TrackArgs &a, int field) {
+  return a.cache + field * a.cache_lanes + static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
+}
+
+// tan(psi) of a fringe-field edge (edge in ops.cuh)
+__device__ __noinline__ double edge_psi_tan(double curv, const double *c) {
+  return tan(sub(ld(c + 2), mul(dvd(mul(mul(2.0, curv), ld(c + 3)), ld(c + 4)), ld(c + 5))));
+}
+
+// sets `bad` when the plane needs the one-lane code
+UFO_DEV void thick_apply(Half &h, const double *t, int64_t n, bool bend, bool &bad) {
+  const double C = t[TC_C * n], S = t[TC_S * n], k = t[TC_K * n], r = t[TC_R * n],
+               z = t[TC_Z * n];
+  const double a = mul(S, h.pu);
+  const int hi = __double2hiint(a);
+  const unsigned e = static_cast<unsigned>(hi) & 0x7ff00000u;
+  const bool zero = ((hi & 0x7fffffff) | __double2loint(a)) == 0;
+  const bool drift = (__double2hiint(k) & 0x7fffffff) == 0;
+  bad = bad || __double2hiint(r) == 0 || (!zero && e - 0x1f000000u > 0x60f00000u - 0x1f000000u);
+  const double q = div_prepared(a, drift ? 1.0 : fabs(k), r, z);
+  double u = add(mul(C, h.u), q);
+  double pu = add(mul(mul(S, h.u), k), mul(C, h.pu));
+  if (bend) {
+    u = add(u, t[TC_D * n]);
+    pu = add(pu, t[TC_DP * n]);
+  }
+  h.pu = pu;  // a drift's k = 0 leaves it unchanged
+  h.u = u;
+}
+
+// ---------------------------------------------------------------- one turn
+UFO_DEV void pair_observe(const Half &h, bool even, const TrackArgs &a, const PairShared &sh,
+                          int k) {
+  const int lane = threadIdx.x;
+  if (k >= sh.obs_left[lane]) return;
+  double *t = sh.obs[lane] + 6 * static_cast<int64_t>(k);
+  t[even ? 0 : 2] = h.u;
+  t[even ? 1 : 3] = h.pu;
+  if (!(a.flags & UFO_TRACK_FIVED)) t[even ? 4 : 5] = a.coords[sh.p[lane] * 6 + (even ? 4 : 5)];
+}
+
+// Out-of-line work takes the lane's state from shared memory and leaves it
+// there: a call with the interpreter's state in registers would have it spilled
+// on the hot path as well (490 bytes at the 128 registers of 16 warps per SM).
+
+// The public ops [first, last) by the one-lane code on the gathered particle
+// state; both lanes of a pair compute it and keep their half.  Called by whole
+// warps.
+template <bool FMA>
+__device__ __noinline__ void pair_wide(const TrackArgs &a, PairShared &sh, int first, int last) {
+  const int lane = threadIdx.x;
+  const bool even = (lane & 1) == 0;
+  const int64_t p = sh.p[lane];
+  Half h{sh.u[lane], sh.pu[lane]};
+  double z = 0.0, dp = 0.0;
+  if (p >= 0) {
+    z = a.coords[p * 6 + 4];
+    dp = a.coords[p * 6 + 5];
+  }
+  for (int i = first; i < last; ++i) {
+    const Op *raw = a.ops + i;
+    if (raw->kind == OP_OBSERVE) {
+      pair_observe(h, even, a, sh, raw->i0);
+      continue;
+    }
+    const double ou = pair_other(h.u), opu = pair_other(h.pu);
+    const P4 r = wide_op<FMA>(even ? h.u : ou, even ? h.pu : opu, even ? ou : h.u,
+                              even ? opu : h.pu, z, dp, sh.o[lane], sh.turn[lane], raw,
+                              sh.tab[lane] + raw->toff);
+    __syncwarp();
+    h = {even ? r.x : r.y, even ? r.px : r.py};
+  }
+  const unsigned nans = __ballot_sync(PAIR_ALL, isnan(h.u) && isnan(h.pu));
+  sh.dead[lane] = p < 0 || ((nans >> (lane & 30)) & 3u) == 3u;
+  sh.u[lane] = h.u;
+  sh.pu[lane] = h.pu;
+}
+
+UFO_DEV PairOp pair_fetch(const int4 *w) {
+  const int4 v = __ldg(w);
+  return {v.x, v.y, v.z, v.w};
+}
+
+// A particle's first turn in a launch: its coefficient-cache fields.
+__device__ __noinline__ void pair_fill(const TrackArgs &a, const PairShared &sh) {
+  const int lane = threadIdx.x;
+  const bool even = (lane & 1) == 0;
+  const double dp = a.coords[sh.p[lane] * 6 + 5], o = sh.o[lane];
+  for (const int4 *w = reinterpret_cast<const int4 *>(a.pair_ops);; ++w) {
+    const PairOp op = pair_fetch(w);
+    const int variant = op.head & 0xff;
+    if (variant == PV_SEGMENT && op.b <= op.a) return;
+    if (!(op.head & PF_FILL)) continue;
+    const double *c = sh.tab[lane] + op.toff;
+    double *t = pair_cache(a, op.a);
+    if (variant == PV_THICKQ) {
+      thick_quad_half(o, op.head, c, t, a.cache_lanes);
+    } else if (variant == PV_THICKB) {
+      thick_bend_half(o, dp, op.head, c, t, a.cache_lanes);
+    } else {  // an edge's factor: tan(e1), or -tan(psi) of the vertical plane
+      const double curv = (op.head & PF_ACHRO) ? ld(c) : mul(ld(c), o);
+      *t = even ? ((op.head & PF_X) ? ld(c + 1) : 0.0) : -edge_psi_tan(curv, c);
+    }
+  }
+}
+
+// What ends a run of the inner loop, which holds no call: the end of the list;
+// a segment to run again; an op without a two-lane form (a segment of its own).
+enum : int { PE_END = 0, PE_REDO = 1, PE_WIDE = 2 };
+
+// Run the list from op `pos`, where a segment's header or its WIDE op stands.
+// PE_REDO leaves the segment's entry state in h and its public ops in [first,
+// last).
+template <bool FMA>
+UFO_DEV int pair_run(Half &h, const PairCtx &x, int &pos, int &first, int &last,
+                     const TrackArgs &a, const PairShared &sh, bool any_bad_o) {
+  const bool even = x.even;
+  const int4 *w = reinterpret_cast<const int4 *>(a.pair_ops) + pos + 1;
+  PairOp op = pair_fetch(w - 1), next = pair_fetch(w);
+  double c0 = ld(x.tab + op.toff);
+  Half in = h;
+  bool bad = false;
+  first = last = 0;
+  for (;;) {
+    // two ops ahead, and the first constant of the next one (the list ends in
+    // two padding ops)
+    const PairOp after = pair_fetch(w + 1);
+    const double next_c0 = ld(x.tab + next.toff);
+    const double *c = x.tab + op.toff;
+    switch (op.head & 0xff) {
+      case PV_SEGMENT: {  // the previous segment's test; the entry state of the next
+        const bool redo = !x.dead && (bad || nf(h.u) || any_bad_o);
+        if (last > first && __any_sync(PAIR_ALL, redo)) {
+          h = in;
+          pos = static_cast<int>(w - 1 - reinterpret_cast<const int4 *>(a.pair_ops));
+          return PE_REDO;
+        }
+        if (op.b <= op.a) return PE_END;
+        first = op.a;
+        last = op.b;
+        in = h;
+        bad = false;
+        break;
+      }
+      case PV_DRIFT:
+        pair_drift<FMA>(h, c0);
+        break;
+      case PV_DRIFT2: {
+        const double t = mul(h.pu, c0);
+        h.u = FMA ? fma_(t, ld(c + 1), h.u) : add(h.u, mul(t, ld(c + 1)));
+        break;
+      }
+      case PV_DRIFT_DIV:
+        h.u = FMA ? fma_(h.pu, ld(c + 3), h.u)
+                  : add(h.u, div_markstein(mul(h.pu, c0), ld(c + 1), ld(c + 2), bad));
+        break;
+      case PV_ALIGN:
+        h.u = sub(h.u, (op.head & (even ? PF_X : PF_Y)) ? ld(c + (even ? 0 : 1)) : 0.0);
+        break;
+      case PV_EDGE: {
+        const double curv = mul(c0, (op.head & PF_ACHRO) ? 1.0 : x.o);
+        const double T = (op.head & (even ? PF_X : PF_Y))
+                             ? flip(ld(c + (even ? 1 : 2)), x.neg ^ static_cast<int>(0x80000000u))
+                             : 0.0;
+        const double t = mul(h.u, curv);
+        h.pu = FMA ? fma_(t, T, h.pu) : add(h.pu, mul(t, T));
+        bad = bad || nf(curv);
+        break;
+      }
+      case PV_EDGE_PSI: {
+        const double curv = (op.head & PF_ACHRO) ? c0 : mul(c0, x.o);
+        const double T = *pair_cache(a, op.a);
+        h.pu = add(h.pu, mul(mul(h.u, curv), T));
+        bad = bad || nf(curv);
+        break;
+      }
+      case PV_THICKQ:
+        thick_apply(h, pair_cache(a, op.a), a.cache_lanes, false, bad);
+        break;
+      case PV_THICKB:
+        thick_apply(h, pair_cache(a, op.a), a.cache_lanes, true, bad);
+        break;
+      case PV_CIRCLE: {
+        const double s = mul(h.u, h.u);
+        const double r2 = add(s, pair_other(s));
+        if (even && !(r2 < c0)) h.u = __longlong_as_double(0x7ff8000000000000ll);
+        break;
+      }
+      case PV_OBSERVE:
+        pair_observe(h, even, a, sh, op.a);
+        break;
+      case PV_LINEAR: {
+        // (x, px) through a 2x2 matrix, (y, py) through a drift: on odd lanes
+        // the matrix [0 ly; 0 1] with y itself as the addend of the first row
+        const double m11 = even ? c0 : 0.0, m12 = ld(c + (even ? 1 : 4));
+        const double m21 = even ? ld(c + 2) : 0.0, m22 = even ? ld(c + 3) : 1.0;
+        const double t2 = mul(m22, h.pu);
+        const double t1 = fma_(m12, h.pu, even ? 0.0 : h.u);
+        h.pu = fma_(m21, h.u, t2);
+        h.u = fma_(m11, h.u, t1);
+        break;
+      }
+      case PV_KICK:
+        pair_kick<FMA, 0>(h, x, static_cast<uint32_t>(op.b), c,
+                          (op.head & PF_ACHRO) ? 1.0 : x.o,
+                          c + __popc(static_cast<uint32_t>(op.b)), bad);
+        break;
+      case PV_KICK + 1:
+        pair_kick<FMA, 1>(h, x, 0, c,
+                          pair_strength<FMA, 1>(x, c0, (op.head & PF_ACHRO) ? 1.0 : x.o), nullptr,
+                          bad);
+        break;
+      case PV_KICK + 2:
+        pair_kick<FMA, 2>(h, x, 0, c,
+                          pair_strength<FMA, 2>(x, c0, (op.head & PF_ACHRO) ? 1.0 : x.o), nullptr,
+                          bad);
+        break;
+      case PV_WIDE:
+        pos = static_cast<int>(w - reinterpret_cast<const int4 *>(a.pair_ops));
+        return PE_WIDE;
+#define UFO_PAIR_TEAPOTS(DIV, WEAK)                                                  \
+  case PV_TEAPOT + 1 + 4 * DIV + 12 * WEAK:                                          \
+    pair_teapot<FMA, 1, FMA ? 0 : DIV, WEAK>(h, x, op, c0, c, bad);                  \
+    break;                                                                           \
+  case PV_TEAPOT + 2 + 4 * DIV + 12 * WEAK:                                          \
+    pair_teapot<FMA, 2, FMA ? 0 : DIV, WEAK>(h, x, op, c0, c, bad);                  \
+    break;                                                                           \
+  case PV_TEAPOT + 3 + 4 * DIV + 12 * WEAK:                                          \
+    pair_teapot<FMA, 3, FMA ? 0 : DIV, WEAK>(h, x, op, c0, c, bad);                  \
+    break;
+      UFO_PAIR_TEAPOTS(0, 0)
+      UFO_PAIR_TEAPOTS(1, 0)
+      UFO_PAIR_TEAPOTS(2, 0)
+      UFO_PAIR_TEAPOTS(0, 1)
+      UFO_PAIR_TEAPOTS(1, 1)
+      UFO_PAIR_TEAPOTS(2, 1)
+#undef UFO_PAIR_TEAPOTS
+      default:  // the general teapots
+        pair_teapot<FMA, 0, FMA ? 0 : DIV_ANY, 2>(h, x, op, c0, c, bad);
+        break;
+    }
+    ++w;
+    op = next;
+    next = after;
+    c0 = next_c0;
+  }
+}
+
+UFO_DEV void pair_store(const Half &h, bool even, int64_t p, int turn, const TrackArgs &a) {
+  if (a.lost && even) a.lost[p] = static_cast<uint32_t>(turn);
+  if (a.final_state) {
+    double *f = a.final_state + p * 6;
+    f[even ? 0 : 2] = h.u;
+    f[even ? 1 : 3] = h.pu;
+    f[even ? 4 : 5] = a.coords[p * 6 + (even ? 4 : 5)];
+  }
+}
+
+UFO_DEV void pair_idle(PairCtx &x, const TrackArgs &a) {
+  x.o = 1.0;
+  x.bad_o = false;
+  x.dead = true;
+  x.tab = a.table;
+}
+
+// The persistent loop of track_kernel with 16 particles per warp: pairs whose
+// particle finished refill from the work counter at turn boundaries.
+template <bool FMA>
+__global__ void __launch_bounds__(32, 16) track_pair_kernel(const __grid_constant__ TrackArgs a) {
+  __shared__ PairShared sh;
+  const int lane = threadIdx.x;
+  const unsigned below = (1u << (lane & 30)) - 1u;  // lanes of the pairs before this one
+  PairCtx x{};
+  x.even = (lane & 1) == 0;
+  x.neg = x.even ? static_cast<int>(0x80000000u) : 0;
+  pair_idle(x, a);
+  sh.p[lane] = -1;
+  Half h{0.0, 0.0};
+  bool idle = true, exhausted = false;
+  bool fresh = false;  // the particle's first turn in this launch: fill the cache
+  while (true) {
+    const unsigned need = __ballot_sync(PAIR_ALL, idle && !exhausted);
+    if (need) {  // both lanes of a pair are in `need` or neither
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(a.queue, static_cast<unsigned long long>(__popc(need) / 2));
+      base = __shfl_sync(PAIR_ALL, base, 0);
+      if (idle && !exhausted) {
+        const int64_t q = static_cast<int64_t>(base) + __popc(need & below) / 2;
+        if (q < a.n) {
+          const double *c = a.coords + q * 6;
+          h.u = c[x.even ? 0 : 2];
+          h.pu = c[x.even ? 1 : 3];
+          const int target = a.pturns ? a.pturns[q] : a.turns;
+          const int64_t sd = a.seed ? static_cast<int64_t>(a.seed[q]) : 0;
+          if (sd < 0 || sd >= a.n_seeds) {  // seed outside the table: not tracked
+            if (a.lost && x.even) a.lost[q] = 0xffffffffu;
+          } else if (target <= 0) {  // nothing to track
+            pair_store(h, x.even, q, 0, a);
+          } else {
+            idle = false;
+            x.o = dvd(1., add(c[5], 1.));  // as load_particle: the same bits
+            x.bad_o = nf(x.o);
+            fresh = true;
+            x.dead = false;
+            x.tab = a.table + sd * a.stride;
+            sh.p[lane] = q;
+            sh.turn[lane] = 0;
+            sh.target[lane] = target;
+          }
+        } else {
+          exhausted = true;
+        }
+      }
+      continue;  // a pair that got a zero-turn particle needs another
+    }
+    if (__all_sync(PAIR_ALL, idle)) break;
+    if (idle) h.u = h.pu = 0.0;  // idle lanes run along on a finite state
+    const int64_t p = sh.p[lane];
+    const int turn = sh.turn[lane];
+    sh.obs_left[lane] = 0;
+    if (a.tracks && !idle && (turn + 1) % a.every == 0) {
+      const int64_t slot = static_cast<int64_t>((turn + 1) / a.every - 1) * a.n_dumps;
+      sh.obs[lane] = a.tracks + (p * a.slots + slot) * 6;
+      sh.obs_left[lane] = a.slots - slot;
+    }
+    const bool any_bad_o = __any_sync(PAIR_ALL, x.bad_o);
+    if (a.cache && __any_sync(PAIR_ALL, fresh)) {
+      sh.o[lane] = x.o;
+      sh.tab[lane] = x.tab;
+      if (fresh) pair_fill(a, sh);
+      __syncwarp();
+      x.o = sh.o[lane];
+      x.tab = sh.tab[lane];
+    }
+    for (int pos = 0, first, last;;) {
+      const int event = pair_run<FMA>(h, x, pos, first, last, a, sh, any_bad_o);
+      if (event == PE_END) break;
+      sh.u[lane] = h.u;
+      sh.pu[lane] = h.pu;
+      sh.o[lane] = x.o;
+      sh.tab[lane] = x.tab;
+      pair_wide<FMA>(a, sh, first, last);
+      h.u = sh.u[lane];
+      h.pu = sh.pu[lane];
+      x.o = sh.o[lane];
+      x.tab = sh.tab[lane];
+      x.dead = sh.dead[lane];
+    }
+    // loss test (is_lost): isnan(x), or |x| > 1, |y| > 1
+    bool out;
+    if (a.mode == UFO_MODE_TRACK)
+      out = x.even && isnan(h.u);
+    else
+      out = fabs(h.u) > 1. || (x.even && isnan(h.u));
+    const bool lost = ((__ballot_sync(PAIR_ALL, out) >> (lane & 30)) & 3u) != 0u;
+    fresh = false;
+    if (!idle) {
+      const int t = sh.turn[lane] + (lost ? 0 : 1);
+      sh.turn[lane] = t;
+      if (lost || t >= sh.target[lane]) {
+        pair_store(h, x.even, sh.p[lane], t, a);
+        sh.p[lane] = -1;
+        idle = true;
+        pair_idle(x, a);
+      }
+    }
+  }
+}
+
+}  // namespace ufo

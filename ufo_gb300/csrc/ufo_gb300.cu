@@ -15,12 +15,16 @@
 // lane granularity instead of work-item granularity.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
+#include <climits>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/ufo_gb300.h"
@@ -71,6 +75,11 @@ struct TrackArgs {
   // neighbours (which tend to survive or be lost together) while the chunks of
   // a region that survives are spread over every SM
   unsigned long long spread;
+  // two-lane kernel (pair.cuh): its opcode list, and the cache
+  // of momentum-dependent coefficients, [field][cache_lanes] (null: none)
+  const struct PairOp *pair_ops;
+  double *cache;
+  int64_t cache_lanes;
 };
 
 UFO_DEV void load_particle(State &s, const TrackArgs &a, int64_t p) {
@@ -105,110 +114,115 @@ UFO_DEV void observe(const State &s, const TrackArgs &a, int64_t p, int k) {
   if (!(a.flags & UFO_TRACK_FIVED)) { t[4] = s.z; t[5] = s.dp; }
 }
 
-// one pass through the line
+// one op on one particle; `see` is called with an observation point's index
 // FULL = false: the lean interpreter for programs made only of drifts, teapot
 // elements, kicks, alignments, constant edges, circular apertures and
 // observation points (chosen on the host); it carries far fewer live values.
+template <bool FMA, bool FULL, class Observe>
+UFO_DEV void apply_op(State &s, const Op &op, const double *c, Observe see) {
+  switch (op.kind) {
+    case OP_TEAPOT:
+      teapot<FMA, FULL>(s, op, c);
+      break;
+    case OP_DRIFT:
+      if (FULL && (op.flags & F_EXACT))
+        drift<FMA>(s, DF_MUL, true, c);
+      else if (op.i0 == DF_MUL)
+        drift_L<FMA>(s, ld(c));
+      else if (op.i0 == DF_DIV)
+        drift_div<FMA>(s, c);
+      else
+        drift<FMA>(s, DF_MUL2, false, c);
+      break;
+    case OP_KICK: {
+      const bool bad = s.bad_o || nf(s.x) || nf(s.y);
+      if (FMA && !bad && (op.flags & F_PSER)) {  // dense series after the coefficients
+        const uint32_t mn = static_cast<uint32_t>(op.i2), ms = static_cast<uint32_t>(op.i3);
+        const PxPy r = kick_pser_ool(s.x, s.y, s.px, s.py, (op.flags & F_ACHRO) ? 1.0 : s.o,
+                                     pser_len(mn, ms), c + __popc(mn) + __popc(ms));
+        s.px = r.px;
+        s.py = r.py;
+        break;
+      }
+      const PxPy r = kick_ool<FMA>(s.x, s.y, s.px, s.py, s.o, s.bad_o, op.i0, op.i1,
+                                   static_cast<uint32_t>(op.i2), static_cast<uint32_t>(op.i3),
+                                   c, op.flags & F_ACHRO, bad);
+      s.px = r.px;
+      s.py = r.py;
+      break;
+    }
+    case OP_ALIGN:
+      switch ((op.flags & F_AX ? 1 : 0) | (op.flags & F_AY ? 2 : 0)) {
+        case 1: s.x = sub(s.x, ld(c)); break;
+        case 2: s.y = sub(s.y, ld(c + 1)); break;
+        case 3: s.x = sub(s.x, ld(c)); s.y = sub(s.y, ld(c + 1)); break;
+        default: break;
+      }
+      break;
+    case OP_EDGE:
+      edge_dispatch<FMA, FULL>(s, op.flags, c);
+      break;
+    case OP_THICKQ:
+      if (FULL) {
+        const P4 r = thick_quad_ool(s.x, s.px, s.y, s.py, s.o, op.flags, c);
+        s.x = r.x; s.px = r.px; s.y = r.y; s.py = r.py;
+      }
+      break;
+    case OP_THICKB:
+      if (FULL) {
+        const P4 r = thick_bend_ool(s.x, s.px, s.y, s.py, s.dp, s.o, op.flags, c);
+        s.x = r.x; s.px = r.px; s.y = r.y; s.py = r.py;
+      }
+      break;
+    case OP_WIRE:
+      if (FULL) {
+        const P4 r = wire_ool(s.x, s.px, s.y, s.py, c);
+        s.x = r.x; s.px = r.px; s.y = r.y; s.py = r.py;
+      }
+      break;
+    case OP_APERTURE: {
+      bool lost;
+      if (!FULL || (op.flags & F_CIRCLE))  // (x*x + y*y < c) == 0
+        lost = !(add(mul(s.x, s.x), mul(s.y, s.y)) < ld(c));
+      else
+        lost = aperture_ool(s.x, s.px, s.y, s.py, s.z, s.dp, s.o, s.turn, c, op.i0);
+      if (lost) s.x = __longlong_as_double(0x7ff8000000000000ll);
+      break;
+    }
+    case OP_OBSERVE:
+      see(op.i0);
+      break;
+    case OP_LINEAR: {
+      // a kick-free teapot element of an FMA program composed on the host:
+      // (x, px) through a 2x2 matrix, (y, py) through a drift
+      const double m11 = ld(c), m12 = ld(c + 1), m21 = ld(c + 2), m22 = ld(c + 3);
+      const double x0 = s.x;
+      s.x = fma_(m11, x0, mul(m12, s.px));
+      s.px = fma_(m21, x0, mul(m22, s.px));
+      s.y = fma_(s.py, ld(c + 4), s.y);
+      break;
+    }
+    case OP_DYNKICK:
+      if (FULL) {
+        const PxPy r = dynkick_ool(s.x, s.px, s.y, s.py, s.z, s.dp, s.o, s.turn, op.i0, op.i1,
+                                   op.flags & F_ACHRO, op.i2, c);
+        s.px = r.px;
+        s.py = r.py;
+      }
+      break;
+    default:
+      break;
+  }
+}
+
+// one pass through the line
 template <bool FMA, bool FULL>
 UFO_DEV void one_turn(State &s, const TrackArgs &a, const double *tab, int64_t p) {
   for (int i = 0; i < a.n_ops; ++i) {
     const int4 w0 = __ldg(reinterpret_cast<const int4 *>(a.ops + i));
     const int4 w1 = __ldg(reinterpret_cast<const int4 *>(a.ops + i) + 1);
     const Op op{w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-    const double *c = tab + op.toff;
-    switch (op.kind) {
-      case OP_TEAPOT:
-        teapot<FMA, FULL>(s, op, c);
-        break;
-      case OP_DRIFT:
-        if (FULL && (op.flags & F_EXACT))
-          drift<FMA>(s, DF_MUL, true, c);
-        else if (op.i0 == DF_MUL)
-          drift_L<FMA>(s, ld(c));
-        else if (op.i0 == DF_DIV)
-          drift_div<FMA>(s, c);
-        else
-          drift<FMA>(s, DF_MUL2, false, c);
-        break;
-      case OP_KICK: {
-        const bool bad = s.bad_o || nf(s.x) || nf(s.y);
-        if (FMA && !bad && (op.flags & F_PSER)) {  // dense series after the coefficients
-          const uint32_t mn = static_cast<uint32_t>(op.i2), ms = static_cast<uint32_t>(op.i3);
-          const PxPy r = kick_pser_ool(s.x, s.y, s.px, s.py, (op.flags & F_ACHRO) ? 1.0 : s.o,
-                                       pser_len(mn, ms), c + __popc(mn) + __popc(ms));
-          s.px = r.px;
-          s.py = r.py;
-          break;
-        }
-        const PxPy r = kick_ool<FMA>(s.x, s.y, s.px, s.py, s.o, s.bad_o, op.i0, op.i1,
-                                     static_cast<uint32_t>(op.i2), static_cast<uint32_t>(op.i3),
-                                     c, op.flags & F_ACHRO, bad);
-        s.px = r.px;
-        s.py = r.py;
-        break;
-      }
-      case OP_ALIGN:
-        switch ((op.flags & F_AX ? 1 : 0) | (op.flags & F_AY ? 2 : 0)) {
-          case 1: s.x = sub(s.x, ld(c)); break;
-          case 2: s.y = sub(s.y, ld(c + 1)); break;
-          case 3: s.x = sub(s.x, ld(c)); s.y = sub(s.y, ld(c + 1)); break;
-          default: break;
-        }
-        break;
-      case OP_EDGE:
-        edge_dispatch<FMA, FULL>(s, op.flags, c);
-        break;
-      case OP_THICKQ:
-        if (FULL) {
-          const P4 r = thick_quad_ool(s.x, s.px, s.y, s.py, s.o, op.flags, c);
-          s.x = r.x; s.px = r.px; s.y = r.y; s.py = r.py;
-        }
-        break;
-      case OP_THICKB:
-        if (FULL) {
-          const P4 r = thick_bend_ool(s.x, s.px, s.y, s.py, s.dp, s.o, op.flags, c);
-          s.x = r.x; s.px = r.px; s.y = r.y; s.py = r.py;
-        }
-        break;
-      case OP_WIRE:
-        if (FULL) {
-          const P4 r = wire_ool(s.x, s.px, s.y, s.py, c);
-          s.x = r.x; s.px = r.px; s.y = r.y; s.py = r.py;
-        }
-        break;
-      case OP_APERTURE: {
-        bool lost;
-        if (!FULL || (op.flags & F_CIRCLE))  // (x*x + y*y < c) == 0
-          lost = !(add(mul(s.x, s.x), mul(s.y, s.y)) < ld(c));
-        else
-          lost = aperture_ool(s.x, s.px, s.y, s.py, s.z, s.dp, s.o, s.turn, c, op.i0);
-        if (lost) s.x = __longlong_as_double(0x7ff8000000000000ll);
-        break;
-      }
-      case OP_OBSERVE:
-        observe(s, a, p, op.i0);
-        break;
-      case OP_LINEAR: {
-        // a kick-free teapot element of an FMA program composed on the host:
-        // (x, px) through a 2x2 matrix, (y, py) through a drift
-        const double m11 = ld(c), m12 = ld(c + 1), m21 = ld(c + 2), m22 = ld(c + 3);
-        const double x0 = s.x;
-        s.x = fma_(m11, x0, mul(m12, s.px));
-        s.px = fma_(m21, x0, mul(m22, s.px));
-        s.y = fma_(s.py, ld(c + 4), s.y);
-        break;
-      }
-      case OP_DYNKICK:
-        if (FULL) {
-          const PxPy r = dynkick_ool(s.x, s.px, s.y, s.py, s.z, s.dp, s.o, s.turn, op.i0, op.i1,
-                                     op.flags & F_ACHRO, op.i2, c);
-          s.px = r.px;
-          s.py = r.py;
-        }
-        break;
-      default:
-        break;
-    }
+    apply_op<FMA, FULL>(s, op, tab + op.toff, [&](int k) { observe(s, a, p, k); });
   }
 }
 
@@ -268,6 +282,10 @@ __global__ void __launch_bounds__(32) track_kernel(TrackArgs a) {
     }
   }
 }
+
+}  // namespace ufo
+#include "pair.cuh"
+namespace ufo {
 
 // ------------------------------------------------- CTA-compacting variant
 // The same persistent loop with many warps per CTA, and one more step once
@@ -739,6 +757,14 @@ struct ufo_prog {
   int n_dumps;
   bool full;  // needs the full interpreter (thick, wire, exact, ...)
   std::vector<int32_t> host_ops;  // for validating replacement tables
+  // two-lane kernel (pair.cuh): null when a op has no two-lane form
+  ufo::PairOp *pair_ops;
+  std::vector<ufo::PairOp> host_pair_ops;
+  bool pair_fma;               // also for FMA launches
+  int cache_fields;            // doubles per lane of the coefficient cache
+  mutable double *cache;       // [cache_fields][cache_lanes]
+  mutable int64_t cache_lanes;
+  mutable bool captured;       // a graph may hold the cache: its layout stays
 };
 
 namespace {
@@ -949,6 +975,194 @@ int validate_ops(const int32_t *ops, int n_ops, int64_t stride, int n_dumps,
   return UFO_OK;
 }
 
+// ------------------------------------------------ two-lane opcode list
+// The exponent shift of div_shift for the divisor d (RN(1/d) = r in the
+// table), or 0 when no power of two serves: with eps = (1/d - r) / ulp(r) and M
+// the significand of 1/d, the candidate k = +-2^-j must satisfy |k - eps| <
+// 1/(2 d') over operand significands up to 2/M (quotients below the next power
+// of two) and up to 2 halved (above it); 0.95 leaves room for the terms of
+// order 2^-53 that the bound drops.
+int shift_form(double d, double r, bool &negative) {
+  if (!(d > 1.0 && d < 1048576.0) || d != std::floor(d) || r != 1.0 / d) return 0;
+  long odd = static_cast<long>(d);
+  while (odd % 2 == 0) odd /= 2;
+  if (odd == 1) return 0;
+  int ez = 0;
+  const double m = 2.0 * std::frexp(r, &ez);  // r = m 2^(ez-1), m in [1, 2)
+  --ez;
+  const double eps = std::ldexp(std::fma(-d, r, 1.0) / d, 52 - ez);
+  negative = eps < 0.0;
+  const double bound = 0.95 / (2.0 * static_cast<double>(odd));
+  for (int j = 1; j <= 8; ++j) {
+    const double k = std::ldexp(negative ? -1.0 : 1.0, -j);
+    const double off = std::fabs(k - eps);
+    if (off * (2.0 / m) < bound && off < bound) return 52 + j - ez;
+  }
+  return 0;
+}
+
+// kick pattern of the interpreters (teapot in ops.cuh)
+int kick_pattern(int nn, int ns, int32_t mn) {
+  return ns != 0 ? 0 : (nn == 2 && mn == 2) ? 1 : (nn == 3 && mn == 4) ? 2 : mn == 0 ? 3 : 0;
+}
+
+// Translate a validated opcode list for the two-lane kernel; false when an op
+// has no two-lane form worth its name (Yoshida and exact-drift elements, which
+// would run as one-lane code on half-empty warps).  Structurally empty ops
+// (zero-angle edges) are left out: they matter to non-finite coordinates alone.
+// Thick elements and fringe edges with the same constants in every row share
+// their cache fields; at most `most_fields` are given out, and further elements
+// compute in every turn.  `fma_ready`: the general kicks carry the dense series
+// that the FMA kernel reads.
+bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t stride, int n_seeds,
+                 int most_fields, std::vector<ufo::PairOp> &out, int &cache_fields,
+                 bool &fma_ready) {
+  out.clear();
+  out.reserve(static_cast<size_t>(n_ops) + n_ops / ufo::PAIR_SEGMENT + 4);
+  cache_fields = 0;
+  fma_ready = true;
+  struct Shared { int op, field; };
+  std::unordered_multimap<uint64_t, Shared> seen;  // constants' hash -> first op
+  size_t head = 0;  // the current segment's header
+  auto open = [&](int first) {
+    head = out.size();
+    out.push_back({ufo::PV_SEGMENT, 0, first, first});
+  };
+  // the half and negative strengths formed on constants must be exact
+  auto plain_strength = [&](int at) {
+    for (int r = 0; r < n_seeds; ++r) {
+      const double k = std::fabs(table[r * stride + at]);
+      if (!(k == 0.0 || (k > 1e-280 && k < 1e280))) return false;
+    }
+    return true;
+  };
+  open(0);
+  for (int i = 0; i < n_ops; ++i) {
+    const int32_t *w = ops + static_cast<size_t>(i) * UFO_OP_WORDS;
+    const int flags = w[1];
+    const int common = (flags & ufo::F_ACHRO) ? ufo::PF_ACHRO : 0;
+    ufo::PairOp op{ufo::PV_WIDE, w[2], i, 0};
+    int fields = 0;
+    bool keep = true;
+    switch (w[0]) {
+      case ufo::OP_NOP: keep = false; break;
+      case ufo::OP_DRIFT:
+        if (flags & ufo::F_EXACT) return false;
+        op.head = w[3] == ufo::DF_MUL ? ufo::PV_DRIFT
+                  : w[3] == ufo::DF_MUL2 ? ufo::PV_DRIFT2 : ufo::PV_DRIFT_DIV;
+        break;
+      case ufo::OP_KICK:
+      case ufo::OP_TEAPOT: {
+        const bool teapot = w[0] == ufo::OP_TEAPOT;
+        const int32_t *k = w + (teapot ? 4 : 3);  // nn, ns, mn, ms
+        const int pattern = (k[2] | k[3]) ? kick_pattern(k[0], k[1], k[2]) : 3;
+        if (pattern == 0 && !(flags & ufo::F_PSER)) fma_ready = false;
+        if (teapot && (flags & (ufo::F_EXACT | ufo::F_YOSHIDA))) return false;
+        if (teapot && (((flags >> ufo::SH_FOUTER) & 3) != ufo::DF_MUL ||
+                       ((flags >> ufo::SH_FINNER) & 3) == ufo::DF_MUL2))
+          return false;
+        if ((k[2] >> 16) || (k[3] >> 16)) break;  // orders above 15
+        const bool div = teapot && w[3] > 1 && ((flags >> ufo::SH_FINNER) & 3) == ufo::DF_DIV;
+        if ((pattern == 1 || pattern == 2) &&
+            !plain_strength(w[2] + (!teapot ? 0 : w[3] <= 1 ? 1 : div ? 5 : 2)))
+          break;
+        op.a = teapot ? w[3] : i;
+        op.b = k[2] | k[3] << 16;
+        if (!teapot) {
+          if (pattern == 3) keep = false;
+          op.head = (ufo::PV_KICK + pattern) | common;
+          break;
+        }
+        int form = ufo::DIV_NONE, shift = 0;
+        bool negative = false;
+        if (div) {
+          form = ufo::DIV_GENERAL;
+          const double *q = table + w[2] + 1;  // [A, d, 1/d, A/d]
+          shift = shift_form(q[1], q[2], negative);
+          for (int r = 1; r < n_seeds && shift; ++r)
+            if (q[r * stride + 1] != q[1] || q[r * stride + 2] != q[2]) shift = 0;
+          if (shift) form = ufo::DIV_SHIFT;
+        }
+        op.head = (ufo::PV_TEAPOT + pattern + 4 * form + ((flags & ufo::F_WEAK) ? 12 : 0)) |
+                  shift << 8 | (shift && negative ? ufo::PF_NEG : 0) | (div ? ufo::PF_DIV : 0) |
+                  ((flags & ufo::F_SPLITO) ? ufo::PF_SPLITO : 0) | common;
+        break;
+      }
+      case ufo::OP_ALIGN:
+        op.head = ufo::PV_ALIGN | ((flags & ufo::F_AX) ? ufo::PF_X : 0) |
+                  ((flags & ufo::F_AY) ? ufo::PF_Y : 0);
+        break;
+      case ufo::OP_EDGE:
+        keep = flags & (ufo::F_T1 | ufo::F_T2 | ufo::F_RTPSI);
+        op.head = ((flags & ufo::F_RTPSI) ? ufo::PV_EDGE_PSI : ufo::PV_EDGE) | common |
+                  ((flags & ufo::F_T1) ? ufo::PF_X : 0) | ((flags & ufo::F_T2) ? ufo::PF_Y : 0);
+        if (flags & ufo::F_RTPSI) {
+          if (!(flags & ufo::F_T2)) return false;
+          fields = 1;
+        }
+        break;
+      case ufo::OP_THICKQ:
+      case ufo::OP_THICKB:
+        op.head = (w[0] == ufo::OP_THICKQ ? ufo::PV_THICKQ : ufo::PV_THICKB) | common |
+                  ((flags & ufo::F_CONST) ? ufo::PF_CONST : 0);
+        fields = w[0] == ufo::OP_THICKQ ? ufo::TC_D : ufo::TC_FIELDS;
+        break;
+      case ufo::OP_APERTURE:
+        if (flags & ufo::F_CIRCLE) op.head = ufo::PV_CIRCLE;
+        break;
+      case ufo::OP_OBSERVE:
+        op.head = ufo::PV_OBSERVE;
+        op.a = w[3];
+        break;
+      case ufo::OP_LINEAR: op.head = ufo::PV_LINEAR; break;
+      default: break;  // wires, dynamic kicks: the one-lane code
+    }
+    if (fields) {
+      const int64_t nc = op_consts(w);
+      auto row = [&](int which, int r) {
+        return table + r * stride + ops[static_cast<size_t>(which) * UFO_OP_WORDS + 2];
+      };
+      uint64_t h = 1469598103934665603ull ^ static_cast<uint64_t>(w[0] * 31 + flags);
+      for (int r = 0; r < n_seeds; ++r)
+        for (int64_t k = 0; k < nc; ++k) {
+          uint64_t bits;
+          std::memcpy(&bits, row(i, r) + k, sizeof bits);
+          h = (h ^ bits) * 1099511628211ull;
+          h ^= h >> 29;
+        }
+      int field = -1;
+      const auto range = seen.equal_range(h);
+      for (auto it = range.first; it != range.second && field < 0; ++it) {
+        const int32_t *v = ops + static_cast<size_t>(it->second.op) * UFO_OP_WORDS;
+        bool same = v[0] == w[0] && v[1] == flags;
+        for (int r = 0; r < n_seeds && same; ++r)
+          same = std::memcmp(row(it->second.op, r), row(i, r), sizeof(double) * nc) == 0;
+        if (same) field = it->second.field;
+      }
+      op.a = field;
+      if (field < 0 && fields <= most_fields - cache_fields) {
+        op.a = cache_fields;
+        op.head |= ufo::PF_FILL;
+        seen.emplace(h, Shared{i, cache_fields});
+        cache_fields += fields;
+      }
+    }
+    if (keep) {
+      // an op without a two-lane form is a segment of its own
+      const bool wide = op.head == ufo::PV_WIDE;
+      const int kept = static_cast<int>(out.size() - 1 - head);
+      if (kept > 0 && (wide || out.back().head == ufo::PV_WIDE || kept == ufo::PAIR_SEGMENT))
+        open(i);
+      out.push_back(op);
+    }
+    out[head].b = i + 1;
+  }
+  if (out[head].b > out[head].a) open(n_ops);  // the end
+  out.push_back({ufo::PV_SEGMENT, 0, 0, 0});   // the kernel fetches two ops ahead
+  out.push_back({ufo::PV_SEGMENT, 0, 0, 0});
+  return true;
+}
+
 // Chunk hand-out order of the compacting kernel: c -> (c * m) mod n_chunks
 // with m coprime to the number of whole 32-particle chunks, near it / golden
 // ratio: a permutation whose early values sample the whole input evenly (a
@@ -974,9 +1188,18 @@ unsigned long long spread_multiplier(int64_t n_particles) {
   return m;
 }
 
+// Warps of the two-lane kernel: 16 particles each; the tuning counts warps of
+// the one-lane kernel, so twice as many, at most the 16 per SM that the
+// registers allow.
+int64_t pair_warps(int64_t n, int sm_count, int warps_per_sm) {
+  const int64_t warps = (n + 15) / 16;
+  const int64_t resident = static_cast<int64_t>(sm_count) * std::min(16, 2 * warps_per_sm);
+  return std::min(warps, resident);
+}
+
 // The launch shared by every entry point: fill the kernel arguments and start
 // the persistent (or plain) kernel on `stream`; `queue` is the work counter.
-int launch_kernels(ufo::TrackArgs &a, bool full, int sm_count, int warps_per_sm,
+int launch_kernels(ufo::TrackArgs &a, bool full, bool pair, int sm_count, int warps_per_sm,
                    cudaStream_t stream) {
   const bool fma = a.flags & UFO_TRACK_FMA;
   if (a.flags & UFO_TRACK_PLAIN) {
@@ -1012,6 +1235,13 @@ int launch_kernels(ufo::TrackArgs &a, bool full, int sm_count, int warps_per_sm,
     else
       full ? ufo::track_kernel_cta<false, true><<<g, tpb, smem, stream>>>(a)
            : ufo::track_kernel_cta<false, false><<<g, tpb, smem, stream>>>(a);
+  } else if (pair) {
+    UFO_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), stream));
+    const unsigned g = static_cast<unsigned>(pair_warps(a.n, sm_count, warps_per_sm));
+    if (fma)
+      ufo::track_pair_kernel<true><<<g, 32, 0, stream>>>(a);
+    else
+      ufo::track_pair_kernel<false><<<g, 32, 0, stream>>>(a);
   } else {
     UFO_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), stream));
     // one warp per block so the block scheduler spreads warps evenly over the
@@ -1060,7 +1290,67 @@ ufo::TrackArgs make_args(const ufo::Op *ops, int n_ops, const double *table, int
   a.pool_seq = nullptr;
   a.pool_cap = 0;
   a.spread = 0;
+  a.pair_ops = nullptr;
+  a.cache = nullptr;
+  a.cache_lanes = 0;
   return a;
+}
+
+// Which launches take the two-lane kernel (measured on one GB300, us per turn,
+// one-lane kernel -> two-lane kernel; 152 SMs, 16 particles per warp):
+//  strict arithmetic: always.  Its operations come in pairs of planes, so the
+//   two-lane form issues no more of them at any size, and the constant division
+//   and the coefficient cache shorten it: FODO ring (128 elements) 1,024
+//   particles 167 -> 69, 65,536 particles 475 -> 434; light-source ring (1,024)
+//   65,536 particles 5,352 -> 4,991; thick 768-element ring, 1,000 particles
+//   1,355 -> 357, 65,536 particles 4,481 -> 1,948.
+//  FMA: up to 12 warps per SM.  The sextupole form and the composed linear
+//   elements cost the two-lane code more instructions (6 for 5, 8 for 5 per 32
+//   particles), so the one-lane kernel wins once the pipe is full:
+//   light-source ring 333 particles 652 -> 345, 20,000 (8.2 warps per SM) 707 ->
+//   597, 65,536 1,511 -> 2,009; ring with errors on every magnet 30,000 (12.3)
+//   442 -> 404, 65,536 826 -> 891.
+bool use_pair(const ufo_ctx *ctx, const ufo_prog *prog, int64_t n, int flags) {
+  if (!prog->pair_ops || ((flags & UFO_TRACK_FMA) && !prog->pair_fma) || (flags & (UFO_TRACK_PLAIN | UFO_TRACK_COMPACT))) return false;
+  if (!(flags & UFO_TRACK_FMA)) return true;
+  return (n + 15) / 16 <= 12 * static_cast<int64_t>(ctx->sm_count);
+}
+
+// The program's coefficient cache for a two-lane launch of `lanes` lanes, grown
+// when needed and until a graph holds it.  Without memory for it (or under the
+// caller's own stream capture, which allows no allocation) the launch takes the
+// one-lane kernel.
+constexpr size_t CACHE_MOST = size_t{4} << 30;
+
+void ensure_cache(const ufo_prog *prog, int64_t lanes, cudaStream_t stream) {
+  if (!prog->cache_fields) return;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (capturing != cudaStreamCaptureStatusNone) prog->captured = true;
+  if (prog->cache_lanes >= lanes || prog->captured) return;
+  // lanes of the largest grid where that is cheap, so that it grows once
+  const size_t per_lane = sizeof(double) * static_cast<size_t>(prog->cache_fields);
+  const int64_t most = static_cast<int64_t>(prog->ctx->sm_count) * 16 * 32;
+  if (per_lane * most <= CACHE_MOST / 8) lanes = std::max(lanes, most);
+  const size_t bytes = per_lane * lanes;
+  if (bytes > CACHE_MOST) return;
+  double *buf = nullptr;
+  if (cudaMalloc(&buf, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  // zeros: lanes without a particle read finite coefficients
+  if (cudaMemsetAsync(buf, 0, bytes, stream) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(buf);
+    return;
+  }
+  cudaFree(prog->cache);  // waits for launches that use it
+  prog->cache = buf;
+  prog->cache_lanes = lanes;
 }
 
 int launch_track(ufo_ctx *ctx, const ufo_prog *prog, const double *d_coords, const int32_t *d_seed,
@@ -1073,7 +1363,19 @@ int launch_track(ufo_ctx *ctx, const ufo_prog *prog, const double *d_coords, con
                                slots, every, d_tracks, d_lost, d_final, ctx->queue);
   a.pool = ctx->pool;
   a.pool_seq = ctx->pool_seq;
-  const int rc = launch_kernels(a, prog->full, ctx->sm_count, ctx->warps_per_sm, stream);
+  bool pair = use_pair(ctx, prog, n, flags);
+  if (pair) {
+    a.pair_ops = prog->pair_ops;
+    if (prog->cache_fields) {
+      const int64_t lanes = 32 * pair_warps(n, ctx->sm_count, ctx->warps_per_sm);
+      ensure_cache(prog, lanes, stream);
+      pair = prog->cache_lanes >= lanes;
+      a.cache = prog->cache;
+      a.cache_lanes = prog->cache_lanes;
+    }
+  }
+  const int rc =
+      launch_kernels(a, prog->full, pair, ctx->sm_count, ctx->warps_per_sm, stream);
   if (rc == UFO_OK) ctx->launches.fetch_add(1);
   return rc;
 }
@@ -1262,9 +1564,18 @@ int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *t
   p->host_ops.assign(ops, ops + static_cast<size_t>(n_ops) * UFO_OP_WORDS);
   p->ops = nullptr;
   p->table = nullptr;
+  p->pair_ops = nullptr;
+  p->cache = nullptr;
+  p->cache_lanes = 0;
+  p->captured = false;
+  const bool pair =
+      decode_pair(ops, n_ops, table, stride, n_seeds, INT_MAX, p->host_pair_ops, p->cache_fields,
+                  p->pair_fma);
+  const size_t pb = sizeof(ufo::PairOp) * p->host_pair_ops.size();
   const size_t ob = sizeof(ufo::Op) * (n_ops > 0 ? n_ops : 1);
   const size_t tb = sizeof(double) * static_cast<size_t>(stride) * n_seeds;
-  if (cudaMalloc(&p->ops, ob) != cudaSuccess || cudaMalloc(&p->table, tb) != cudaSuccess) {
+  if (cudaMalloc(&p->ops, ob) != cudaSuccess || cudaMalloc(&p->table, tb) != cudaSuccess ||
+      (pair && cudaMalloc(&p->pair_ops, pb) != cudaSuccess)) {
     cudaFree(p->ops);
     cudaFree(p->table);
     delete p;
@@ -1274,10 +1585,14 @@ int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *t
                                   ctx->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(p->table, table, tb, cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess && pair)
+    e = cudaMemcpyAsync(p->pair_ops, p->host_pair_ops.data(), pb, cudaMemcpyHostToDevice,
+                        ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
     cudaFree(p->ops);
     cudaFree(p->table);
+    cudaFree(p->pair_ops);
     delete p;
     return cuda_fail(e, "program upload");
   }
@@ -1293,6 +1608,24 @@ int ufo_prog_set_table(ufo_prog *prog, const double *table, int n_seeds) {
   if (rc) return rc;
   UFO_CUDA(cudaSetDevice(prog->ctx->device));
   const size_t tb = sizeof(double) * static_cast<size_t>(prog->stride) * n_seeds;
+  if (prog->pair_ops) {
+    // new constants may share other cache fields or admit another division form
+    int fields = 0;
+    std::vector<ufo::PairOp> ops2;
+    decode_pair(prog->host_ops.data(), prog->n_ops, table, prog->stride, n_seeds,
+                prog->captured ? prog->cache_fields : INT_MAX, ops2, fields, prog->pair_fma);
+    if (ops2.size() != prog->host_pair_ops.size() ||
+        std::memcmp(ops2.data(), prog->host_pair_ops.data(), sizeof(ufo::PairOp) * ops2.size())) {
+      UFO_CUDA(cudaMemcpyAsync(prog->pair_ops, ops2.data(), sizeof(ufo::PairOp) * ops2.size(),
+                               cudaMemcpyHostToDevice, prog->ctx->stream));
+      UFO_CUDA(cudaStreamSynchronize(prog->ctx->stream));
+      prog->host_pair_ops.swap(ops2);
+      if (fields > prog->cache_fields) {  // grown at the next launch
+        prog->cache_lanes = 0;
+        prog->cache_fields = fields;
+      }
+    }
+  }
   UFO_CUDA(cudaMemcpyAsync(prog->table, table, tb, cudaMemcpyHostToDevice, prog->ctx->stream));
   UFO_CUDA(cudaStreamSynchronize(prog->ctx->stream));
   return UFO_OK;
@@ -1306,6 +1639,8 @@ void ufo_prog_destroy(ufo_prog *prog) {
   cudaDeviceSynchronize();
   cudaFree(prog->ops);
   cudaFree(prog->table);
+  cudaFree(prog->pair_ops);
+  cudaFree(prog->cache);
   delete prog;
 }
 
@@ -1471,7 +1806,7 @@ extern "C" int ufo_track_noalloc(const int32_t *ops, int n_ops, const double *d_
                                d_coords, d_seed, d_pturns, n, turns, mode,
                                flags & ~UFO_TRACK_PLAIN, slots, every, d_tracks, d_lost, d_final,
                                &d.scratch->queue);
-  return launch_kernels(a, needs_full(ops, n_ops), d.sm_count, 16, st);
+  return launch_kernels(a, needs_full(ops, n_ops), false, d.sm_count, 16, st);
 }
 
 // ===================================================== tuning and graphs
@@ -1555,6 +1890,10 @@ extern "C" int ufo_graph_create(ufo_ctx *ctx, const ufo_prog *prog, const double
   if (n <= 0) return fail(UFO_E_ARG, "empty launch");
   if (!d_coords) return fail(UFO_E_ARG, "null coordinates");
   UFO_CUDA(cudaSetDevice(ctx->device));
+  if (use_pair(ctx, prog, n, flags)) {  // nothing may be allocated under capture
+    ensure_cache(prog, 32 * pair_warps(n, ctx->sm_count, ctx->warps_per_sm), ctx->stream);
+    UFO_CUDA(cudaStreamSynchronize(ctx->stream));
+  }
   cudaStream_t cap;
   UFO_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
   cudaGraph_t graph = nullptr;
