@@ -174,3 +174,40 @@ def test_graph_of_a_thick_batch_keeps_its_cache():
     b.dprog.set_table(b.prog.table * 1.0)
     b.launch()
     assert _same(first, b.download())
+
+
+@pytest.mark.parametrize('name', ['c1', 'alba_kick', 'mixed'])
+@pytest.mark.parametrize('n', [1, 3, 700])
+def test_closed_orbits_of_lane_pairs_are_the_one_thread_searchs(name, n):
+    """The four-trial search (one and four orbits per warp) against the
+    one-thread search, which batches beyond 64 orbits per SM take: regular
+    starts, a start on the orbit (equal residuals), far and non-finite ones."""
+    import ufo_gb300 as u
+    from ufo_gb300 import capi, compiler as C
+    line, flags = _rings()[name]
+    ctx = u.context(0)
+    at = [i for i, e in enumerate(line.flatten()) if type(e).__name__ == 'Quadrupole'][:3]
+    params = [(i, 'dx') for i in at]
+    rows = np.random.default_rng(5).normal(0, 1e-4, (7, len(at)))
+    rows[0] = 0.0  # the orbit is exactly zero
+    dp = capi.DeviceProgram(ctx, C.compile_line(line, flags, params, [], seed_values=rows))
+    start = _beam(n)[:, :4] * 0.1
+    start[0] = 0.0
+    if n > 3:
+        start[5] = 0.5
+        start[6, 1] = np.nan
+        start[7, 2] = np.inf
+    seed = (np.arange(n) % 7).astype(np.int32)
+
+    def orbits(st, sd, steps):
+        out = np.empty_like(st)
+        capi.check(capi.load().ufo_closed_orbit(ctx.handle, dp.handle, capi.ptr(st),
+                                                capi.ptr(sd), len(st), steps, capi.ptr(out)))
+        return out
+    import torch
+    many = 64 * torch.cuda.get_device_properties(0).multi_processor_count + 1
+    reps = -(-many // n)
+    for steps in (0, 1, 37):
+        got = orbits(start, seed, steps)
+        ref = orbits(np.tile(start, (reps, 1)), np.tile(seed, reps), steps)[:n]
+        assert np.array_equal(got, ref, equal_nan=True)

@@ -1853,7 +1853,25 @@ extern "C" int ufo_closed_orbit(ufo_ctx *ctx, const ufo_prog *prog, const double
                                prog->n_dumps, nullptr, d_seed, nullptr, n, 1, UFO_MODE_TRACK, 0, 0,
                                1, nullptr, nullptr, nullptr, ctx->queue);
   const unsigned blocks = static_cast<unsigned>((n + 31) / 32);
-  if (prog->full)
+  // Four lane pairs per orbit: one orbit per warp while the sub-partitions last
+  // (no orbit waits for another's shrink), then four.  The one-thread search
+  // wins back where its warps fill the GPU (n > 64 per SM), except that it
+  // recomputes the thick elements' functions in every turn.
+  bool pair = prog->pair_ops && (prog->cache_fields || n <= 64 * static_cast<int64_t>(ctx->sm_count));
+  const int per_warp = n <= 4 * static_cast<int64_t>(ctx->sm_count) ? 1 : 4;
+  const int64_t warps = std::min((n + per_warp - 1) / per_warp,
+                                 16 * static_cast<int64_t>(ctx->sm_count));
+  if (pair && prog->cache_fields) {
+    ensure_cache(prog, 32 * warps, st);
+    pair = prog->cache_lanes >= 32 * warps;
+    a.cache = prog->cache;
+    a.cache_lanes = prog->cache_lanes;
+  }
+  if (pair) {
+    a.pair_ops = prog->pair_ops;
+    ufo::co_pair_kernel<<<static_cast<unsigned>(warps), 32, 0, st>>>(a, d_start, d_orbits,
+                                                                     iterations, per_warp);
+  } else if (prog->full)
     ufo::co_amoeba_kernel<true><<<blocks, 32, 0, st>>>(a, d_start, d_orbits, iterations);
   else
     ufo::co_amoeba_kernel<false><<<blocks, 32, 0, st>>>(a, d_start, d_orbits, iterations);
