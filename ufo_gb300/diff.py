@@ -135,17 +135,16 @@ class DiffProgram:
         reference pads coefficient lists with zeros), keeping the order a
         parameter scales; the constant table is repacked."""
         out_ops, cols = [], []
-        for op in ops:
-            kind, off, M, ps, pm = int(op[0]), int(op[2]), int(op[4]), int(op[5]), int(op[6])
-            op = op.copy()
+        nonzero = np.any(tab != 0, axis=0)
+        for op in ops.tolist():
+            kind, off, M, ps, pm = op[0], op[2], op[4], op[5], op[6]
             op[2] = len(cols)
             if kind in (D_TEAPOT, D_KICK):
                 h = KHDR
                 hdr = list(range(off, off + h))
-                a = tab[:, off + h:off + h + M]
-                b = tab[:, off + h + M:off + h + 2 * M]
-                nz = np.nonzero(np.any(a != 0, axis=0) | np.any(b != 0, axis=0))[0]
-                Mt = max(int(nz.max()) + 1 if len(nz) else 1, pm + 1 if ps >= 0 else 1)
+                nz = nonzero[off + h:off + h + M] | nonzero[off + h + M:off + h + 2 * M]
+                Mt = max(int(nz.nonzero()[0][-1]) + 1 if nz.any() else 1,
+                         pm + 1 if ps >= 0 else 1)
                 op[4] = Mt
                 cols += hdr + list(range(off + h, off + h + Mt)) + \
                     list(range(off + h + M, off + h + M + Mt))
@@ -162,13 +161,14 @@ class DiffProgram:
         """Opcode list and constant columns for all seed rows of ``prog.table``
         at once: each constant is an array over the rows (or a scalar)."""
         T = prog.table
+        one = T[0].tolist() if T.shape[0] == 1 else None  # one row: plain floats
         ops, tab = [], []
         kicks = 0
-        for r, elem in zip(prog.ops, prog.op_elem):
-            kind, fl, off = int(r[0]), int(r[1]), int(r[2])
+        for r, elem in zip(prog.ops.tolist(), prog.op_elem):
+            kind, fl, off = r[0], r[1], r[2]
 
             def c(k, off=off):
-                return T[:, off + k]
+                return one[off + k] if one is not None else T[:, off + k]
 
             achro = 1 if fl & C.F_ACHRO else 0
             if kind in (C.OP_NOP, C.OP_OBSERVE, C.OP_APERTURE):
@@ -260,9 +260,10 @@ class DiffProgram:
             else:
                 raise NotImplementedError(f'{C.OP_NAMES[kind]} elements are not differentiated')
         S = T.shape[0]
-        tab = np.stack([np.broadcast_to(np.asarray(v, np.float64), (S,)) for v in tab + [0.0]],
-                       axis=1) if tab else np.zeros((S, 1))
-        return ops, tab, kicks
+        out = np.zeros((S, len(tab) + 1))
+        for j, v in enumerate(tab):
+            out[:, j] = v
+        return ops, out, kicks
 
 
 class DiffEngine:
