@@ -85,18 +85,18 @@ __device__ __forceinline__ void series(const double *__restrict__ a, int M, doub
   s0r = __ldg(a + M - 1);
   s0i = __ldg(b + M - 1);
   s1r = s1i = s2r = s2i = 0.0;
-  for (int n = M - 2; n >= 0; --n) {
+  for (int n = M - 2; n >= 0; --n) {  // x's product first, in both components
     if (ND >= 2) {
-      const double tr = fma(s2r, x, fma(-s2i, y, s1r));
+      const double tr = fma(-s2i, y, fma(s2r, x, s1r));
       s2i = fma(s2r, y, fma(s2i, x, s1i));
       s2r = tr;
     }
     if (ND >= 1) {
-      const double tr = fma(s1r, x, fma(-s1i, y, s0r));
+      const double tr = fma(-s1i, y, fma(s1r, x, s0r));
       s1i = fma(s1r, y, fma(s1i, x, s0i));
       s1r = tr;
     }
-    const double tr = fma(s0r, x, fma(-s0i, y, __ldg(a + n)));
+    const double tr = fma(-s0i, y, fma(s0r, x, __ldg(a + n)));
     s0i = fma(s0r, y, fma(s0i, x, __ldg(b + n)));
     s0r = tr;
   }
@@ -129,8 +129,8 @@ __device__ __forceinline__ void fwd_kick(St &s, const double *a, int M, double o
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const double dx = s.T[j], dy = s.T[8 + j];
-      s.T[4 + j] -= fma(ar, dx, -ai * dy);
-      s.T[12 + j] += fma(ai, dx, ar * dy);
+      s.T[4 + j] = fma(ai, dy, fma(-ar, dx, s.T[4 + j]));
+      s.T[12 + j] = fma(ai, dx, fma(ar, dy, s.T[12 + j]));
     }
   } else {
     series<0>(a, M, s.x, s.y, sr, si, ar, ai, br, bi);
@@ -233,14 +233,17 @@ __device__ __forceinline__ double thick_plane_rev(double &qb, double &pqb, doubl
   const double A = -K * Sw, dA = fma(-K, dSw, -Sw);
   double Kb = fma(qb, fma(dC, q, fma(dSw, pq, disp * dD1)),
                   pqb * fma(dA, q, fma(dC, pq, disp * dSw)));
-  if (tangent)
+  if (tangent) {
+    double kt[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      Kb = fma(bq[j], fma(dC, tq[j], dSw * tp[j]), fma(bp[j], fma(dA, tq[j], dC * tp[j]), Kb));
+      kt[j] = fma(bq[j], fma(dC, tq[j], dSw * tp[j]), bp[j] * fma(dA, tq[j], dC * tp[j]));
       const double b = bq[j];
       bq[j] = fma(C, b, A * bp[j]);
       bp[j] = fma(Sw, b, C * bp[j]);
     }
+    Kb += (kt[0] + kt[1]) + (kt[2] + kt[3]);
+  }
   const double b = qb;
   qb = fma(C, b, A * pqb);
   pqb = fma(Sw, b, C * pqb);
@@ -397,8 +400,8 @@ __device__ __forceinline__ void rev_kick(Bar &b, const DiffArgs &a, int tt, int 
   a1 *= o;
   b1 *= o;
   // state: px' = px - Re S, py' = py + Im S
-  double xb = fma(-b.px, a1, b.py * b1);
-  double yb = fma(b.px, b1, b.py * a1);
+  double xb = fma(b.py, b1, fma(-b.px, a1, b.x));
+  double yb = fma(b.px, b1, fma(b.py, a1, b.y));
   if (pm >= 0) {  // dS/dc = o z^pm / pm!
     double zr, zi;
     zpow(x, y, pm, zr, zi);
@@ -407,29 +410,32 @@ __device__ __forceinline__ void rev_kick(Bar &b, const DiffArgs &a, int tt, int 
   if (tangent) {
     a2 *= 2.0 * o;
     b2 *= 2.0 * o;
-    double Ab = 0.0, Bb = 0.0;
+    double At[4], Bt[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const double dx = a.tape[tidx(a, tt, k, 2 + q, nf, j)];
       const double dy = a.tape[tidx(a, tt, k, 6 + q, nf, j)];
       const double pxb = b.T[4 + q], pyb = b.T[12 + q];
       // T_px -= a1 dx - b1 dy ; T_py += b1 dx + a1 dy
-      b.T[q] += fma(-pxb, a1, pyb * b1);
-      b.T[8 + q] += fma(pxb, b1, pyb * a1);
-      Ab += fma(-pxb, dx, pyb * dy);
-      Bb += fma(pxb, dy, pyb * dx);
+      b.T[q] = fma(pyb, b1, fma(-pxb, a1, b.T[q]));
+      b.T[8 + q] = fma(pxb, b1, fma(pyb, a1, b.T[8 + q]));
+      At[q] = fma(-pxb, dx, pyb * dy);
+      Bt[q] = fma(pyb, dx, pxb * dy);
     }
+    // summed in the order of the eight-lane form's butterfly
+    const double Ab = (At[0] + At[1]) + (At[2] + At[3]);
+    const double Bb = (Bt[0] + Bt[1]) + (Bt[2] + Bt[3]);
     // a1 + i b1 = S'(z): d/dx = S'' , d/dy = i S''
-    xb += fma(Ab, a2, Bb * b2);
-    yb += fma(-Ab, b2, Bb * a2);
+    xb = fma(Bb, b2, fma(Ab, a2, xb));
+    yb = fma(Ab, -b2, fma(Bb, a2, yb));
     if (pm >= 1) {  // dS'/dc = o z^(pm-1) / (pm-1)!
       double zr, zi;
       zpow(x, y, pm - 1, zr, zi);
       g1 += o * fma(Ab, zr, Bb * zi);
     }
   }
-  b.x += xb;
-  b.y += yb;
+  b.x = xb;
+  b.y = yb;
 }
 
 // reverse of turn `tt` of the segment from its tape; accumulates parameter
@@ -635,83 +641,100 @@ struct Half {
 
 __device__ __forceinline__ double other(double v) { return __shfl_xor_sync(ALL_LANES, v, 1); }
 
+// -v by its sign bit: as a floating-point negation that no FMA absorbs it would
+// take a slot of the FP64 pipe (and its 115-cycle way to a select or shuffle)
+__device__ __forceinline__ double neg(double v) {
+  return __hiloint2double(__double2hiint(v) ^ static_cast<int>(0x80000000u), __double2loint(v));
+}
+// v != 0 without the pipe's comparison
+__device__ __forceinline__ bool nonzero(double v) {
+  return ((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) != 0;
+}
+
 // S(z)/o (and S'(z)/o with ND = 1) split over the pair: `r0` / `r1` are this
-// lane's part (real on even lanes, imaginary on odd lanes)
+// lane's part (real on even lanes, imaginary on odd lanes).  Both parts of a
+// Horner step are (own x + c) -+ other y, so a lane's own value goes straight
+// into the next FMA (64.6 cycles) while the other lane's is on its way through
+// the shuffle (about 75 more than that): sy = -y on even, y on odd lanes.
+// Measured, 777 particles through the 1,024-element ring with errors: 2.58 ->
+// 1.84 ms per turn forward, with the operands' signs changed outside the FP64
+// pipe and the opcodes fetched ahead.
 template <int ND>
-__device__ __forceinline__ void series_pair(const double *__restrict__ a, int M, double x, double y,
+__device__ __forceinline__ void series_pair(const double *__restrict__ a, int M, double x, double sy,
                                             bool even, double &r0, double &r1) {
-  const double *b = a + M;
-  const double p = even ? x : y, q = even ? y : x;
-  r0 = even ? __ldg(a + M - 1) : __ldg(b + M - 1);
+  const double *c = even ? a : a + M;
+  r0 = __ldg(c + M - 1);
   r1 = 0.0;
   for (int n = M - 2; n >= 0; --n) {
     const double o0 = other(r0);
-    const double sr0 = even ? r0 : o0, si0 = even ? o0 : r0;
     if (ND >= 1) {
       const double o1 = other(r1);
-      const double sr1 = even ? r1 : o1, si1 = even ? o1 : r1;
-      // re: fma(s1r, x, fma(-s1i, y, s0r)); im: fma(s1r, y, fma(s1i, x, s0i))
-      r1 = fma(sr1, p, fma(even ? -si1 : si1, q, even ? sr0 : si0));
+      r1 = fma(o1, sy, fma(r1, x, r0));
     }
-    const double c = even ? __ldg(a + n) : __ldg(b + n);
-    r0 = fma(sr0, p, fma(even ? -si0 : si0, q, c));
+    r0 = fma(o0, sy, fma(r0, x, __ldg(c + n)));
   }
+}
+
+// this lane's tape entry of kick 0 of turn tt (plain mode)
+__device__ __forceinline__ double *tape_turn(const DiffArgs &a, int tt, int j) {
+  return a.tape + tidx(a, tt, 0, 0, 4, j);
 }
 
 // a kick element of the pair with its M coefficients (this lane's part: the
 // normal list on even lanes, the skew list on odd lanes) loaded into
 // registers once for all N slices; the unrolled Horner issues no loads
-template <int M>
-__device__ __forceinline__ void kick_elem_pair(Half &h, const DiffArgs &a, const double *c, bool tp,
-                                               int N, double oo, bool even, int j, bool write,
-                                               int tt, bool tape, int &kidx) {
+template <int M, bool TAPE>
+__device__ __forceinline__ void kick_elem_pair(Half &h, const double *c, bool tp, int N, double oo,
+                                               bool even, bool write, double *&tape) {
   double cf[M];
   const double *src = c + KHDR + (even ? 0 : M);
 #pragma unroll
   for (int n = 0; n < M; ++n) cf[n] = __ldg(src + n);
   const double Lo = __ldg(c), Li = __ldg(c + 1), W = __ldg(c + 2), Lx = __ldg(c + 5);
+  const double so = even ? neg(oo) : oo, sw = even ? neg(W) : 0.0;
+  const bool weak = tp && nonzero(W);
   if (tp) h.u = fma(h.pu, Lo, h.u);
   for (int sl = 0; sl < N; ++sl) {
-    const int k = kidx++;
     const double w = other(h.u);
-    const double x = even ? h.u : w, y = even ? w : h.u;
-    const double p = even ? x : y, q = even ? y : x;
+    const double x = even ? h.u : w, sy = even ? neg(w) : h.u;
     double r0 = cf[M - 1], r1 = 0.0;
-    if (tape) {
 #pragma unroll
-      for (int n = M - 2; n >= 0; --n) {
-        const double o0 = other(r0), o1 = other(r1);
-        const double sr0 = even ? r0 : o0, si0 = even ? o0 : r0;
-        const double sr1 = even ? r1 : o1, si1 = even ? o1 : r1;
-        r1 = fma(sr1, p, fma(even ? -si1 : si1, q, even ? sr0 : si0));
-        r0 = fma(sr0, p, fma(even ? -si0 : si0, q, cf[n]));
+    for (int n = M - 2; n >= 0; --n) {
+      const double o0 = other(r0);
+      if (TAPE) {
+        const double o1 = other(r1);
+        r1 = fma(o1, sy, fma(r1, x, r0));
       }
-      if (write) {
-        double *t0 = a.tape + tidx(a, tt, k, 0, 4, j);
-        t0[even ? 0 : TLANES] = h.u;
-        t0[(even ? 2 : 3) * TLANES] = oo * r1;
-      }
-    } else {
-#pragma unroll
-      for (int n = M - 2; n >= 0; --n) {
-        const double o0 = other(r0);
-        const double sr0 = even ? r0 : o0, si0 = even ? o0 : r0;
-        r0 = fma(sr0, p, fma(even ? -si0 : si0, q, cf[n]));
-      }
+      r0 = fma(o0, sy, fma(r0, x, cf[n]));
     }
-    h.pu = fma(even ? -oo : oo, r0, h.pu);
-    if (tp && W != 0.0 && even) h.pu = fma(-W, h.u, h.pu);
+    if (TAPE) {
+      if (write) {
+        tape[even ? 0 : TLANES] = h.u;
+        tape[(even ? 2 : 3) * TLANES] = oo * r1;
+      }
+      tape += 4 * TLANES;
+    }
+    h.pu = fma(so, r0, h.pu);
+    if (weak) h.pu = fma(sw, h.u, h.pu);
     if (tp) h.u = fma(h.pu, sl < N - 1 ? Li : Lx, h.u);
   }
 }
 
-// one turn forward of the pair; with `tape` the rich tape is written as turn
-// `tt` of the group (x, Re S' by the even lane; y, Im S' by the odd lane)
+__device__ __forceinline__ DOp fetch(const DOp *p) {
+  const int4 v = __ldg(reinterpret_cast<const int4 *>(p));
+  const int4 w = __ldg(reinterpret_cast<const int4 *>(p) + 1);
+  return {v.x, v.y, v.z, v.w, w.x, w.y, w.z, w.w};
+}
+
+// one turn forward of the pair; with TAPE the rich tape is written from `tape`
+// on (x, Re S' by the even lane; y, Im S' by the odd lane)
+template <bool TAPE>
 __device__ void turn_forward_pair(Half &h, const DiffArgs &a, const double *T0, double o,
-                                  bool even, int j, bool write, int tt, bool tape) {
-  int kidx = 0;
+                                  bool even, bool write, double *tape) {
+  DOp next = fetch(a.ops);
   for (int i = 0; i < a.n_ops; ++i) {
-    const DOp op = a.ops[i];
+    const DOp op = next;
+    if (i + 1 < a.n_ops) next = fetch(a.ops + i + 1);
     const double *c = T0 + op.toff;
     const double oo = op.achro ? 1.0 : o;
     switch (op.kind) {
@@ -724,17 +747,17 @@ __device__ void turn_forward_pair(Half &h, const DiffArgs &a, const double *T0, 
       case D_EDGE: {
         const double curv = __ldg(c) * oo;
         const double t = h.u * curv;
-        h.pu = fma(even ? t : -t, even ? __ldg(c + 1) : edge_t2(op.flags, c, curv), h.pu);
+        h.pu = fma(t, even ? __ldg(c + 1) : neg(edge_t2(op.flags, c, curv)), h.pu);
         break;
       }
       case D_THICK: {
         const double L = __ldg(c), k1 = __ldg(c + 1), hh = __ldg(c + 2);
-        const int k = kidx;
-        kidx += THICK_SLOTS;
-        if (tape && write) {  // entry state: x, px by the even lane; y, py by the odd lane
-          double *t0 = a.tape + tidx(a, tt, k, 0, 4, j);
-          t0[even ? 0 : TLANES] = h.u;
-          t0[(even ? 2 : 3) * TLANES] = h.pu;
+        if (TAPE) {  // entry state: x, px by the even lane; y, py by the odd lane
+          if (write) {
+            tape[even ? 0 : TLANES] = h.u;
+            tape[(even ? 2 : 3) * TLANES] = h.pu;
+          }
+          tape += THICK_SLOTS * 4 * TLANES;
         }
         const double K = even ? oo * fma(hh, hh, k1) : -oo * k1;
         const double disp = (even && (op.flags & DT_BEND)) ? (1.0 / o - 1.0) * hh * oo : 0.0;
@@ -746,35 +769,32 @@ __device__ void turn_forward_pair(Half &h, const DiffArgs &a, const double *T0, 
         const bool tp = op.kind == D_TEAPOT;
         const int N = tp ? op.N : 1;
         switch (op.M) {  // common orders: coefficients in registers
-          case 1: kick_elem_pair<1>(h, a, c, tp, N, oo, even, j, write, tt, tape, kidx); continue;
-          case 2: kick_elem_pair<2>(h, a, c, tp, N, oo, even, j, write, tt, tape, kidx); continue;
-          case 3: kick_elem_pair<3>(h, a, c, tp, N, oo, even, j, write, tt, tape, kidx); continue;
-          case 4: kick_elem_pair<4>(h, a, c, tp, N, oo, even, j, write, tt, tape, kidx); continue;
-          case 5: kick_elem_pair<5>(h, a, c, tp, N, oo, even, j, write, tt, tape, kidx); continue;
-          case 6: kick_elem_pair<6>(h, a, c, tp, N, oo, even, j, write, tt, tape, kidx); continue;
-          case 7: kick_elem_pair<7>(h, a, c, tp, N, oo, even, j, write, tt, tape, kidx); continue;
-          case 8: kick_elem_pair<8>(h, a, c, tp, N, oo, even, j, write, tt, tape, kidx); continue;
+          case 1: kick_elem_pair<1, TAPE>(h, c, tp, N, oo, even, write, tape); continue;
+          case 2: kick_elem_pair<2, TAPE>(h, c, tp, N, oo, even, write, tape); continue;
+          case 3: kick_elem_pair<3, TAPE>(h, c, tp, N, oo, even, write, tape); continue;
+          case 4: kick_elem_pair<4, TAPE>(h, c, tp, N, oo, even, write, tape); continue;
+          case 5: kick_elem_pair<5, TAPE>(h, c, tp, N, oo, even, write, tape); continue;
+          case 6: kick_elem_pair<6, TAPE>(h, c, tp, N, oo, even, write, tape); continue;
+          case 7: kick_elem_pair<7, TAPE>(h, c, tp, N, oo, even, write, tape); continue;
+          case 8: kick_elem_pair<8, TAPE>(h, c, tp, N, oo, even, write, tape); continue;
           default: break;
         }
         const double Lo = __ldg(c), Li = __ldg(c + 1), W = __ldg(c + 2), Lx = __ldg(c + 5);
         if (tp) h.u = fma(h.pu, Lo, h.u);
         for (int sl = 0; sl < N; ++sl) {
-          const int k = kidx++;
           const double w = other(h.u);
-          const double x = even ? h.u : w, y = even ? w : h.u;
+          const double x = even ? h.u : w, sy = even ? neg(w) : h.u;
           double s0, s1;
-          if (tape) {
-            series_pair<1>(c + KHDR, op.M, x, y, even, s0, s1);
+          series_pair<TAPE ? 1 : 0>(c + KHDR, op.M, x, sy, even, s0, s1);
+          if (TAPE) {
             if (write) {
-              double *t0 = a.tape + tidx(a, tt, k, 0, 4, j);
-              t0[even ? 0 : TLANES] = h.u;
-              t0[(even ? 2 : 3) * TLANES] = oo * s1;
+              tape[even ? 0 : TLANES] = h.u;
+              tape[(even ? 2 : 3) * TLANES] = oo * s1;
             }
-          } else {
-            series_pair<0>(c + KHDR, op.M, x, y, even, s0, s1);
+            tape += 4 * TLANES;
           }
-          h.pu = fma(even ? -oo : oo, s0, h.pu);
-          if (tp && W != 0.0 && even) h.pu = fma(-W, h.u, h.pu);
+          h.pu = fma(even ? neg(oo) : oo, s0, h.pu);
+          if (tp && nonzero(W)) h.pu = fma(even ? neg(W) : 0.0, h.u, h.pu);
           if (tp) h.u = fma(h.pu, sl < N - 1 ? Li : Lx, h.u);
         }
         break;
@@ -785,40 +805,48 @@ __device__ void turn_forward_pair(Half &h, const DiffArgs &a, const double *T0, 
   }
 }
 
-// reverse of a kick element of the pair with the tape values of its N slices
-// (x, y, Re S', Im S') loaded up front, before the dependent cotangent chain
+// Reverse of a kick element of the pair with the tape values of its N slices
+// (x, y, Re S', Im S') loaded up front, before the dependent cotangent chain;
+// `tape` points past them and moves to the element's first slice.
+//   xb += -pxb a1 + pyb b1,  yb += pyb a1 + pxb b1  (a1 + i b1 = S'):
+// both parts are own a1 first, then the other lane's b1.
+// A part of N slices; `last`: it ends with the element's last slice, `first`: it
+// starts with the first.
 template <int N>
-__device__ __forceinline__ void rev_elem_pair(Half &bh, const DiffArgs &a, const double *c, bool tp,
-                                              double oo, bool even, int j, bool write, int tt,
-                                              int pm, int &kidx, double &g0) {
+__device__ __forceinline__ void rev_part_pair(Half &bh, const DiffArgs &a, const double *c, bool tp,
+                                              bool last, bool first, bool even, int j, bool write,
+                                              int tt, int pm, int &kidx, const double *&tape,
+                                              double &g0) {
   double tx[N], ty[N], ta[N], tb[N];
 #pragma unroll
   for (int q = 0; q < N; ++q) {
-    const double *t0 = a.tape + tidx(a, tt, kidx - 1 - q, 0, 4, j);
+    const double *t0 = tape - (q + 1) * 4 * TLANES;
     tx[q] = t0[0];
     ty[q] = t0[TLANES];
-    ta[q] = t0[2 * TLANES];
+    ta[q] = even ? neg(t0[2 * TLANES]) : t0[2 * TLANES];
     tb[q] = t0[3 * TLANES];
   }
+  tape -= N * 4 * TLANES;
   const double Lo = __ldg(c), Li = __ldg(c + 1), W = __ldg(c + 2), Lx = __ldg(c + 5);
+  const double sw = even ? neg(W) : 0.0;
+  const bool weak = tp && nonzero(W);
 #pragma unroll
   for (int q = 0; q < N; ++q) {  // slice N-1-q
-    if (tp) bh.pu = fma(bh.u, q > 0 ? Li : Lx, bh.pu);
-    if (tp && W != 0.0 && even) bh.u = fma(-W, bh.pu, bh.u);
+    if (tp) bh.pu = fma(bh.u, q == 0 && last ? Lx : Li, bh.pu);
+    if (weak) bh.u = fma(sw, bh.pu, bh.u);
     --kidx;
     if (write && even && kidx % CHUNK == 0 && kidx >= 2 * CHUNK)
       prefetch_chunk(a, tt, kidx - 2 * CHUNK, j);
-    const double a1 = ta[q], b1 = tb[q];
     const double w = other(bh.pu);
-    const double pxb = even ? bh.pu : w, pyb = even ? w : bh.pu;
-    bh.u = fma(even ? -pxb : pxb, even ? a1 : b1, fma(pyb, even ? b1 : a1, bh.u));
+    bh.u = fma(w, tb[q], fma(bh.pu, ta[q], bh.u));
     if (pm >= 0) {
       double zr, zi;
       zpow_small(tx[q], ty[q], pm, zr, zi);
+      const double pxb = even ? bh.pu : w, pyb = even ? w : bh.pu;
       g0 = fma(-pxb, zr, fma(pyb, zi, g0));
     }
   }
-  if (tp) bh.pu = fma(bh.u, Lo, bh.pu);
+  if (tp && first) bh.pu = fma(bh.u, Lo, bh.pu);
 }
 
 // reverse of turn `tt` of the group from the rich tape, split over the pair
@@ -831,8 +859,11 @@ __device__ void turn_reverse_pair(Half &bh, const DiffArgs &a, const double *T0,
     prefetch_chunk(a, tt, top, j);
     prefetch_chunk(a, tt, top - CHUNK, j);
   }
+  const double *tape = tape_turn(a, tt, j) + static_cast<int64_t>(kidx) * 4 * TLANES;
+  DOp next = a.n_ops > 0 ? fetch(a.ops + a.n_ops - 1) : DOp{};
   for (int i = a.n_ops - 1; i >= 0; --i) {
-    const DOp op = a.ops[i];
+    const DOp op = next;
+    if (i > 0) next = fetch(a.ops + i - 1);
     const double *c = T0 + op.toff;
     const double oo = op.achro ? 1.0 : o;
     switch (op.kind) {
@@ -844,16 +875,16 @@ __device__ void turn_reverse_pair(Half &bh, const DiffArgs &a, const double *T0,
       case D_EDGE: {
         const double curv = __ldg(c) * oo;
         const double t = bh.pu * curv;
-        bh.u = fma(even ? t : -t, even ? __ldg(c + 1) : edge_t2(op.flags, c, curv), bh.u);
+        bh.u = fma(t, even ? __ldg(c + 1) : neg(edge_t2(op.flags, c, curv)), bh.u);
         break;
       }
       case D_THICK: {
         const double L = __ldg(c), k1 = __ldg(c + 1), hh = __ldg(c + 2);
         kidx -= THICK_SLOTS;
+        tape -= THICK_SLOTS * 4 * TLANES;
         const int m = ((kidx + THICK_SLOTS - 1) / CHUNK) * CHUNK;  // a chunk start in range
         if (write && even && m >= kidx && m >= 2 * CHUNK) prefetch_chunk(a, tt, m - 2 * CHUNK, j);
-        const double *t0 = a.tape + tidx(a, tt, kidx, 0, 4, j);
-        const double q = t0[even ? 0 : TLANES], pq = t0[(even ? 2 : 3) * TLANES];
+        const double q = tape[even ? 0 : TLANES], pq = tape[(even ? 2 : 3) * TLANES];
         const double K = even ? oo * fma(hh, hh, k1) : -oo * k1;
         const double disp = (even && (op.flags & DT_BEND)) ? (1.0 / o - 1.0) * hh * oo : 0.0;
         const double kb = thick_plane_rev(bh.u, bh.pu, nullptr, nullptr, nullptr, nullptr, q, pq,
@@ -869,40 +900,22 @@ __device__ void turn_reverse_pair(Half &bh, const DiffArgs &a, const double *T0,
       case D_TEAPOT: {
         const bool tp = op.kind == D_TEAPOT;
         const int N = tp ? op.N : 1;
-        const double Lo = __ldg(c), Li = __ldg(c + 1), W = __ldg(c + 2), Lx = __ldg(c + 5);
         const int pm = op.pslot >= 0 ? op.pm : -1;
         double g0 = 0.0;
-        bool done = true;
-        switch (N) {  // common slice counts: the element's tape values up front
-          case 1: rev_elem_pair<1>(bh, a, c, tp, oo, even, j, write, tt, pm, kidx, g0); break;
-          case 2: rev_elem_pair<2>(bh, a, c, tp, oo, even, j, write, tt, pm, kidx, g0); break;
-          case 4: rev_elem_pair<4>(bh, a, c, tp, oo, even, j, write, tt, pm, kidx, g0); break;
-          case 8: rev_elem_pair<8>(bh, a, c, tp, oo, even, j, write, tt, pm, kidx, g0); break;
-          default: done = false; break;
-        }
-        for (int sl = N - 1; !done && sl >= 0; --sl) {
-          if (tp) bh.pu = fma(bh.u, sl < N - 1 ? Li : Lx, bh.pu);
-          if (tp && W != 0.0 && even) bh.u = fma(-W, bh.pu, bh.u);
-          --kidx;
-          if (write && even && kidx % CHUNK == 0 && kidx >= 2 * CHUNK)
-            prefetch_chunk(a, tt, kidx - 2 * CHUNK, j);
-          const double *t0 = a.tape + tidx(a, tt, kidx, 0, 4, j);
-          const double a1 = t0[2 * TLANES], b1 = t0[3 * TLANES];
-          const double w = other(bh.pu);
-          const double pxb = even ? bh.pu : w, pyb = even ? w : bh.pu;
-          // x: fma(-pxb, a1, fma(pyb, b1, xb)); y: fma(pxb, b1, fma(pyb, a1, yb))
-          bh.u = fma(even ? -pxb : pxb, even ? a1 : b1, fma(pyb, even ? b1 : a1, bh.u));
-          if (pm >= 0) {
-            double zr, zi;
-            zpow_small(t0[0], t0[TLANES], pm, zr, zi);
-            g0 = fma(-pxb, zr, fma(pyb, zi, g0));
-          }
-        }
-        if (tp && !done) bh.pu = fma(bh.u, Lo, bh.pu);
+        double p0 = 0.0;  // the parameter's sum so far, fetched ahead
+        double *pp = nullptr;
         if (op.pslot >= 0 && write && even) {
-          double &p = a.pbar[static_cast<int64_t>(op.pslot) * a.n_jobs + j];
-          p = fma(g0 * oo, __ldg(c + 3), p);
+          pp = a.pbar + static_cast<int64_t>(op.pslot) * a.n_jobs + j;
+          p0 = *pp;
         }
+        int left = N;
+        for (; left >= 8; left -= 8)
+          rev_part_pair<8>(bh, a, c, tp, left == N, left == 8, even, j, write, tt, pm, kidx, tape, g0);
+        for (; left >= 4; left -= 4)
+          rev_part_pair<4>(bh, a, c, tp, left == N, left == 4, even, j, write, tt, pm, kidx, tape, g0);
+        for (; left >= 1; --left)
+          rev_part_pair<1>(bh, a, c, tp, left == N, left == 1, even, j, write, tt, pm, kidx, tape, g0);
+        if (pp) *pp = fma(g0 * oo, __ldg(c + 3), p0);
         break;
       }
       default:
@@ -940,7 +953,7 @@ __global__ void diff_forward_pair(DiffArgs a) {
       d[f0 * static_cast<int64_t>(a.n_jobs)] = h.u;
       d[(f0 + 1) * static_cast<int64_t>(a.n_jobs)] = h.pu;
     }
-    turn_forward_pair(h, a, T0, o, even, j, write, 0, false);
+    turn_forward_pair<false>(h, a, T0, o, even, write, nullptr);
   }
   if (write) {
     if (ck && a.turns % a.ck == 0) {
@@ -980,7 +993,7 @@ __global__ void diff_tape_pair(DiffArgs a, int sg0, int G) {
   // the longer count; lanes past their own segment end do not write
   const int tmax = __reduce_max_sync(ALL_LANES, t1 - t0);
   for (int k = 0; k < tmax; ++k)
-    turn_forward_pair(h, a, T0, o, even, j, write && k < t1 - t0, g * a.ck + k, true);
+    turn_forward_pair<true>(h, a, T0, o, even, write && k < t1 - t0, tape_turn(a, g * a.ck + k, j));
 }
 
 __global__ void diff_reverse_plain_pair(DiffArgs a, int sg0, int sg_hi) {
@@ -1008,6 +1021,356 @@ __global__ void diff_reverse_plain_pair(DiffArgs a, int sg0, int sg_hi) {
   }
 }
 
+// ---------------------------------------------------------------- eight lanes
+// Tangent mode runs every job on eight lanes: plane (as the pairs above) x
+// column of the 4x4 tangent; the state is carried by all four column lanes.
+// The few jobs of an optics evaluation (three momenta per row) leave the GPU
+// empty, so a turn's time is one lane's FP64 instructions: per kick of order M
+// 75 with a job per lane, 28 with eight lanes (M = 6).  Measured on one GB300,
+// 1,024-element ring with errors, 3 jobs, per turn: forward 7.9 -> 3.6 ms, taped
+// forward and reverse 21.7 -> 10.1 ms.
+struct Oct {
+  double u, pu;  // this plane's coordinates (or their cotangents)
+  double tu, tp; // this plane's two tangent rows in this lane's column
+};
+
+struct OctLane {
+  bool even, write;  // plane; the lane's results are kept
+  int col, j;
+  double *tape;      // this lane's first entry of the turn
+};
+
+// this turn's tape entry of kick 0, field 0
+__device__ __forceinline__ double *oct_tape(const DiffArgs &a, int tt, int j) {
+  return a.tape + tidx(a, tt, 0, 0, 10, j);
+}
+
+// fields of a slot: x, y, T rows x and y (or, in a thick element's second slot,
+// px, py and their rows)
+__device__ __forceinline__ void oct_put(double *t, const OctLane &l, double v, double tv) {
+  if (!l.write) return;
+  if (l.col == 0) t[(l.even ? 0 : 1) * TLANES] = v;
+  t[((l.even ? 2 : 6) + l.col) * TLANES] = tv;
+}
+
+__device__ __forceinline__ void oct_drift(Oct &s, double L) {
+  s.u = fma(s.pu, L, s.u);
+  s.tu = fma(s.tp, L, s.tu);
+}
+
+// a kick element; MM: its number of terms (0: M, at run time)
+template <int MM, bool TAPE>
+__device__ __forceinline__ void kick_elem_oct(Oct &s, const double *c, int M, bool tp, int N,
+                                              double oo, const OctLane &l, double *&tape) {
+  const bool even = l.even;
+  constexpr int R = MM > 0 ? MM : 1;
+  double cf[R];
+#pragma unroll
+  for (int n = 0; n < R; ++n) cf[n] = __ldg(c + KHDR + (even ? 0 : M) + n);
+  const double Lo = __ldg(c), Li = __ldg(c + 1), W = __ldg(c + 2), Lx = __ldg(c + 5);
+  const double so = even ? neg(oo) : oo, sw = even ? neg(W) : 0.0;
+  const bool weak = tp && nonzero(W);
+  if (tp) oct_drift(s, Lo);
+  for (int sl = 0; sl < N; ++sl) {
+    if (TAPE) {
+      oct_put(tape, l, s.u, s.tu);
+      tape += 10 * TLANES;
+    }
+    const double w = other(s.u), ot = other(s.tu);
+    const double x = even ? s.u : w, sy = even ? neg(w) : s.u;
+    double s0, s1;
+    if (MM > 0) {
+      s0 = cf[R - 1];
+      s1 = 0.0;
+#pragma unroll
+      for (int n = R - 2; n >= 0; --n) {
+        const double o0 = other(s0), o1 = other(s1);
+        s1 = fma(o1, sy, fma(s1, x, s0));
+        s0 = fma(o0, sy, fma(s0, x, cf[n]));
+      }
+    } else {
+      series_pair<1>(c + KHDR, M, x, sy, even, s0, s1);
+    }
+    s1 *= oo;
+    s.pu = fma(so, s0, s.pu);
+    const double o1 = other(s1);
+    s.tp = fma(even ? o1 : s1, ot, fma(even ? neg(s1) : o1, s.tu, s.tp));
+    if (weak) {
+      s.pu = fma(sw, s.u, s.pu);
+      s.tp = fma(sw, s.tu, s.tp);
+    }
+    if (tp) oct_drift(s, sl < N - 1 ? Li : Lx);
+  }
+}
+
+template <bool TAPE>
+__device__ void turn_forward_oct(Oct &s, const DiffArgs &a, const double *T0, double o,
+                                 const OctLane &l, double *tape) {
+  const bool even = l.even;
+  DOp next = fetch(a.ops);
+  for (int i = 0; i < a.n_ops; ++i) {
+    const DOp op = next;
+    if (i + 1 < a.n_ops) next = fetch(a.ops + i + 1);
+    const double *c = T0 + op.toff;
+    const double oo = op.achro ? 1.0 : o;
+    switch (op.kind) {
+      case D_DRIFT:
+        oct_drift(s, __ldg(c));
+        break;
+      case D_ALIGN:
+        s.u -= __ldg(c + (even ? 0 : 1));
+        break;
+      case D_EDGE: {
+        const double curv = __ldg(c) * oo;
+        const double e = even ? __ldg(c + 1) : neg(edge_t2(op.flags, c, curv));
+        s.pu = fma(s.u * curv, e, s.pu);
+        s.tp = fma(s.tu * curv, e, s.tp);
+        break;
+      }
+      case D_KICK:
+      case D_TEAPOT: {
+        const bool tp = op.kind == D_TEAPOT;
+        const int N = tp ? op.N : 1;
+        switch (op.M) {  // common orders: coefficients in registers
+          case 1: kick_elem_oct<1, TAPE>(s, c, op.M, tp, N, oo, l, tape); break;
+          case 2: kick_elem_oct<2, TAPE>(s, c, op.M, tp, N, oo, l, tape); break;
+          case 3: kick_elem_oct<3, TAPE>(s, c, op.M, tp, N, oo, l, tape); break;
+          case 4: kick_elem_oct<4, TAPE>(s, c, op.M, tp, N, oo, l, tape); break;
+          case 5: kick_elem_oct<5, TAPE>(s, c, op.M, tp, N, oo, l, tape); break;
+          case 6: kick_elem_oct<6, TAPE>(s, c, op.M, tp, N, oo, l, tape); break;
+          default: kick_elem_oct<0, TAPE>(s, c, op.M, tp, N, oo, l, tape); break;
+        }
+        break;
+      }
+      case D_THICK: {
+        const double L = __ldg(c), k1 = __ldg(c + 1), h = __ldg(c + 2);
+        if (TAPE) {
+          oct_put(tape, l, s.u, s.tu);
+          oct_put(tape + 10 * TLANES, l, s.pu, s.tp);
+          tape += THICK_SLOTS * 10 * TLANES;
+        }
+        const double K = even ? oo * fma(h, h, k1) : -oo * k1;
+        const double disp = (even && (op.flags & DT_BEND)) ? (1.0 / o - 1.0) * h * oo : 0.0;
+        double C, Sw, D1, dC, dSw, dD1;
+        thick_fns<false>(K, L, C, Sw, D1, dC, dSw, dD1);
+        const double A = -K * Sw, u0 = s.u, t0 = s.tu;
+        s.u = fma(C, u0, fma(Sw, s.pu, disp * D1));
+        s.pu = fma(A, u0, fma(C, s.pu, disp * Sw));
+        s.tu = fma(C, t0, Sw * s.tp);
+        s.tp = fma(A, t0, C * s.tp);
+        break;
+      }
+      default:
+        break;
+    }
+  }
+}
+
+// sum over the four columns; every lane gets it
+__device__ __forceinline__ double oct_sum(double v) {
+  v += __shfl_xor_sync(ALL_LANES, v, 2);
+  return v + __shfl_xor_sync(ALL_LANES, v, 4);
+}
+
+// reverse of one turn from the tape that turn_forward_oct<true> wrote
+__device__ void turn_reverse_oct(Oct &b, const DiffArgs &a, const double *T0, double o,
+                                 const OctLane &l, const double *tape) {
+  const bool even = l.even;
+  tape += static_cast<int64_t>(a.kicks_per_turn) * 10 * TLANES;
+  const bool keeps = l.write && even && l.col == 0;  // the lane that owns the sums
+  DOp next = a.n_ops > 0 ? fetch(a.ops + a.n_ops - 1) : DOp{};
+  for (int i = a.n_ops - 1; i >= 0; --i) {
+    const DOp op = next;
+    if (i > 0) next = fetch(a.ops + i - 1);
+    const double *c = T0 + op.toff;
+    const double oo = op.achro ? 1.0 : o;
+    switch (op.kind) {
+      case D_DRIFT:
+        b.pu = fma(b.u, __ldg(c), b.pu);
+        b.tp = fma(b.tu, __ldg(c), b.tp);
+        break;
+      case D_ALIGN:
+        break;  // translation: cotangents unchanged
+      case D_EDGE: {
+        const double curv = __ldg(c) * oo;
+        const double e = even ? __ldg(c + 1) : neg(edge_t2(op.flags, c, curv));
+        b.u = fma(b.pu * curv, e, b.u);
+        b.tu = fma(b.tp * curv, e, b.tu);
+        break;
+      }
+      case D_KICK:
+      case D_TEAPOT: {
+        const bool tp = op.kind == D_TEAPOT;
+        const int N = tp ? op.N : 1;
+        const double Lo = __ldg(c), Li = __ldg(c + 1), W = __ldg(c + 2), Lx = __ldg(c + 5);
+        const double sw = even ? neg(W) : 0.0;
+        const bool weak = tp && nonzero(W);
+        const int pm = op.pslot >= 0 ? op.pm : -1;
+        const double *coef = c + KHDR + (even ? 0 : op.M);
+        double g0 = 0.0, g1 = 0.0;
+        for (int sl = N - 1; sl >= 0; --sl) {
+          tape -= 10 * TLANES;
+          const double x = tape[0], y = tape[TLANES];
+          const double dx = tape[(2 + l.col) * TLANES], dy = tape[(6 + l.col) * TLANES];
+          if (tp) {
+            const double L = sl < N - 1 ? Li : Lx;
+            b.pu = fma(b.u, L, b.pu);
+            b.tp = fma(b.tu, L, b.tp);
+          }
+          if (weak) {
+            b.u = fma(sw, b.pu, b.u);
+            b.tu = fma(sw, b.tp, b.tu);
+          }
+          // this lane's parts of S, S', S''/2 (series<2>)
+          const double sy = even ? neg(y) : y;
+          double s0 = __ldg(coef + op.M - 1), s1 = 0.0, s2 = 0.0;
+          for (int n = op.M - 2; n >= 0; --n) {
+            const double o0 = other(s0), o1 = other(s1), o2 = other(s2);
+            s2 = fma(o2, sy, fma(s2, x, s1));
+            s1 = fma(o1, sy, fma(s1, x, s0));
+            s0 = fma(o0, sy, fma(s0, x, __ldg(coef + n)));
+          }
+          s1 *= oo;
+          s2 *= 2.0 * oo;
+          const double o1 = other(s1), o2 = other(s2);
+          const double A = even ? neg(s1) : o1, B = even ? o1 : s1;    // -+a1, b1
+          const double A2 = even ? s2 : o2, B2 = even ? o2 : neg(s2);  // a2, +-b2
+          const double w = other(b.pu), wt = other(b.tp);
+          const double sum = oct_sum(fma(even ? neg(b.tp) : b.tp, dx, wt * dy));  // Ab | Bb
+          const double osum = other(sum);
+          if (pm >= 0) {
+            const double pxb = even ? b.pu : w, pyb = even ? w : b.pu;
+            double zr, zi;
+            zpow_small(x, y, pm, zr, zi);
+            g0 += oo * fma(-pxb, zr, pyb * zi);
+            if (pm >= 1) {
+              const double Ab = even ? sum : osum, Bb = even ? osum : sum;
+              zpow_small(x, y, pm - 1, zr, zi);
+              g1 += oo * fma(Ab, zr, Bb * zi);
+            }
+          }
+          b.u = fma(w, B, fma(b.pu, A, b.u));
+          b.tu = fma(wt, B, fma(b.tp, A, b.tu));
+          b.u = fma(osum, B2, fma(sum, A2, b.u));
+        }
+        if (tp) {
+          b.pu = fma(b.u, Lo, b.pu);
+          b.tp = fma(b.tu, Lo, b.tp);
+        }
+        if (op.pslot >= 0 && keeps) {
+          double &p = a.pbar[static_cast<int64_t>(op.pslot) * a.n_jobs + l.j];
+          p = fma(g0, __ldg(c + 3), fma(g1, __ldg(c + 4), p));
+        }
+        break;
+      }
+      case D_THICK: {
+        const double L = __ldg(c), k1 = __ldg(c + 1), h = __ldg(c + 2);
+        tape -= THICK_SLOTS * 10 * TLANES;
+        const double *t1 = tape + 10 * TLANES;
+        const int v = (even ? 0 : 1) * TLANES, r = ((even ? 2 : 6) + l.col) * TLANES;
+        const double q = tape[v], pq = t1[v], tq = tape[r], tpq = t1[r];
+        const double K = even ? oo * fma(h, h, k1) : -oo * k1;
+        const double disp = (even && (op.flags & DT_BEND)) ? (1.0 / o - 1.0) * h * oo : 0.0;
+        double C, Sw, D1, dC, dSw, dD1;
+        thick_fns<true>(K, L, C, Sw, D1, dC, dSw, dD1);
+        const double A = -K * Sw, dA = fma(-K, dSw, -Sw);
+        double Kb = fma(b.u, fma(dC, q, fma(dSw, pq, disp * dD1)),
+                        b.pu * fma(dA, q, fma(dC, pq, disp * dSw)));
+        Kb += oct_sum(fma(b.tu, fma(dC, tq, dSw * tpq), b.tp * fma(dA, tq, dC * tpq)));
+        const double bu = b.u, bt = b.tu;
+        b.u = fma(C, bu, A * b.pu);
+        b.pu = fma(Sw, bu, C * b.pu);
+        b.tu = fma(C, bt, A * b.tp);
+        b.tp = fma(Sw, bt, C * b.tp);
+        const double ko = other(Kb);
+        if (op.pslot >= 0 && keeps) {  // dK_x/dk1 = o, dK_y/dk1 = -o
+          double &p = a.pbar[static_cast<int64_t>(op.pslot) * a.n_jobs + l.j];
+          p = fma(oo, Kb - ko, p);
+        }
+        break;
+      }
+      default:
+        break;
+    }
+  }
+}
+
+__device__ __forceinline__ OctLane oct_lane(const DiffArgs &a) {
+  const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t job = t >> 3;
+  OctLane l;
+  l.even = (t & 1) == 0;
+  l.col = static_cast<int>(t >> 1) & 3;
+  l.write = job < a.n_jobs;  // lanes past the end run along on the last job
+  l.j = static_cast<int>(l.write ? job : a.n_jobs - 1);
+  return l;
+}
+
+// the rows of this lane in a [4 coordinates][16 tangent entries] record with
+// `n` between entries
+__device__ __forceinline__ void oct_save(const Oct &s, const OctLane &l, double *d, int64_t n) {
+  if (!l.write) return;
+  if (l.col == 0) {
+    d[(l.even ? 0 : 2) * n] = s.u;
+    d[(l.even ? 1 : 3) * n] = s.pu;
+  }
+  d[(4 + (l.even ? 0 : 8) + l.col) * n] = s.tu;
+  d[(4 + (l.even ? 4 : 12) + l.col) * n] = s.tp;
+}
+
+__global__ void __launch_bounds__(32) diff_forward_oct(DiffArgs a) {
+  const OctLane l = oct_lane(a);
+  Oct s;
+  s.u = a.z0[4 * l.j + (l.even ? 0 : 2)];
+  s.pu = a.z0[4 * l.j + (l.even ? 1 : 3)];
+  s.tu = l.col == (l.even ? 0 : 2) ? 1.0 : 0.0;
+  s.tp = l.col == (l.even ? 1 : 3) ? 1.0 : 0.0;
+  const double o = a.o[l.j];
+  const double *T0 = a.tab + (a.seed ? static_cast<int64_t>(a.seed[l.j]) : 0) * a.tab_stride;
+  const int64_t J = a.n_jobs;
+  for (int t = 0; t < a.turns; ++t) {
+    if (a.ckpt && t % a.ck == 0)
+      oct_save(s, l, a.ckpt + static_cast<int64_t>(t / a.ck) * 20 * J + l.j, J);
+    turn_forward_oct<false>(s, a, T0, o, l, nullptr);
+  }
+  if (a.ckpt && a.turns % a.ck == 0)
+    oct_save(s, l, a.ckpt + static_cast<int64_t>(a.turns / a.ck) * 20 * J + l.j, J);
+  oct_save(s, l, a.zT + 20 * static_cast<int64_t>(l.j), 1);
+}
+
+__global__ void __launch_bounds__(32) diff_reverse_oct(DiffArgs a) {
+  const OctLane l = oct_lane(a);
+  const double o = a.o[l.j];
+  const double *T0 = a.tab + (a.seed ? static_cast<int64_t>(a.seed[l.j]) : 0) * a.tab_stride;
+  const int64_t J = a.n_jobs;
+  if (l.write)
+    for (int k = threadIdx.x & 7; k < a.n_params; k += 8) a.pbar[k * J + l.j] = 0.0;
+  Oct b;
+  b.u = a.zbar[4 * l.j + (l.even ? 0 : 2)];
+  b.pu = a.zbar[4 * l.j + (l.even ? 1 : 3)];
+  b.tu = a.Tbar[16 * static_cast<int64_t>(l.j) + (l.even ? 0 : 8) + l.col];
+  b.tp = a.Tbar[16 * static_cast<int64_t>(l.j) + (l.even ? 4 : 12) + l.col];
+  __syncwarp();
+  for (int sg = (a.turns - 1) / a.ck; sg >= 0; --sg) {
+    const int t0 = sg * a.ck, t1 = min(a.turns, t0 + a.ck);
+    const double *d = a.ckpt + static_cast<int64_t>(sg) * 20 * J + l.j;
+    Oct s;
+    s.u = d[(l.even ? 0 : 2) * J];
+    s.pu = d[(l.even ? 1 : 3) * J];
+    s.tu = d[(4 + (l.even ? 0 : 8) + l.col) * J];
+    s.tp = d[(4 + (l.even ? 4 : 12) + l.col) * J];
+    for (int t = t0; t < t1; ++t)
+      turn_forward_oct<true>(s, a, T0, o, l, oct_tape(a, t - t0, l.j));
+    __syncwarp();  // the tape's entries are read by other lanes than wrote them
+    for (int t = t1 - 1; t >= t0; --t) turn_reverse_oct(b, a, T0, o, l, oct_tape(a, t - t0, l.j));
+    __syncwarp();
+  }
+  if (l.write && l.col == 0) {
+    a.zbar0[4 * l.j + (l.even ? 0 : 2)] = b.u;
+    a.zbar0[4 * l.j + (l.even ? 1 : 3)] = b.pu;
+  }
+}
+
 }  // namespace ufo_diff
 
 // ---------------------------------------------------------------- C ABI
@@ -1030,6 +1393,16 @@ static void prefer_l1() {
   cudaFuncSetAttribute(ufo_diff::diff_reverse_plain_pair,
                        cudaFuncAttributePreferredSharedMemoryCarveout, 0);
   done = true;
+}
+
+// Eight lanes per job while their warps are at most two per sub-partition: two
+// queue for the FP64 pipe in the time the one-lane form's single warp takes.
+static bool oct_lanes_pay(int n_jobs) {
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+    return false;
+  return n_jobs <= 32 * sms;
 }
 
 int ufo_diff_forward(const int32_t *ops, int n_ops, const double *tab, int64_t tab_stride,
@@ -1057,7 +1430,9 @@ int ufo_diff_forward(const int32_t *ops, int n_ops, const double *tab, int64_t t
   a.zT = zT;
   const int tpb = 32;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (tangent) {
+  if (tangent && oct_lanes_pay(n_jobs)) {
+    ufo_diff::diff_forward_oct<<<(n_jobs + 3) / 4, tpb, 0, st>>>(a);
+  } else if (tangent) {
     ufo_diff::diff_forward<<<(n_jobs + tpb - 1) / tpb, tpb, 0, st>>>(a);
   } else {  // two lanes per job
     const int64_t threads = 2 * static_cast<int64_t>(n_jobs);
@@ -1098,7 +1473,10 @@ int ufo_diff_reverse(const int32_t *ops, int n_ops, const double *tab, int64_t t
   const int tpb = 32;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (tangent) {
-    ufo_diff::diff_reverse<<<(n_jobs + tpb - 1) / tpb, tpb, 0, st>>>(a);
+    if (oct_lanes_pay(n_jobs))
+      ufo_diff::diff_reverse_oct<<<(n_jobs + 3) / 4, tpb, 0, st>>>(a);
+    else
+      ufo_diff::diff_reverse<<<(n_jobs + tpb - 1) / tpb, tpb, 0, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
   // plain mode: groups of up to tape_segments segments, last group first

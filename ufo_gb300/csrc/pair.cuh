@@ -437,7 +437,10 @@ UFO_DEV void thick_apply(Half &h, const double *t, int64_t n, bool bend, bool &b
   const bool zero = ((hi & 0x7fffffff) | __double2loint(a)) == 0;
   const bool drift = (__double2hiint(k) & 0x7fffffff) == 0;
   bad = bad || __double2hiint(r) == 0 || (!zero && e - 0x1f000000u > 0x60f00000u - 0x1f000000u);
-  const double q = div_prepared(a, drift ? 1.0 : fabs(k), r, z);
+  // |k| by its sign bit (an FP64 instruction otherwise)
+  const double d = __hiloint2double(drift ? 0x3ff00000 : __double2hiint(k) & 0x7fffffff,
+                                    __double2loint(k));
+  const double q = div_prepared(a, d, r, z);
   double u = add(mul(C, h.u), q);
   double pu = add(mul(mul(S, h.u), k), mul(C, h.pu));
   if (bend) {

@@ -190,7 +190,7 @@ class DiffProgram:
                     # ufo/methods.py:199-211)
                     ops.append([D_EDGE, DE_RTPSI, len(tab), 0, 0, -1, 0, achro])
                     tab += [c(0), c(1) if fl & C.F_T1 else 0.0, c(2), c(3), c(4), c(5)]
-                else:
+                elif fl & (C.F_T1 | C.F_T2):  # without face angles it does nothing
                     ops.append([D_EDGE, 0, len(tab), 0, 0, -1, 0, achro])
                     tab += [c(0), c(1) if fl & C.F_T1 else 0.0, c(2) if fl & C.F_T2 else 0.0]
             elif kind in (C.OP_TEAPOT, C.OP_KICK):
@@ -405,6 +405,7 @@ def closed_orbits(engine, dps, z0=None, max_iter=30, seed=None):
     z = np.zeros((n, 4)) if z0 is None else np.array(z0, np.float64)
     best = np.full(n, np.inf)
     zbest = z.copy()
+    Jbest = np.full((n, 4, 4), np.nan)  # the Jacobian at the best iterate
     active = np.ones(n, bool)  # per-job stopping: a job's iterates do not depend on the batch
     for _ in range(max_iter):
         out, _ = engine.forward(z, o, 1, tangent=True, seed=seed)
@@ -415,13 +416,16 @@ def closed_orbits(engine, dps, z0=None, max_iter=30, seed=None):
         better = active & (nrm < best)
         best = np.where(better, nrm, best)
         zbest[better] = z[better]
+        Jbest[better] = J[better]
         active = better & (nrm > 0)
         if not np.any(active):
             break
         dz = np.zeros_like(z)
         dz[active] = np.linalg.solve(J[active] - np.eye(4)[None], -res[active, :, None])[:, :, 0]
         z = np.where(active[:, None], z + dz, z)
-    # the Jacobian at the final iterate
+    if np.all(np.isfinite(best)):
+        return zbest, Jbest, best
+    # a job that never improved keeps its start, whose Jacobian is taken there
     out, _ = engine.forward(zbest, o, 1, tangent=True, seed=seed)
     return zbest, out[:, 4:].reshape(n, 4, 4), best
 
