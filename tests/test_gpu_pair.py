@@ -211,3 +211,26 @@ def test_closed_orbits_of_lane_pairs_are_the_one_thread_searchs(name, n):
         got = orbits(start, seed, steps)
         ref = orbits(np.tile(start, (reps, 1)), np.tile(seed, reps), steps)[:n]
         assert np.array_equal(got, ref, equal_nan=True)
+
+
+@pytest.mark.parametrize('name', ['c1', 'alba_thick', 'mixed'])
+@pytest.mark.parametrize('n,turns', [(152 * 8 * 16 + 1, 2), (40_000, 5), (50_001, 37)])
+def test_time_slices_give_whole_runs(name, n, turns):
+    """Launches of more particles than stay resident are cut into slices of
+    turns; every particle, special values and observations included, ends as in
+    the plain kernel."""
+    import ufo_gb300 as u
+    from ufo_gb300 import capi, compiler as C
+    line, flags = _rings()[name]
+    if name == 'alba_thick' and turns > 5:
+        turns = 3
+    ctx = u.context(0)
+    coords = np.concatenate([_special(333), _beam(n - 333, 3.0)])
+    seed = np.zeros(n, np.int32)
+    for fma in (0, u.FMA):
+        dp = capi.DeviceProgram(ctx, C.compile_line(line, flags | fma, where=[2, -1]))
+        tf = capi.UFO_TRACK_FMA if fma else 0
+        out = [capi.track(ctx, dp, coords, turns, capi.UFO_MODE_TRACK, tf | f, seed=seed,
+                          slots=2 * (turns // 2), every=2)
+               for f in (capi.UFO_TRACK_PLAIN, 0)]
+        assert _same(*out), fma

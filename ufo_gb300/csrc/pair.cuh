@@ -40,6 +40,7 @@ struct PairCtx {
   double o;       // 1 / (1 + dp)
   const double *tab;
   int neg;        // sign bit on even lanes: a - b as a + (b ^ neg)
+  int group;      // the warp's lanes of the coefficient cache
   bool even;
   bool dead;      // no particle, or all four coordinates are NaN (they stay NaN)
   bool bad_o;     // o is not finite
@@ -418,8 +419,9 @@ __device__ __noinline__ void thick_bend_half(double o, double dp, int flags, con
   thick_put(t, out, n, true);
 }
 
-UFO_DEV double *pair_cache(const TrackArgs &a, int field) {
-  return a.cache + field * a.cache_lanes + static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
+// this lane's entry of a cache field; `group`: the warp's 32 lanes of the cache
+UFO_DEV double *pair_cache(const TrackArgs &a, int field, int group) {
+  return a.cache + field * a.cache_lanes + static_cast<int64_t>(group) * 32 + threadIdx.x;
 }
 
 // tan(psi) of a fringe-field edge (edge in ops.cuh)
@@ -505,7 +507,7 @@ UFO_DEV PairOp pair_fetch(const int4 *w) {
 }
 
 // A particle's first turn in a launch: its coefficient-cache fields.
-__device__ __noinline__ void pair_fill(const TrackArgs &a, const PairShared &sh) {
+__device__ __noinline__ void pair_fill(const TrackArgs &a, const PairShared &sh, int group) {
   const int lane = threadIdx.x;
   const bool even = (lane & 1) == 0;
   const int64_t p = sh.p[lane];
@@ -516,7 +518,7 @@ __device__ __noinline__ void pair_fill(const TrackArgs &a, const PairShared &sh)
     if (variant == PV_SEGMENT && op.b <= op.a) return;
     if (!(op.head & PF_FILL)) continue;
     const double *c = sh.tab[lane] + op.toff;
-    double *t = pair_cache(a, op.a);
+    double *t = pair_cache(a, op.a, group);
     if (variant == PV_THICKQ) {
       thick_quad_half(o, op.head, c, t, a.cache_lanes);
     } else if (variant == PV_THICKB) {
@@ -593,16 +595,16 @@ UFO_DEV int pair_run(Half &h, const PairCtx &x, int &pos, int &first, int &last,
       }
       case PV_EDGE_PSI: {
         const double curv = (op.head & PF_ACHRO) ? c0 : mul(c0, x.o);
-        const double T = *pair_cache(a, op.a);
+        const double T = *pair_cache(a, op.a, x.group);
         h.pu = add(h.pu, mul(mul(h.u, curv), T));
         bad = bad || nf(curv);
         break;
       }
       case PV_THICKQ:
-        thick_apply(h, pair_cache(a, op.a), a.cache_lanes, false, bad);
+        thick_apply(h, pair_cache(a, op.a, x.group), a.cache_lanes, false, bad);
         break;
       case PV_THICKB:
-        thick_apply(h, pair_cache(a, op.a), a.cache_lanes, true, bad);
+        thick_apply(h, pair_cache(a, op.a, x.group), a.cache_lanes, true, bad);
         break;
       case PV_CIRCLE: {
         const double s = mul(h.u, h.u);
@@ -676,7 +678,7 @@ UFO_DEV void pair_prepare(PairCtx &x, const TrackArgs &a, PairShared &sh, bool f
   const int lane = threadIdx.x;
   sh.o[lane] = x.o;
   sh.tab[lane] = x.tab;
-  if (fresh) pair_fill(a, sh);
+  if (fresh) pair_fill(a, sh, x.group);
   __syncwarp();
   x.o = sh.o[lane];
   x.tab = sh.tab[lane];
@@ -718,6 +720,27 @@ UFO_DEV void pair_idle(PairCtx &x, const TrackArgs &a) {
   x.tab = a.table;
 }
 
+// this turn's observation slots of the lane's particle
+UFO_DEV void pair_slots(const TrackArgs &a, PairShared &sh, bool idle) {
+  const int lane = threadIdx.x, turn = sh.turn[lane];
+  sh.obs_left[lane] = 0;
+  if (a.tracks && !idle && (turn + 1) % a.every == 0) {
+    const int64_t slot = static_cast<int64_t>((turn + 1) / a.every - 1) * a.n_dumps;
+    sh.obs[lane] = a.tracks + (sh.p[lane] * a.slots + slot) * 6;
+    sh.obs_left[lane] = a.slots - slot;
+  }
+}
+
+// the loss test (is_lost) of the lane's particle: isnan(x), or |x| > 1, |y| > 1
+UFO_DEV bool pair_lost(const Half &h, bool even, int mode) {
+  bool out;
+  if (mode == UFO_MODE_TRACK)
+    out = even && isnan(h.u);
+  else
+    out = fabs(h.u) > 1. || (even && isnan(h.u));
+  return ((__ballot_sync(PAIR_ALL, out) >> (threadIdx.x & 30)) & 3u) != 0u;
+}
+
 // The persistent loop of track_kernel with 16 particles per warp: pairs whose
 // particle finished refill from the work counter at turn boundaries.
 template <bool FMA>
@@ -728,6 +751,7 @@ __global__ void __launch_bounds__(32, 16) track_pair_kernel(const __grid_constan
   PairCtx x{};
   x.even = (lane & 1) == 0;
   x.neg = x.even ? static_cast<int>(0x80000000u) : 0;
+  x.group = blockIdx.x;
   pair_idle(x, a);
   sh.p[lane] = PAIR_NONE;
   Half h{0.0, 0.0};
@@ -770,24 +794,11 @@ __global__ void __launch_bounds__(32, 16) track_pair_kernel(const __grid_constan
     }
     if (__all_sync(PAIR_ALL, idle)) break;
     if (idle) h.u = h.pu = 0.0;  // idle lanes run along on a finite state
-    const int64_t p = sh.p[lane];
-    const int turn = sh.turn[lane];
-    sh.obs_left[lane] = 0;
-    if (a.tracks && !idle && (turn + 1) % a.every == 0) {
-      const int64_t slot = static_cast<int64_t>((turn + 1) / a.every - 1) * a.n_dumps;
-      sh.obs[lane] = a.tracks + (p * a.slots + slot) * 6;
-      sh.obs_left[lane] = a.slots - slot;
-    }
+    pair_slots(a, sh, idle);
     const bool any_bad_o = __any_sync(PAIR_ALL, x.bad_o);
     if (__any_sync(PAIR_ALL, fresh)) pair_prepare(x, a, sh, fresh);
     pair_turn<FMA>(h, x, a, sh, any_bad_o);
-    // loss test (is_lost): isnan(x), or |x| > 1, |y| > 1
-    bool out;
-    if (a.mode == UFO_MODE_TRACK)
-      out = x.even && isnan(h.u);
-    else
-      out = fabs(h.u) > 1. || (x.even && isnan(h.u));
-    const bool lost = ((__ballot_sync(PAIR_ALL, out) >> (lane & 30)) & 3u) != 0u;
+    const bool lost = pair_lost(h, x.even, a.mode);
     fresh = false;
     if (!idle) {
       const int t = sh.turn[lane] + (lost ? 0 : 1);
@@ -799,6 +810,130 @@ __global__ void __launch_bounds__(32, 16) track_pair_kernel(const __grid_constan
         pair_idle(x, a);
       }
     }
+  }
+}
+
+// ---------------------------------------------------------------- time slices
+// A launch of more warps' worth of particles than stay resident, all with the
+// same turns, ends unevenly: the work counter hands out whole runs, so after
+// the first round of resident warps each SM sub-partition holds anything from
+// none to four of the rest, and the fullest sets the time.  The sliced kernels
+// hand out (slice of turns, group of particles) instead, slice by slice, so a
+// sub-partition that is ahead takes more slices and all finish together.
+// A group's state rests in the output arrays between its slices: coordinates in
+// `final`, turns so far in `lost` with the top bit set while it runs.  Its word
+// in `claims` counts the slices handed out and not yet run (low half) and those
+// run (high half).  Whoever raises the low half from 0 runs the group; a warp
+// that finds it raised leaves the slice to that runner, which goes on until the
+// count is back at 0.  So no warp waits for another, and every slice runs once,
+// in order.  The last slice runs to the end whatever its length.
+struct Slices {
+  unsigned long long *claims;  // [groups], zero at launch
+  int groups, count, turns;    // slices per group, turns per slice
+};
+
+// The group of the next slice that this warp may run, or -1 when all are handed
+// out; `done`: the group's slices run so far.
+UFO_DEV int slice_take(const Slices &s, unsigned long long *queue, int &done) {
+  const unsigned all = 0xffffffffu;
+  const unsigned long long total = static_cast<unsigned long long>(s.groups) * s.count;
+  while (true) {
+    unsigned long long t = 0, old = 0;
+    if ((threadIdx.x & 31) == 0) {
+      t = atomicAdd(queue, 1ull);
+      if (t < total) old = atomicAdd(s.claims + t % s.groups, 1ull);
+    }
+    t = __shfl_sync(all, t, 0);
+    old = __shfl_sync(all, old, 0);
+    if (t >= total) return -1;
+    if ((old & 0xffffffffull) == 0) {
+      __threadfence();  // the state that the last runner left
+      done = static_cast<int>(old >> 32);
+      return static_cast<int>(t % s.groups);
+    }
+  }
+}
+
+// A slice of `group` has run: true when another was handed out meanwhile.
+UFO_DEV bool slice_more(const Slices &s, int group, int &done) {
+  __threadfence();
+  __syncwarp();
+  unsigned long long old = 0;
+  if ((threadIdx.x & 31) == 0) old = atomicAdd(s.claims + group, (1ull << 32) - 1ull);
+  old = __shfl_sync(0xffffffffu, old, 0);
+  ++done;
+  return (old & 0xffffffffull) > 1;
+}
+
+constexpr uint32_t SLICE_RUNNING = 0x80000000u;
+
+template <bool FMA>
+__global__ void __launch_bounds__(32, 16)
+    track_pair_sliced(const __grid_constant__ TrackArgs a, const Slices s) {
+  __shared__ PairShared sh;
+  const int lane = threadIdx.x;
+  PairCtx x{};
+  x.even = (lane & 1) == 0;
+  x.neg = x.even ? static_cast<int>(0x80000000u) : 0;
+  int done, group;
+  while ((group = slice_take(s, a.queue, done)) >= 0) {
+    x.group = group;
+    do {
+      const int64_t p = static_cast<int64_t>(group) * 16 + lane / 2;
+      pair_idle(x, a);
+      sh.p[lane] = PAIR_NONE;
+      Half h{0.0, 0.0};
+      bool idle = true;
+      if (p < a.n) {
+        const int64_t sd = a.seed ? static_cast<int64_t>(a.seed[p]) : 0;
+        const uint32_t at = done ? __ldcg(a.lost + p) : SLICE_RUNNING;
+        if (sd < 0 || sd >= a.n_seeds) {  // seed outside the table: not tracked
+          if (!done && x.even) a.lost[p] = 0xffffffffu;
+        } else if (at & SLICE_RUNNING) {
+          idle = false;
+          const double *c = (done ? a.final_state : a.coords) + p * 6 + (x.even ? 0 : 2);
+          h.u = __ldcg(c);
+          h.pu = __ldcg(c + 1);
+          x.o = dvd(1., add(a.coords[p * 6 + 5], 1.));  // as load_particle: the same bits
+          x.bad_o = nf(x.o);
+          x.dead = false;
+          x.tab = a.table + sd * a.stride;
+          sh.p[lane] = p;
+          sh.turn[lane] = static_cast<int>(at & ~SLICE_RUNNING);
+        }
+      }
+      const bool mine = !idle;
+      const bool last = done == s.count - 1;
+      if (!done && __any_sync(PAIR_ALL, !idle)) pair_prepare(x, a, sh, !idle);
+      for (int k = 0; (last || k < s.turns) && __any_sync(PAIR_ALL, !idle); ++k) {
+        if (!mine) h.u = h.pu = 0.0;  // idle lanes run along on a finite state
+        if (!idle && sh.turn[lane] >= a.turns) idle = true;  // nothing to track
+        if (__all_sync(PAIR_ALL, idle)) break;
+        pair_slots(a, sh, idle);
+        const Half before = h;
+        pair_turn<FMA>(h, x, a, sh, __any_sync(PAIR_ALL, x.bad_o));
+        const bool lost = pair_lost(h, x.even, a.mode);
+        if (idle) {
+          h = before;  // a finished particle keeps its state
+        } else {
+          const int t = sh.turn[lane] + (lost ? 0 : 1);
+          sh.turn[lane] = t;
+          if (lost || t >= a.turns) {
+            idle = true;
+            x.dead = true;
+          }
+        }
+      }
+      if (mine) {
+        double *f = a.final_state + p * 6;
+        f[x.even ? 0 : 2] = h.u;
+        f[x.even ? 1 : 3] = h.pu;
+        if (!done) f[x.even ? 4 : 5] = a.coords[p * 6 + (x.even ? 4 : 5)];
+        if (x.even)
+          a.lost[p] = static_cast<uint32_t>(sh.turn[lane]) | (idle ? 0u : SLICE_RUNNING);
+      }
+      __syncwarp();
+    } while (slice_more(s, group, done));
   }
 }
 
@@ -826,6 +961,7 @@ __device__ __noinline__ double orbit_residual(double t0, double t1, const double
   x.neg = x.even ? static_cast<int>(0x80000000u) : 0;
   x.o = 1.0;
   x.tab = tab;
+  x.group = blockIdx.x;
   x.dead = x.bad_o = false;
   Half h{t0, t1};
   pair_turn<false>(h, x, a, sh, false);
@@ -848,6 +984,7 @@ __global__ void __launch_bounds__(32, 16)
   PairCtx x{};
   x.even = (lane & 1) == 0;
   x.neg = x.even ? static_cast<int>(0x80000000u) : 0;
+  x.group = blockIdx.x;
   sh.turn[lane] = 0;
   sh.obs_left[lane] = 0;
   const int64_t groups = (a.n + per_warp - 1) / per_warp;

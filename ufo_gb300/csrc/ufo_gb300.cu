@@ -761,6 +761,7 @@ struct ufo_prog {
   ufo::PairOp *pair_ops;
   std::vector<ufo::PairOp> host_pair_ops;
   bool pair_fma;               // also for FMA launches
+  bool pair_general;           // most kicks are general
   int cache_fields;            // doubles per lane of the coefficient cache
   mutable double *cache;       // [cache_fields][cache_lanes]
   mutable int64_t cache_lanes;
@@ -1016,11 +1017,12 @@ int kick_pattern(int nn, int ns, int32_t mn) {
 // that the FMA kernel reads.
 bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t stride, int n_seeds,
                  int most_fields, std::vector<ufo::PairOp> &out, int &cache_fields,
-                 bool &fma_ready) {
+                 bool &fma_ready, bool &mostly_general) {
   out.clear();
   out.reserve(static_cast<size_t>(n_ops) + n_ops / ufo::PAIR_SEGMENT + 4);
   cache_fields = 0;
   fma_ready = true;
+  int kicks = 0, general = 0;
   struct Shared { int op, field; };
   std::unordered_multimap<uint64_t, Shared> seen;  // constants' hash -> first op
   size_t head = 0;  // the current segment's header
@@ -1057,6 +1059,8 @@ bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t str
         const int32_t *k = w + (teapot ? 4 : 3);  // nn, ns, mn, ms
         const int pattern = (k[2] | k[3]) ? kick_pattern(k[0], k[1], k[2]) : 3;
         if (pattern == 0 && !(flags & ufo::F_PSER)) fma_ready = false;
+        ++kicks;
+        general += pattern == 0;
         if (teapot && (flags & (ufo::F_EXACT | ufo::F_YOSHIDA))) return false;
         if (teapot && (((flags >> ufo::SH_FOUTER) & 3) != ufo::DF_MUL ||
                        ((flags >> ufo::SH_FINNER) & 3) == ufo::DF_MUL2))
@@ -1160,6 +1164,7 @@ bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t str
   if (out[head].b > out[head].a) open(n_ops);  // the end
   out.push_back({ufo::PV_SEGMENT, 0, 0, 0});   // the kernel fetches two ops ahead
   out.push_back({ufo::PV_SEGMENT, 0, 0, 0});
+  mostly_general = 2 * general > kicks;
   return true;
 }
 
@@ -1199,8 +1204,8 @@ int64_t pair_warps(int64_t n, int sm_count, int warps_per_sm) {
 
 // The launch shared by every entry point: fill the kernel arguments and start
 // the persistent (or plain) kernel on `stream`; `queue` is the work counter.
-int launch_kernels(ufo::TrackArgs &a, bool full, bool pair, int sm_count, int warps_per_sm,
-                   cudaStream_t stream) {
+int launch_kernels(ufo::TrackArgs &a, bool full, bool pair, const ufo::Slices &slices,
+                   int sm_count, int warps_per_sm, cudaStream_t stream) {
   const bool fma = a.flags & UFO_TRACK_FMA;
   if (a.flags & UFO_TRACK_PLAIN) {
     const unsigned blocks = static_cast<unsigned>((a.n + 127) / 128);
@@ -1235,6 +1240,14 @@ int launch_kernels(ufo::TrackArgs &a, bool full, bool pair, int sm_count, int wa
     else
       full ? ufo::track_kernel_cta<false, true><<<g, tpb, smem, stream>>>(a)
            : ufo::track_kernel_cta<false, false><<<g, tpb, smem, stream>>>(a);
+  } else if (slices.groups) {
+    UFO_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), stream));
+    UFO_CUDA(cudaMemsetAsync(slices.claims, 0, sizeof(unsigned long long) * slices.groups, stream));
+    const unsigned g = static_cast<unsigned>(sm_count * warps_per_sm);
+    if (fma)
+      ufo::track_pair_sliced<true><<<g, 32, 0, stream>>>(a, slices);
+    else
+      ufo::track_pair_sliced<false><<<g, 32, 0, stream>>>(a, slices);
   } else if (pair) {
     UFO_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), stream));
     const unsigned g = static_cast<unsigned>(pair_warps(a.n, sm_count, warps_per_sm));
@@ -1304,6 +1317,9 @@ ufo::TrackArgs make_args(const ufo::Op *ops, int n_ops, const double *table, int
 //   particles 167 -> 69, 65,536 particles 475 -> 434; light-source ring (1,024)
 //   65,536 particles 5,352 -> 4,991; thick 768-element ring, 1,000 particles
 //   1,355 -> 357, 65,536 particles 4,481 -> 1,948.
+//   A ring with general error kicks on most magnets (a coefficient enters one
+//   lane's sum, so half its products are idle) gains up to 12 warps per SM:
+//   light-source ring with errors 1,000 particles 15,590 -> 8,480, 30,000 even.
 //  FMA: up to 12 warps per SM.  The sextupole form and the composed linear
 //   elements cost the two-lane code more instructions (6 for 5, 8 for 5 per 32
 //   particles), so the one-lane kernel wins once the pipe is full:
@@ -1312,7 +1328,7 @@ ufo::TrackArgs make_args(const ufo::Op *ops, int n_ops, const double *table, int
 //   442 -> 404, 65,536 826 -> 891.
 bool use_pair(const ufo_ctx *ctx, const ufo_prog *prog, int64_t n, int flags) {
   if (!prog->pair_ops || ((flags & UFO_TRACK_FMA) && !prog->pair_fma) || (flags & (UFO_TRACK_PLAIN | UFO_TRACK_COMPACT))) return false;
-  if (!(flags & UFO_TRACK_FMA)) return true;
+  if (!(flags & UFO_TRACK_FMA) && !prog->pair_general) return true;
   return (n + 15) / 16 <= 12 * static_cast<int64_t>(ctx->sm_count);
 }
 
@@ -1353,6 +1369,42 @@ void ensure_cache(const ufo_prog *prog, int64_t lanes, cudaStream_t stream) {
   prog->cache_lanes = lanes;
 }
 
+// Time slices (Slices in pair.cuh) for a two-lane launch of equal turns with
+// more groups than 8 warps per SM: as many warps as fill every sub-partition
+// evenly (a multiple of 4 per SM) and leave groups in hand.  Below that a
+// sub-partition's first and second warp hide each other's latency, so an uneven
+// second one costs nothing.  Measured (us per turn, strict, without -> with):
+// FODO ring 65,536 particles 434 -> 379, light-source ring 4,991 -> 4,259, thick
+// ring 1,948 -> 1,777, 30,000 particles of the FODO ring 182 -> 175.  The
+// one-lane kernel keeps whole runs: the 12 warps per SM that leave it groups in
+// hand cost it more than the even end gains (FMA, light-source ring 1,511 ->
+// 1,685).  Particles of a dynamic-aperture scan are lost early (the lane refill
+// serves them), and uneven turn counts run longest first.
+ufo::Slices plan_slices(const ufo_ctx *ctx, const ufo::TrackArgs &a, int &warps_per_sm) {
+  ufo::Slices s{};
+  const int64_t groups = (a.n + 15) / 16;
+  const int64_t most = std::min(16, 2 * warps_per_sm);
+  const int64_t w = std::min(most, (groups - 1) / ctx->sm_count) / 4 * 4;
+  const int64_t slots = static_cast<int64_t>(ctx->sm_count) * ufo::CTA_MAX_WARPS * 32;
+  if (a.mode != UFO_MODE_TRACK || a.pturns || !a.lost || !a.final_state || a.turns < 2 || w < 8 ||
+      groups > slots)
+    return s;
+  s.claims = ctx->pool_seq;  // one word per lane of the largest compacting grid
+  s.groups = static_cast<int>(groups);
+  // slice length: a launch ends within about half a slice (a share of Q / 2T),
+  // and each slice costs about 5 us of exchange against some 0.6 us per op and
+  // turn: the sum is least near Q = sqrt(16 T / ops)
+  s.turns = std::max(1, static_cast<int>(std::sqrt(16.0 * a.turns / std::max(1, a.n_ops))));
+  s.count = (a.turns + s.turns - 1) / s.turns;
+  warps_per_sm = static_cast<int>(w);
+  return s;
+}
+
+// lanes of the coefficient cache: per group where groups move between warps
+int64_t cache_lanes_for(const ufo_ctx *ctx, const ufo::Slices &s, int64_t n) {
+  return 32 * (s.groups ? s.groups : pair_warps(n, ctx->sm_count, ctx->warps_per_sm));
+}
+
 int launch_track(ufo_ctx *ctx, const ufo_prog *prog, const double *d_coords, const int32_t *d_seed,
                  const int32_t *d_pturns, int64_t n, int turns, int mode, int flags, int64_t slots,
                  int every, double *d_tracks, uint32_t *d_lost, double *d_final,
@@ -1364,18 +1416,27 @@ int launch_track(ufo_ctx *ctx, const ufo_prog *prog, const double *d_coords, con
   a.pool = ctx->pool;
   a.pool_seq = ctx->pool_seq;
   bool pair = use_pair(ctx, prog, n, flags);
+  int warps_per_sm = ctx->warps_per_sm;  // of the launch
+  ufo::Slices slices{};
   if (pair) {
+    slices = plan_slices(ctx, a, warps_per_sm);
     a.pair_ops = prog->pair_ops;
     if (prog->cache_fields) {
-      const int64_t lanes = 32 * pair_warps(n, ctx->sm_count, ctx->warps_per_sm);
+      int64_t lanes = cache_lanes_for(ctx, slices, n);
       ensure_cache(prog, lanes, stream);
+      if (prog->cache_lanes < lanes && slices.groups) {  // fewer lanes without slices
+        slices = ufo::Slices{};
+        warps_per_sm = ctx->warps_per_sm;
+        lanes = cache_lanes_for(ctx, slices, n);
+        ensure_cache(prog, lanes, stream);
+      }
       pair = prog->cache_lanes >= lanes;
       a.cache = prog->cache;
       a.cache_lanes = prog->cache_lanes;
     }
   }
   const int rc =
-      launch_kernels(a, prog->full, pair, ctx->sm_count, ctx->warps_per_sm, stream);
+      launch_kernels(a, prog->full, pair, slices, ctx->sm_count, warps_per_sm, stream);
   if (rc == UFO_OK) ctx->launches.fetch_add(1);
   return rc;
 }
@@ -1570,7 +1631,7 @@ int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *t
   p->captured = false;
   const bool pair =
       decode_pair(ops, n_ops, table, stride, n_seeds, INT_MAX, p->host_pair_ops, p->cache_fields,
-                  p->pair_fma);
+                  p->pair_fma, p->pair_general);
   const size_t pb = sizeof(ufo::PairOp) * p->host_pair_ops.size();
   const size_t ob = sizeof(ufo::Op) * (n_ops > 0 ? n_ops : 1);
   const size_t tb = sizeof(double) * static_cast<size_t>(stride) * n_seeds;
@@ -1613,7 +1674,8 @@ int ufo_prog_set_table(ufo_prog *prog, const double *table, int n_seeds) {
     int fields = 0;
     std::vector<ufo::PairOp> ops2;
     decode_pair(prog->host_ops.data(), prog->n_ops, table, prog->stride, n_seeds,
-                prog->captured ? prog->cache_fields : INT_MAX, ops2, fields, prog->pair_fma);
+                prog->captured ? prog->cache_fields : INT_MAX, ops2, fields, prog->pair_fma,
+                prog->pair_general);
     if (ops2.size() != prog->host_pair_ops.size() ||
         std::memcmp(ops2.data(), prog->host_pair_ops.data(), sizeof(ufo::PairOp) * ops2.size())) {
       UFO_CUDA(cudaMemcpyAsync(prog->pair_ops, ops2.data(), sizeof(ufo::PairOp) * ops2.size(),
@@ -1806,7 +1868,7 @@ extern "C" int ufo_track_noalloc(const int32_t *ops, int n_ops, const double *d_
                                d_coords, d_seed, d_pturns, n, turns, mode,
                                flags & ~UFO_TRACK_PLAIN, slots, every, d_tracks, d_lost, d_final,
                                &d.scratch->queue);
-  return launch_kernels(a, needs_full(ops, n_ops), false, d.sm_count, 16, st);
+  return launch_kernels(a, needs_full(ops, n_ops), false, ufo::Slices{}, d.sm_count, 16, st);
 }
 
 // ===================================================== tuning and graphs
@@ -1909,7 +1971,8 @@ extern "C" int ufo_graph_create(ufo_ctx *ctx, const ufo_prog *prog, const double
   if (!d_coords) return fail(UFO_E_ARG, "null coordinates");
   UFO_CUDA(cudaSetDevice(ctx->device));
   if (use_pair(ctx, prog, n, flags)) {  // nothing may be allocated under capture
-    ensure_cache(prog, 32 * pair_warps(n, ctx->sm_count, ctx->warps_per_sm), ctx->stream);
+    // enough for a launch with and without time slices
+    ensure_cache(prog, 32 * ((n + 15) / 16), ctx->stream);
     UFO_CUDA(cudaStreamSynchronize(ctx->stream));
   }
   cudaStream_t cap;
