@@ -44,6 +44,11 @@ UFO_DEV double ld(const double *p) { return __ldg(p); }
 // not finite: exponent field all ones (integer test, no FP64 pipe)
 UFO_DEV bool nf(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
 
+UFO_DEV bool is_nan(double v) {
+  const unsigned h = static_cast<unsigned>(__double2hiint(v)) & 0x7fffffffu;
+  return h > 0x7ff00000u || (h == 0x7ff00000u && __double2loint(v) != 0);
+}
+
 // Correctly rounded a/d given r = RN(1/d): q0 = RN(a*r) is within an ulp of a/d
 // and Markstein's correction q = RN(q0 + RN(a - q0*d)*r) (the remainder is
 // exact under FMA) returns RN(a/d) (P. Markstein, IBM J. Res. Dev. 34 (1990);
@@ -53,7 +58,8 @@ __device__ __noinline__ double div_ieee(double a, double d) { return __ddiv_rn(a
 
 UFO_DEV double divc(double a, double d, double r) {
   const unsigned e = static_cast<unsigned>(__double2hiint(a)) & 0x7ff00000u;
-  if (e < 0x07700000u || e > 0x77f00000u) return div_ieee(a, d);
+  if (e < 0x07700000u || e > 0x77f00000u)  // a lost particle's NaN needs no division
+    return is_nan(a) ? a : div_ieee(a, d);
   const double q0 = mul(a, r);
   const double rem = fma_(-q0, d, a);
   return fma_(rem, r, q0);
@@ -76,6 +82,13 @@ struct State {
   int turn;
   bool bad_o;  // oodppo not finite: every kick takes the untrimmed path
 };
+
+// A lost particle: all four coordinates are NaN and stay so whatever the
+// expression, so the trimmed paths serve it (the untrimmed ones run out of line
+// for one lane at a time, and a scan's lost particles finish their turn there).
+UFO_DEV bool all_nan(const State &s) {
+  return is_nan(s.x) && is_nan(s.px) && is_nan(s.y) && is_nan(s.py);
+}
 
 // ---------------------------------------------------------------- drifts
 // methods.drift (ufo/methods.py:28-43) on the pasted length text
@@ -501,7 +514,7 @@ __device__ __noinline__ PxPy slow_slice(double x, double y, double px, double py
 template <bool FMA, int PAT, bool WEAK>
 UFO_DEV void tp_slice(State &s, int nn, int ns, uint32_t mn, uint32_t ms, const double *ck,
                       bool achro, double t, double t2, double W, const double *ps = nullptr) {
-  if (s.bad_o || nf(s.x) || nf(s.y)) {
+  if ((s.bad_o || nf(s.x) || nf(s.y)) && !all_nan(s)) {
     const PxPy r = slow_slice<FMA>(s.x, s.y, s.px, s.py, s.o, s.bad_o, nn, ns, mn, ms, ck, achro,
                                    WEAK, W);
     s.px = r.px;
@@ -764,7 +777,7 @@ template <bool FMA, bool T1, bool T2>
 UFO_DEV void edge_v(State &s, int flags, const double *c) {
   const bool achro = flags & F_ACHRO;
   if (!T1 && !T2) {
-    if (s.bad_o || nf(s.x) || nf(s.y)) {
+    if ((s.bad_o || nf(s.x) || nf(s.y)) && !all_nan(s)) {
       const PxPy r = edge_ool(s.x, s.y, s.px, s.py, s.o, s.bad_o, flags, c);
       s.px = r.px;
       s.py = r.py;
@@ -772,7 +785,7 @@ UFO_DEV void edge_v(State &s, int flags, const double *c) {
     return;
   }
   const double curv = mul(ld(c), achro ? 1.0 : s.o);
-  if (nf(s.x) || nf(s.y) || nf(curv)) {
+  if ((nf(s.x) || nf(s.y) || nf(curv)) && !all_nan(s)) {
     const PxPy r = edge_ool(s.x, s.y, s.px, s.py, s.o, s.bad_o, flags, c);
     s.px = r.px;
     s.py = r.py;

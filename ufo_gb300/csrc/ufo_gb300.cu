@@ -135,7 +135,7 @@ UFO_DEV void apply_op(State &s, const Op &op, const double *c, Observe see) {
         drift<FMA>(s, DF_MUL2, false, c);
       break;
     case OP_KICK: {
-      const bool bad = s.bad_o || nf(s.x) || nf(s.y);
+      const bool bad = (s.bad_o || nf(s.x) || nf(s.y)) && !all_nan(s);
       if (FMA && !bad && (op.flags & F_PSER)) {  // dense series after the coefficients
         const uint32_t mn = static_cast<uint32_t>(op.i2), ms = static_cast<uint32_t>(op.i3);
         const PxPy r = kick_pser_ool(s.x, s.y, s.px, s.py, (op.flags & F_ACHRO) ? 1.0 : s.o,
@@ -814,6 +814,8 @@ int ensure_constants(int device) {
   return UFO_OK;
 }
 
+constexpr int DEFAULT_WARPS = 16;  // resident warps per SM of the persistent grid
+
 int popc32(uint32_t v) { return __builtin_popcount(v); }
 
 bool mask_fits(int n, int32_t mask) {
@@ -1195,11 +1197,15 @@ unsigned long long spread_multiplier(int64_t n_particles) {
 
 // Warps of the two-lane kernel: 16 particles each; the tuning counts warps of
 // the one-lane kernel, so twice as many, at most the 16 per SM that the
-// registers allow.
-int64_t pair_warps(int64_t n, int sm_count, int warps_per_sm) {
-  const int64_t warps = (n + 15) / 16;
-  const int64_t resident = static_cast<int64_t>(sm_count) * std::min(16, 2 * warps_per_sm);
-  return std::min(warps, resident);
+// registers allow.  A dynamic-aperture scan at the default tuning gets 8 per SM:
+// most of its particles are lost in the first turns, and lanes that refill from
+// a longer queue stay fuller (49,152 particles of the FODO ring with errors, 64
+// turns, 15 % survive: FMA 25 ms with 16, 16 ms with 8; strict 132 and 79 ms),
+// while two warps per sub-partition still fill most of the FP64 pipe.
+int64_t pair_warps(const ufo::TrackArgs &a, int sm_count, int warps_per_sm) {
+  const int64_t per_sm = a.mode == UFO_MODE_SA && warps_per_sm == DEFAULT_WARPS
+                             ? 8 : std::min(16, 2 * warps_per_sm);
+  return std::min((a.n + 15) / 16, sm_count * per_sm);
 }
 
 // The launch shared by every entry point: fill the kernel arguments and start
@@ -1250,7 +1256,7 @@ int launch_kernels(ufo::TrackArgs &a, bool full, bool pair, const ufo::Slices &s
       ufo::track_pair_sliced<false><<<g, 32, 0, stream>>>(a, slices);
   } else if (pair) {
     UFO_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), stream));
-    const unsigned g = static_cast<unsigned>(pair_warps(a.n, sm_count, warps_per_sm));
+    const unsigned g = static_cast<unsigned>(pair_warps(a, sm_count, warps_per_sm));
     if (fma)
       ufo::track_pair_kernel<true><<<g, 32, 0, stream>>>(a);
     else
@@ -1320,16 +1326,25 @@ ufo::TrackArgs make_args(const ufo::Op *ops, int n_ops, const double *table, int
 //   A ring with general error kicks on most magnets (a coefficient enters one
 //   lane's sum, so half its products are idle) gains up to 12 warps per SM:
 //   light-source ring with errors 1,000 particles 15,590 -> 8,480, 30,000 even.
-//  FMA: up to 12 warps per SM.  The sextupole form and the composed linear
-//   elements cost the two-lane code more instructions (6 for 5, 8 for 5 per 32
-//   particles), so the one-lane kernel wins once the pipe is full:
-//   light-source ring 333 particles 652 -> 345, 20,000 (8.2 warps per SM) 707 ->
-//   597, 65,536 1,511 -> 2,009; ring with errors on every magnet 30,000 (12.3)
-//   442 -> 404, 65,536 826 -> 891.
-bool use_pair(const ufo_ctx *ctx, const ufo_prog *prog, int64_t n, int flags) {
+//  FMA: up to 9 warps per SM, 14 where most kicks are general.  The sextupole
+//   form and the composed linear elements cost the two-lane code more
+//   instructions (6 for 5, 8 for 5 per 32 particles), so the one-lane kernel
+//   wins once its pipe is full: light-source ring 333 particles 652 -> 345,
+//   20,000 (8.2 warps per SM) 699 -> 615, 24,000 (9.9) 705 -> 770; ring with
+//   errors on every magnet 1,000 346 -> 192, 33,000 (13.6) 442 -> 439, 38,900
+//   (16) 477 -> 516.
+//  Dynamic-aperture scans of such a ring: always (pair_warps).
+//  Uneven turn counts on such a ring: always.  The last, longest particles run
+//   in few warps, and twice as many half-size warps leave the queue more evenly:
+//   error seeds of 64 to 256 turns, 39,873 particles 132 -> 110 ms, 85,102
+//   particles 223 -> 167 ms, 15,978 the same.
+bool use_pair(const ufo_ctx *ctx, const ufo_prog *prog, int64_t n, int mode, int flags,
+              bool uneven) {
   if (!prog->pair_ops || ((flags & UFO_TRACK_FMA) && !prog->pair_fma) || (flags & (UFO_TRACK_PLAIN | UFO_TRACK_COMPACT))) return false;
   if (!(flags & UFO_TRACK_FMA) && !prog->pair_general) return true;
-  return (n + 15) / 16 <= 12 * static_cast<int64_t>(ctx->sm_count);
+  if (prog->pair_general && (uneven || mode == UFO_MODE_SA)) return true;
+  const int most = !prog->pair_general ? 9 : (flags & UFO_TRACK_FMA) ? 14 : 12;
+  return (n + 15) / 16 <= most * static_cast<int64_t>(ctx->sm_count);
 }
 
 // The program's coefficient cache for a two-lane launch of `lanes` lanes, grown
@@ -1401,8 +1416,8 @@ ufo::Slices plan_slices(const ufo_ctx *ctx, const ufo::TrackArgs &a, int &warps_
 }
 
 // lanes of the coefficient cache: per group where groups move between warps
-int64_t cache_lanes_for(const ufo_ctx *ctx, const ufo::Slices &s, int64_t n) {
-  return 32 * (s.groups ? s.groups : pair_warps(n, ctx->sm_count, ctx->warps_per_sm));
+int64_t cache_lanes_for(const ufo_ctx *ctx, const ufo::Slices &s, const ufo::TrackArgs &a) {
+  return 32 * (s.groups ? s.groups : pair_warps(a, ctx->sm_count, ctx->warps_per_sm));
 }
 
 int launch_track(ufo_ctx *ctx, const ufo_prog *prog, const double *d_coords, const int32_t *d_seed,
@@ -1415,19 +1430,19 @@ int launch_track(ufo_ctx *ctx, const ufo_prog *prog, const double *d_coords, con
                                slots, every, d_tracks, d_lost, d_final, ctx->queue);
   a.pool = ctx->pool;
   a.pool_seq = ctx->pool_seq;
-  bool pair = use_pair(ctx, prog, n, flags);
+  bool pair = use_pair(ctx, prog, n, mode, flags, d_pturns != nullptr);
   int warps_per_sm = ctx->warps_per_sm;  // of the launch
   ufo::Slices slices{};
   if (pair) {
     slices = plan_slices(ctx, a, warps_per_sm);
     a.pair_ops = prog->pair_ops;
     if (prog->cache_fields) {
-      int64_t lanes = cache_lanes_for(ctx, slices, n);
+      int64_t lanes = cache_lanes_for(ctx, slices, a);
       ensure_cache(prog, lanes, stream);
       if (prog->cache_lanes < lanes && slices.groups) {  // fewer lanes without slices
         slices = ufo::Slices{};
         warps_per_sm = ctx->warps_per_sm;
-        lanes = cache_lanes_for(ctx, slices, n);
+        lanes = cache_lanes_for(ctx, slices, a);
         ensure_cache(prog, lanes, stream);
       }
       pair = prog->cache_lanes >= lanes;
@@ -1481,7 +1496,7 @@ int ufo_ctx_create(int device, ufo_ctx **out) {
   cudaError_t e = cudaGetDeviceProperties(&prop, device);
   if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaGetDeviceProperties"); }
   c->sm_count = prop.multiProcessorCount;
-  c->warps_per_sm = 16;
+  c->warps_per_sm = DEFAULT_WARPS;
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaStreamCreate"); }
   e = cudaMalloc(&c->queue, 64);
@@ -1970,7 +1985,7 @@ extern "C" int ufo_graph_create(ufo_ctx *ctx, const ufo_prog *prog, const double
   if (n <= 0) return fail(UFO_E_ARG, "empty launch");
   if (!d_coords) return fail(UFO_E_ARG, "null coordinates");
   UFO_CUDA(cudaSetDevice(ctx->device));
-  if (use_pair(ctx, prog, n, flags)) {  // nothing may be allocated under capture
+  if (use_pair(ctx, prog, n, mode, flags, d_pturns != nullptr)) {  // nothing may be allocated under capture
     // enough for a launch with and without time slices
     ensure_cache(prog, 32 * ((n + 15) / 16), ctx->stream);
     UFO_CUDA(cudaStreamSynchronize(ctx->stream));
