@@ -151,6 +151,31 @@ def test_seeds_turn_counts_and_new_tables():
         assert _same(*out)
 
 
+def test_tables_that_change_the_two_lane_form():
+    """Strengths too small for the two-lane form send their elements through the
+    one-lane code; tables may switch between the two."""
+    import ufo_gb300 as u
+    from ufo_gb300 import capi, compiler as C
+    ctx = u.context(0)
+    line, flags = _rings()['c1']
+    at = [i for i, e in enumerate(line.flatten()) if type(e).__name__ == 'Quadrupole']
+    params = [(i, 'k1') for i in at]
+    coords = _beam(100)
+    plain = np.full((1, len(at)), 1.1)
+    tiny = plain.copy()
+    tiny[0, ::2] = 1e-300
+    tiny[0, 1::4] = 1e300
+    for fma in (0, u.FMA):
+        tf = capi.UFO_TRACK_FMA if fma else 0
+        dp = capi.DeviceProgram(ctx, C.compile_line(line, flags | fma, params, [-1],
+                                                    seed_values=plain))
+        for rows in (plain, tiny, plain):
+            dp.set_table(C.compile_line(line, flags | fma, params, [-1], seed_values=rows).table)
+            out = [capi.track(ctx, dp, coords, 3, capi.UFO_MODE_TRACK, tf | f, slots=0)[1:]
+                   for f in (capi.UFO_TRACK_PLAIN, 0)]
+            assert _same(*out)
+
+
 def test_graph_of_a_thick_batch_keeps_its_cache():
     """A captured graph goes on using the coefficient cache while larger
     launches and new tables of the same program come and go."""

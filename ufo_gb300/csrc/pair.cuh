@@ -74,7 +74,8 @@ UFO_DEV double pick(bool first, double a, double b) { return first ? a : b; }
 //   toff  first constant in the table row
 //   a     slices; first field in the coefficient cache (-1: none); observation
 //         index; first op of a segment in the public list
-//   b     normal mask | skew mask << 16; end of the segment
+//   b     general kicks: normal mask | skew mask << 16; end of the segment; with
+//         PF_THEN the first constant of a plain drift that follows the op
 struct PairOp {
   int head, toff, a, b;
 };
@@ -84,7 +85,8 @@ enum : int {
   PF_X = 1 << 19, PF_Y = 1 << 20,  // the plane has the term (align, edge)
   PF_CONST = 1 << 21,
   PF_DIV = 1 << 23,    // the table holds [A, d, 1/d, A/d] for the inner drift
-  PF_FILL = 1 << 24    // this op fills its cache fields
+  PF_FILL = 1 << 24,   // this op fills its cache fields
+  PF_THEN = 1 << 25    // a plain drift follows, run with this op (strict list only)
 };
 enum : int {
   PV_SEGMENT = 0, PV_DRIFT, PV_DRIFT2, PV_DRIFT_DIV, PV_ALIGN, PV_EDGE, PV_EDGE_PSI, PV_THICKQ,
@@ -271,7 +273,7 @@ template <bool FMA, int PAT, int DIV, int WEAK>
 UFO_DEV void pair_teapot(Half &h, const PairCtx &x, const PairOp &op, double Lo, const double *c,
                          bool &bad) {
   const int N = op.a;
-  const uint32_t masks = static_cast<uint32_t>(op.b);
+  const uint32_t masks = static_cast<uint32_t>(op.b);  // general kicks only
   const double o1 = (op.head & PF_ACHRO) ? 1.0 : x.o;
   const bool table_div = op.head & PF_DIV;
   const int variant = (op.head & 0xff) - PV_TEAPOT;
@@ -288,7 +290,7 @@ UFO_DEV void pair_teapot(Half &h, const PairCtx &x, const PairOp &op, double Lo,
     d = ld(c + 2);
     r = ld(c + 3);
   }
-  const int nk = __popc(masks);
+  const int nk = PAT == 0 ? __popc(masks) : PAT == 3 ? 0 : 1;
   const double W = weak && x.even ? ld(ck + nk) : 0.0;
   const double Lx = (op.head & PF_SPLITO) ? ld(ck + nk + (weak ? 1 : 0)) : Lo;
   const double t = pair_strength<FMA, PAT>(x, PAT == 1 || PAT == 2 ? ld(ck) : 0.0, o1);
@@ -296,6 +298,8 @@ UFO_DEV void pair_teapot(Half &h, const PairCtx &x, const PairOp &op, double Lo,
       FMA && PAT == 0 ? ck + nk + (weak ? 1 : 0) + ((op.head & PF_SPLITO) ? 1 : 0) : nullptr;
   const int shift_hi = ((op.head >> 8) & 0xff) << 20;
   const int sign = static_cast<int>(static_cast<unsigned>(op.head & PF_NEG) << 15);
+  const bool then = !FMA && PAT != 0 && (op.head & PF_THEN);
+  const double Lt = then ? ld(x.tab + op.b) : 0.0;
   pair_drift<FMA>(h, Lo);
   for (int sl = 1;; ++sl) {
     pair_kick<FMA, PAT>(h, x, masks, ck, t, ps, bad);
@@ -309,6 +313,7 @@ UFO_DEV void pair_teapot(Half &h, const PairCtx &x, const PairOp &op, double Lo,
       h.u = add(h.u, div_markstein(mul(h.pu, A), d, r, bad));
   }
   pair_drift<FMA>(h, Lx);
+  if (then) pair_drift<FMA>(h, Lt);
 }
 
 // ---------------------------------------------------------------- thick
@@ -537,6 +542,15 @@ enum : int { PE_END = 0, PE_REDO = 1, PE_WIDE = 2 };
 // Run the list from op `pos`, where a segment's header or its WIDE op stands.
 // PE_REDO leaves the segment's entry state in h and its public ops in [first,
 // last).
+// The drift that goes with an op, in the ops' own code: common code after the
+// dispatch costs every op some 100 cycles.  Only the strict list has it (FODO
+// ring 1,024 particles 67 -> 60 us per turn, thick ring 350 -> 318): FMA programs
+// have their drifts merged into the magnets, and the code alone slowed them by 6 %.
+template <bool FMA>
+UFO_DEV void pair_then(Half &h, const PairCtx &x, const PairOp &op) {
+  if (!FMA && (op.head & PF_THEN)) pair_drift<FMA>(h, ld(x.tab + op.b));
+}
+
 template <bool FMA>
 UFO_DEV int pair_run(Half &h, const PairCtx &x, int &pos, int &first, int &last,
                      const TrackArgs &a, const PairShared &sh, bool any_bad_o) {
@@ -570,6 +584,7 @@ UFO_DEV int pair_run(Half &h, const PairCtx &x, int &pos, int &first, int &last,
       }
       case PV_DRIFT:
         pair_drift<FMA>(h, c0);
+        pair_then<FMA>(h, x, op);
         break;
       case PV_DRIFT2: {
         const double t = mul(h.pu, c0);
@@ -582,6 +597,7 @@ UFO_DEV int pair_run(Half &h, const PairCtx &x, int &pos, int &first, int &last,
         break;
       case PV_ALIGN:
         h.u = sub(h.u, (op.head & (even ? PF_X : PF_Y)) ? ld(c + (even ? 0 : 1)) : 0.0);
+        pair_then<FMA>(h, x, op);
         break;
       case PV_EDGE: {
         const double curv = mul(c0, (op.head & PF_ACHRO) ? 1.0 : x.o);
@@ -591,6 +607,7 @@ UFO_DEV int pair_run(Half &h, const PairCtx &x, int &pos, int &first, int &last,
         const double t = mul(h.u, curv);
         h.pu = FMA ? fma_(t, T, h.pu) : add(h.pu, mul(t, T));
         bad = bad || nf(curv);
+        pair_then<FMA>(h, x, op);
         break;
       }
       case PV_EDGE_PSI: {
@@ -598,13 +615,16 @@ UFO_DEV int pair_run(Half &h, const PairCtx &x, int &pos, int &first, int &last,
         const double T = *pair_cache(a, op.a, x.group);
         h.pu = add(h.pu, mul(mul(h.u, curv), T));
         bad = bad || nf(curv);
+        pair_then<FMA>(h, x, op);
         break;
       }
       case PV_THICKQ:
         thick_apply(h, pair_cache(a, op.a, x.group), a.cache_lanes, false, bad);
+        pair_then<FMA>(h, x, op);
         break;
       case PV_THICKB:
         thick_apply(h, pair_cache(a, op.a, x.group), a.cache_lanes, true, bad);
+        pair_then<FMA>(h, x, op);
         break;
       case PV_CIRCLE: {
         const double s = mul(h.u, h.u);

@@ -757,9 +757,11 @@ struct ufo_prog {
   int n_dumps;
   bool full;  // needs the full interpreter (thick, wire, exact, ...)
   std::vector<int32_t> host_ops;  // for validating replacement tables
-  // two-lane kernel (pair.cuh): null when a op has no two-lane form
+  // two-lane kernel (pair.cuh): the strict list, then at pair_fma_at the FMA one;
+  // null when an op has no two-lane form
   ufo::PairOp *pair_ops;
   std::vector<ufo::PairOp> host_pair_ops;
+  size_t pair_fma_at;
   bool pair_fma;               // also for FMA launches
   bool pair_general;           // most kicks are general
   int cache_fields;            // doubles per lane of the coefficient cache
@@ -1017,11 +1019,9 @@ int kick_pattern(int nn, int ns, int32_t mn) {
 // their cache fields; at most `most_fields` are given out, and further elements
 // compute in every turn.  `fma_ready`: the general kicks carry the dense series
 // that the FMA kernel reads.
-bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t stride, int n_seeds,
-                 int most_fields, std::vector<ufo::PairOp> &out, int &cache_fields,
-                 bool &fma_ready, bool &mostly_general) {
-  out.clear();
-  out.reserve(static_cast<size_t>(n_ops) + n_ops / ufo::PAIR_SEGMENT + 4);
+bool decode_list(const int32_t *ops, int n_ops, const double *table, int64_t stride, int n_seeds,
+                 int most_fields, bool fold_drifts, std::vector<ufo::PairOp> &out,
+                 int &cache_fields, bool &fma_ready, bool &mostly_general) {
   cache_fields = 0;
   fma_ready = true;
   int kicks = 0, general = 0;
@@ -1073,7 +1073,7 @@ bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t str
             !plain_strength(w[2] + (!teapot ? 0 : w[3] <= 1 ? 1 : div ? 5 : 2)))
           break;
         op.a = teapot ? w[3] : i;
-        op.b = k[2] | k[3] << 16;
+        op.b = pattern == 0 ? k[2] | k[3] << 16 : 0;
         if (!teapot) {
           if (pattern == 3) keep = false;
           op.head = (ufo::PV_KICK + pattern) | common;
@@ -1153,6 +1153,19 @@ bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t str
         cache_fields += fields;
       }
     }
+    // A plain drift goes with the op before it (strict list): an op of its own
+    // costs its dispatch, about 200 cycles beside the 129 of its arithmetic.
+    ufo::PairOp &before = out.back();
+    const int variant = before.head & 0xff;
+    if (fold_drifts && keep && op.head == ufo::PV_DRIFT && out.size() - 1 > head &&
+        !(before.head & ufo::PF_THEN) &&
+        (variant == ufo::PV_DRIFT || variant == ufo::PV_ALIGN || variant == ufo::PV_EDGE ||
+         variant == ufo::PV_EDGE_PSI || variant == ufo::PV_THICKQ || variant == ufo::PV_THICKB ||
+         (variant >= ufo::PV_TEAPOT && (variant - ufo::PV_TEAPOT) % 4 != 0))) {
+      before.head |= ufo::PF_THEN;
+      before.b = op.toff;
+      keep = false;
+    }
     if (keep) {
       // an op without a two-lane form is a segment of its own
       const bool wide = op.head == ufo::PV_WIDE;
@@ -1167,6 +1180,23 @@ bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t str
   out.push_back({ufo::PV_SEGMENT, 0, 0, 0});   // the kernel fetches two ops ahead
   out.push_back({ufo::PV_SEGMENT, 0, 0, 0});
   mostly_general = 2 * general > kicks;
+  return true;
+}
+
+// Both lists, at fixed places whatever the constants make of them (a captured
+// graph keeps their addresses): the second at `fma_at`, each padded to two
+// entries per op -- every op a segment of its own -- and the ends.
+bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t stride, int n_seeds,
+                 int most_fields, std::vector<ufo::PairOp> &out, size_t &fma_at,
+                 int &cache_fields, bool &fma_ready, bool &mostly_general) {
+  out.clear();
+  fma_at = 2 * static_cast<size_t>(n_ops) + 4;
+  for (const bool strict : {true, false}) {
+    if (!decode_list(ops, n_ops, table, stride, n_seeds, most_fields, strict, out, cache_fields,
+                     fma_ready, mostly_general))
+      return false;
+    out.resize(strict ? fma_at : 2 * fma_at);
+  }
   return true;
 }
 
@@ -1435,7 +1465,7 @@ int launch_track(ufo_ctx *ctx, const ufo_prog *prog, const double *d_coords, con
   ufo::Slices slices{};
   if (pair) {
     slices = plan_slices(ctx, a, warps_per_sm);
-    a.pair_ops = prog->pair_ops;
+    a.pair_ops = prog->pair_ops + ((flags & UFO_TRACK_FMA) ? prog->pair_fma_at : 0);
     if (prog->cache_fields) {
       int64_t lanes = cache_lanes_for(ctx, slices, a);
       ensure_cache(prog, lanes, stream);
@@ -1645,8 +1675,8 @@ int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *t
   p->cache_lanes = 0;
   p->captured = false;
   const bool pair =
-      decode_pair(ops, n_ops, table, stride, n_seeds, INT_MAX, p->host_pair_ops, p->cache_fields,
-                  p->pair_fma, p->pair_general);
+      decode_pair(ops, n_ops, table, stride, n_seeds, INT_MAX, p->host_pair_ops, p->pair_fma_at,
+                  p->cache_fields, p->pair_fma, p->pair_general);
   const size_t pb = sizeof(ufo::PairOp) * p->host_pair_ops.size();
   const size_t ob = sizeof(ufo::Op) * (n_ops > 0 ? n_ops : 1);
   const size_t tb = sizeof(double) * static_cast<size_t>(stride) * n_seeds;
@@ -1689,10 +1719,9 @@ int ufo_prog_set_table(ufo_prog *prog, const double *table, int n_seeds) {
     int fields = 0;
     std::vector<ufo::PairOp> ops2;
     decode_pair(prog->host_ops.data(), prog->n_ops, table, prog->stride, n_seeds,
-                prog->captured ? prog->cache_fields : INT_MAX, ops2, fields, prog->pair_fma,
-                prog->pair_general);
-    if (ops2.size() != prog->host_pair_ops.size() ||
-        std::memcmp(ops2.data(), prog->host_pair_ops.data(), sizeof(ufo::PairOp) * ops2.size())) {
+                prog->captured ? prog->cache_fields : INT_MAX, ops2, prog->pair_fma_at, fields,
+                prog->pair_fma, prog->pair_general);
+    if (std::memcmp(ops2.data(), prog->host_pair_ops.data(), sizeof(ufo::PairOp) * ops2.size())) {
       UFO_CUDA(cudaMemcpyAsync(prog->pair_ops, ops2.data(), sizeof(ufo::PairOp) * ops2.size(),
                                cudaMemcpyHostToDevice, prog->ctx->stream));
       UFO_CUDA(cudaStreamSynchronize(prog->ctx->stream));
