@@ -517,11 +517,10 @@ __device__ __noinline__ void pair_fill(const TrackArgs &a, const PairShared &sh,
   const bool even = (lane & 1) == 0;
   const int64_t p = sh.p[lane];
   const double dp = p >= 0 ? a.coords[p * 6 + 5] : 0.0, o = sh.o[lane];
-  for (const int4 *w = reinterpret_cast<const int4 *>(a.pair_ops);; ++w) {
+  for (const int4 *w = reinterpret_cast<const int4 *>(a.pair_fills);; ++w) {
     const PairOp op = pair_fetch(w);
     const int variant = op.head & 0xff;
-    if (variant == PV_SEGMENT && op.b <= op.a) return;
-    if (!(op.head & PF_FILL)) continue;
+    if (variant == PV_SEGMENT) return;  // the end
     const double *c = sh.tab[lane] + op.toff;
     double *t = pair_cache(a, op.a, group);
     if (variant == PV_THICKQ) {
