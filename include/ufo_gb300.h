@@ -37,6 +37,8 @@ extern "C" {
 /* track flags */
 #define UFO_TRACK_FMA 1      /* fused multiply-add arithmetic (tolerance parity) */
 #define UFO_TRACK_FIVED 2    /* do not write z, dp into tracks (ufo/track.py:62-65) */
+/* Without PLAIN or COMPACT the library chooses between the persistent kernels:
+ * one particle per lane, or its two planes on two lanes. */
 #define UFO_TRACK_PLAIN 4    /* one thread per particle, no lane refill */
 #define UFO_TRACK_COMPACT 8  /* persistent CTAs (one per SM, warps_per_sm warps, at most
                                 16) that pack survivors into full warps once every particle
@@ -66,7 +68,12 @@ void ufo_ctx_destroy(ufo_ctx *ctx);
 
 /* Upload a compiled line: `ops` int32[n_ops][8], `table` f64[n_seeds][stride],
  * `n_dumps` observation points per turn.  Replaces the kernel build of
- * ufo/track.py:84-118 (cl.Program(...).build). */
+ * ufo/track.py:84-118 (cl.Program(...).build).
+ * A program with thick elements or chromatic fringe edges keeps a device cache of
+ * their momentum-dependent coefficients: allocated by its first launch (or graph
+ * creation) outside a stream capture, at most 4 GiB, freed with the program, and
+ * shared like the context's counters.  A launch without it gives the same results
+ * from the one-lane kernel. */
 int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *table,
                     int64_t stride, int n_seeds, int n_dumps, ufo_prog **out);
 /* Replace the per-seed constants (same stride); new parameter values between
@@ -157,8 +164,9 @@ int ufo_track_noalloc(const int32_t *ops, int n_ops, const double *d_table, int6
 int ufo_closed_orbit(ufo_ctx *ctx, const ufo_prog *prog, const double *start,
                      const int32_t *seed, int64_t n, int iterations, double *orbits);
 
-/* Resident warps per SM of the persistent grid (default 16); set by the
- * autotuner (ufo_gb300/batch.py: autotune).  No reference counterpart. */
+/* Resident warps per SM of the persistent grid (default 16; the two-lane kernel,
+ * whose warps hold half the particles, takes twice as many, at most 16, and 8 for
+ * a dynamic-aperture scan at the default); set by the autotuner (ufo_gb300/batch.py: autotune).  No reference counterpart. */
 int ufo_ctx_set_tuning(ufo_ctx *ctx, int warps_per_sm);
 
 /* One tracking launch (work-counter reset + persistent kernel over all
