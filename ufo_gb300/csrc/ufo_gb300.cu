@@ -1032,6 +1032,7 @@ bool decode_list(const int32_t *ops, int n_ops, const double *table, int64_t str
   struct Shared { int op, field; };
   std::unordered_multimap<uint64_t, Shared> seen;  // constants' hash -> first op
   size_t head = 0;  // the current segment's header
+  int64_t last_end = -1;  // where the constants of the last general teapot end
   auto open = [&](int first) {
     head = out.size();
     out.push_back({ufo::PV_SEGMENT, 0, first, first});
@@ -1095,12 +1096,38 @@ bool decode_list(const int32_t *ops, int n_ops, const double *table, int64_t str
         }
         op.head = (ufo::PV_TEAPOT + pattern + 4 * form + ((flags & ufo::F_WEAK) ? 12 : 0)) |
                   shift << 8 | (shift && negative ? ufo::PF_NEG : 0) | (div ? ufo::PF_DIV : 0) |
-                  ((flags & ufo::F_SPLITO) ? ufo::PF_SPLITO : 0) | common;
+                  ((flags & ufo::F_SPLITO) ? ufo::PF_SPLITO : 0) | common |
+                  ((flags & ufo::F_PSER) ? ufo::PF_PSER : 0);
+        if (pattern == 0) {
+          // the shift before a general teapot runs with it: see PF_PRE
+          last_end = w[2] + op_consts(w);
+          const ufo::PairOp &before = out.back();
+          const int gap = w[2] - before.toff;
+          if (out.size() - 1 > head && (before.head & 0xff) == ufo::PV_ALIGN &&
+              !(before.head & ufo::PF_THEN) && (gap == 2 || gap == 5)) {
+            op.head |= ufo::PF_PRE | (gap == 5 ? ufo::PF_PRE_EDGE : 0) |
+                       (before.head & (ufo::PF_X | ufo::PF_Y));
+            out.pop_back();
+          }
+        }
         break;
       }
       case ufo::OP_ALIGN:
         op.head = ufo::PV_ALIGN | ((flags & ufo::F_AX) ? ufo::PF_X : 0) |
                   ((flags & ufo::F_AY) ? ufo::PF_Y : 0);
+        {  // the shift after a general teapot
+          ufo::PairOp &before = out.back();
+          const int variant = (before.head & 0xff) - ufo::PV_TEAPOT;
+          const int planes = op.head & (ufo::PF_X | ufo::PF_Y);
+          const int64_t gap = w[2] - last_end;
+          if (out.size() - 1 > head && variant >= 0 && variant % 4 == 0 &&
+              !(before.head & ufo::PF_POST) && (gap == 0 || gap == 3) &&
+              (!(before.head & ufo::PF_PRE) ||
+               (before.head & (ufo::PF_X | ufo::PF_Y)) == planes)) {
+            before.head |= ufo::PF_POST | (gap == 3 ? ufo::PF_POST_EDGE : 0) | planes;
+            keep = false;
+          }
+        }
         break;
       case ufo::OP_EDGE:
         keep = flags & (ufo::F_T1 | ufo::F_T2 | ufo::F_RTPSI);

@@ -241,7 +241,8 @@ class StableAperture:
 
     # resident warps per SM of the compacting kernel for a scan: measured
     # best on the 196,608-particle dynamic-aperture grid with the CTAs
-    # exchanging particles (16: 8.1e9, 8: 7.8e9 particle*element*turns/s)
+    # exchanging particles (16: 8.1e9, 8: 7.8e9 particle*element*turns/s; 16
+    # with lost particles on the trimmed path: 9.4e9)
     COMPACT_WARPS_PER_SM = 16
 
     def run(self, threads=1, compact=None):
@@ -254,8 +255,8 @@ class StableAperture:
         every particle has been handed out, each CTA packs its survivors into
         its lowest warps at every turn and the CTAs even out their particle
         counts through a pool, so the long-lived particles of an uneven scan
-        fill whole warps on every SM.  ``compact=False``: one launch of the
-        one-warp persistent kernel.  Loss turns and coordinates are the same
+        fill whole warps on every SM.  ``compact=False``: one launch of a
+        free-running persistent kernel.  Loss turns and coordinates are the same
         in every case."""
         pool = np.asarray(self.parameters, dtype=np.float64)
         seed_values, seed = self._c.seeds(pool)
