@@ -1012,6 +1012,87 @@ int kick_pattern(int nn, int ns, int32_t mn) {
   return ns != 0 ? 0 : (nn == 2 && mn == 2) ? 1 : (nn == 3 && mn == 4) ? 2 : mn == 0 ? 3 : 0;
 }
 
+// What the two-lane lists need to know of every row's constants, gathered in one
+// pass over the table row by row (op by op, each look misses the cache: 20,000
+// rows of 833 ops took 170 ms more at every new table).
+struct RowScan {
+  int strength = -1;     // where a short form's strength stands; -1: none
+  int division = -1;     // where an inner drift's [d, 1/d] stand; -1: none
+  bool plain = true;     // strengths whose half and negative are exact, in every row
+  bool same = true;      // the division is row 0's in every row
+  int twin = -1;         // an earlier op with the same cacheable constants in every row
+};
+
+bool plain_strength(double k) {
+  k = std::fabs(k);
+  return k == 0.0 || (k > 1e-280 && k < 1e280);
+}
+
+std::vector<RowScan> scan_rows(const int32_t *ops, int n_ops, const double *table, int64_t stride,
+                               int n_seeds) {
+  std::vector<RowScan> scan(static_cast<size_t>(n_ops));
+  std::vector<int> looked, twins;
+  std::unordered_multimap<uint64_t, int> seen;  // row 0's constants -> op
+  auto word = [&](int i) { return ops + static_cast<size_t>(i) * UFO_OP_WORDS; };
+  auto bytes = [&](int i) { return sizeof(double) * static_cast<size_t>(op_consts(word(i))); };
+  for (int i = 0; i < n_ops; ++i) {
+    const int32_t *w = word(i);
+    RowScan &s = scan[static_cast<size_t>(i)];
+    if (w[0] == ufo::OP_KICK ||
+        (w[0] == ufo::OP_TEAPOT && !(w[1] & (ufo::F_YOSHIDA | ufo::F_EXACT)))) {
+      const bool teapot = w[0] == ufo::OP_TEAPOT;
+      const bool div = teapot && w[3] > 1 && ((w[1] >> ufo::SH_FINNER) & 3) == ufo::DF_DIV;
+      const int pattern = kick_pattern(w[teapot ? 4 : 3], w[teapot ? 5 : 4], w[teapot ? 6 : 5]);
+      if (pattern == 1 || pattern == 2)
+        s.strength = w[2] + (!teapot ? 0 : w[3] <= 1 ? 1 : div ? 5 : 2);
+      if (div) s.division = w[2] + 2;
+      if (s.strength >= 0 || s.division >= 0) looked.push_back(i);
+    } else if (w[0] == ufo::OP_THICKQ || w[0] == ufo::OP_THICKB ||
+               (w[0] == ufo::OP_EDGE && (w[1] & ufo::F_RTPSI))) {
+      uint64_t h = 1469598103934665603ull ^ static_cast<uint64_t>(w[0] * 31 + w[1]);
+      for (int64_t k = 0; k < op_consts(w); ++k) {
+        uint64_t bits;
+        std::memcpy(&bits, table + w[2] + k, sizeof bits);
+        h = (h ^ bits) * 1099511628211ull;
+        h ^= h >> 29;
+      }
+      const auto range = seen.equal_range(h);
+      for (auto it = range.first; it != range.second && s.twin < 0; ++it) {
+        const int32_t *v = word(it->second);
+        if (v[0] == w[0] && v[1] == w[1] &&
+            std::memcmp(table + v[2], table + w[2], bytes(i)) == 0)
+          s.twin = it->second;
+      }
+      if (s.twin < 0)
+        seen.emplace(h, i);
+      else
+        twins.push_back(i);
+    }
+  }
+  for (int r = 0; r < n_seeds; ++r) {
+    const double *row = table + static_cast<int64_t>(r) * stride;
+    for (const int i : looked) {
+      RowScan &s = scan[static_cast<size_t>(i)];
+      if (s.strength >= 0) s.plain = s.plain && plain_strength(row[s.strength]);
+      if (s.division >= 0)
+        s.same = s.same && row[s.division] == table[s.division] &&
+                 row[s.division + 1] == table[s.division + 1];
+    }
+    for (size_t k = 0; r > 0 && k < twins.size();) {
+      const int i = twins[k];
+      RowScan &s = scan[static_cast<size_t>(i)];
+      if (std::memcmp(row + word(s.twin)[2], row + word(i)[2], bytes(i)) == 0) {
+        ++k;
+      } else {  // on its own from here
+        s.twin = -1;
+        twins[k] = twins.back();
+        twins.pop_back();
+      }
+    }
+  }
+  return scan;
+}
+
 // where a list's cache-filling ops start
 size_t pair_fill_at(int n_ops) { return 2 * static_cast<size_t>(n_ops) + 4; }
 
@@ -1023,27 +1104,18 @@ size_t pair_fill_at(int n_ops) { return 2 * static_cast<size_t>(n_ops) + 4; }
 // their cache fields; at most `most_fields` are given out, and further elements
 // compute in every turn.  `fma_ready`: the general kicks carry the dense series
 // that the FMA kernel reads.
-bool decode_list(const int32_t *ops, int n_ops, const double *table, int64_t stride, int n_seeds,
-                 int most_fields, bool fold_drifts, std::vector<ufo::PairOp> &out,
+bool decode_list(const int32_t *ops, int n_ops, const double *table,
+                 const std::vector<RowScan> &scan, int most_fields, bool fold_drifts, std::vector<ufo::PairOp> &out,
                  int &cache_fields, bool &fma_ready, bool &mostly_general) {
   cache_fields = 0;
   fma_ready = true;
   int kicks = 0, general = 0;
-  struct Shared { int op, field; };
-  std::unordered_multimap<uint64_t, Shared> seen;  // constants' hash -> first op
+  std::vector<int> field_of(static_cast<size_t>(n_ops), -1);
   size_t head = 0;  // the current segment's header
   int64_t last_end = -1;  // where the constants of the last general teapot end
   auto open = [&](int first) {
     head = out.size();
     out.push_back({ufo::PV_SEGMENT, 0, first, first});
-  };
-  // the half and negative strengths formed on constants must be exact
-  auto plain_strength = [&](int at) {
-    for (int r = 0; r < n_seeds; ++r) {
-      const double k = std::fabs(table[r * stride + at]);
-      if (!(k == 0.0 || (k > 1e-280 && k < 1e280))) return false;
-    }
-    return true;
   };
   open(0);
   for (int i = 0; i < n_ops; ++i) {
@@ -1074,9 +1146,8 @@ bool decode_list(const int32_t *ops, int n_ops, const double *table, int64_t str
           return false;
         if ((k[2] >> 16) || (k[3] >> 16)) break;  // orders above 15
         const bool div = teapot && w[3] > 1 && ((flags >> ufo::SH_FINNER) & 3) == ufo::DF_DIV;
-        if ((pattern == 1 || pattern == 2) &&
-            !plain_strength(w[2] + (!teapot ? 0 : w[3] <= 1 ? 1 : div ? 5 : 2)))
-          break;
+        // the half and negative strengths formed on constants must be exact
+        if (!scan[static_cast<size_t>(i)].plain) break;
         op.a = teapot ? w[3] : i;
         op.b = pattern == 0 ? k[2] | k[3] << 16 : 0;
         if (!teapot) {
@@ -1089,9 +1160,7 @@ bool decode_list(const int32_t *ops, int n_ops, const double *table, int64_t str
         if (div) {
           form = ufo::DIV_GENERAL;
           const double *q = table + w[2] + 1;  // [A, d, 1/d, A/d]
-          shift = shift_form(q[1], q[2], negative);
-          for (int r = 1; r < n_seeds && shift; ++r)
-            if (q[r * stride + 1] != q[1] || q[r * stride + 2] != q[2]) shift = 0;
+          if (scan[static_cast<size_t>(i)].same) shift = shift_form(q[1], q[2], negative);
           if (shift) form = ufo::DIV_SHIFT;
         }
         op.head = (ufo::PV_TEAPOT + pattern + 4 * form + ((flags & ufo::F_WEAK) ? 12 : 0)) |
@@ -1155,34 +1224,15 @@ bool decode_list(const int32_t *ops, int n_ops, const double *table, int64_t str
       default: break;  // wires, dynamic kicks: the one-lane code
     }
     if (fields) {
-      const int64_t nc = op_consts(w);
-      auto row = [&](int which, int r) {
-        return table + r * stride + ops[static_cast<size_t>(which) * UFO_OP_WORDS + 2];
-      };
-      uint64_t h = 1469598103934665603ull ^ static_cast<uint64_t>(w[0] * 31 + flags);
-      for (int r = 0; r < n_seeds; ++r)
-        for (int64_t k = 0; k < nc; ++k) {
-          uint64_t bits;
-          std::memcpy(&bits, row(i, r) + k, sizeof bits);
-          h = (h ^ bits) * 1099511628211ull;
-          h ^= h >> 29;
-        }
-      int field = -1;
-      const auto range = seen.equal_range(h);
-      for (auto it = range.first; it != range.second && field < 0; ++it) {
-        const int32_t *v = ops + static_cast<size_t>(it->second.op) * UFO_OP_WORDS;
-        bool same = v[0] == w[0] && v[1] == flags;
-        for (int r = 0; r < n_seeds && same; ++r)
-          same = std::memcmp(row(it->second.op, r), row(i, r), sizeof(double) * nc) == 0;
-        if (same) field = it->second.field;
-      }
+      const int twin = scan[static_cast<size_t>(i)].twin;
+      const int field = twin >= 0 ? field_of[static_cast<size_t>(twin)] : -1;
       op.a = field;
       if (field < 0 && fields <= most_fields - cache_fields) {
         op.a = cache_fields;
         op.head |= ufo::PF_FILL;
-        seen.emplace(h, Shared{i, cache_fields});
         cache_fields += fields;
       }
+      field_of[static_cast<size_t>(i)] = op.a;
     }
     // A plain drift goes with the op before it (strict list): an op of its own
     // costs its dispatch, about 200 cycles beside the 129 of its arithmetic.
@@ -1225,9 +1275,10 @@ bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t str
   out.clear();
   const size_t fill_at = pair_fill_at(n_ops);
   fma_at = fill_at + n_ops + 1;
+  const std::vector<RowScan> scan = scan_rows(ops, n_ops, table, stride, n_seeds);
   for (const bool strict : {true, false}) {
     const size_t start = out.size();
-    if (!decode_list(ops, n_ops, table, stride, n_seeds, most_fields, strict, out, cache_fields,
+    if (!decode_list(ops, n_ops, table, scan, most_fields, strict, out, cache_fields,
                      fma_ready, mostly_general))
       return false;
     const size_t end = out.size();
@@ -2058,6 +2109,7 @@ extern "C" int ufo_graph_create(ufo_ctx *ctx, const ufo_prog *prog, const double
   if (use_pair(ctx, prog, n, mode, flags, d_pturns != nullptr)) {  // nothing may be allocated under capture
     // enough for a launch with and without time slices
     ensure_cache(prog, 32 * ((n + 15) / 16), ctx->stream);
+    ensure_cache(prog, 32 * std::min((n + 15) / 16, int64_t{16} * ctx->sm_count), ctx->stream);
     UFO_CUDA(cudaStreamSynchronize(ctx->stream));
   }
   cudaStream_t cap;
