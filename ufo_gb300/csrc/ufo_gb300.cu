@@ -13,6 +13,10 @@
 // instruction the same whether 1 or 32 lanes are active.  This is the
 // reference's atomic work queue (ufo/track.py:110-112, ufo/sa.py:122-124) at
 // lane granularity instead of work-item granularity.
+//
+// pair.cuh holds the two-lane kernel (a particle's planes on neighbouring lanes),
+// which strict launches and small ones take: use_pair has the rule and its
+// measurements.
 #include <cuda_runtime.h>
 
 #include <algorithm>
