@@ -13,24 +13,9 @@
 #pragma once
 #include <cstdint>
 
+#include "opcodes.h"
+
 namespace ufo {
-
-enum : int {
-  OP_NOP = 0, OP_DRIFT, OP_KICK, OP_TEAPOT, OP_ALIGN, OP_EDGE, OP_THICKQ, OP_THICKB, OP_WIRE,
-  OP_APERTURE, OP_OBSERVE, OP_DYNKICK, OP_LINEAR
-};
-enum : int { DF_MUL = 0, DF_MUL2 = 1, DF_DIV = 2 };
-enum : int {
-  F_ACHRO = 1 << 0, F_EXACT = 1 << 1, F_WEAK = 1 << 2, F_RTPSI = 1 << 3, F_T1 = 1 << 4,
-  F_T2 = 1 << 5, F_CONST = 1 << 6, F_AX = 1 << 7, F_AY = 1 << 8, F_T1Z = 1 << 9,
-  F_T2Z = 1 << 10, F_WEAKZ = 1 << 11, F_YOSHIDA = 1 << 12, F_CIRCLE = 1 << 13, F_SPLITO = 1 << 14,
-  F_PSER = 1 << 15
-};
-constexpr int SH_FOUTER = 16, SH_FINNER = 18;
-
-struct Op {
-  int kind, flags, toff, i0, i1, i2, i3, i4;
-};
 
 #define UFO_DEV __device__ __forceinline__
 

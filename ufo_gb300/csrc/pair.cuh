@@ -28,6 +28,7 @@
 // the step from 64.7 to 114-115 cycles).  The code therefore keeps selects and
 // sign changes on constants and off the chain, and tests once per segment.
 #pragma once
+#include "pair_list.h"
 
 namespace ufo {
 
@@ -68,44 +69,6 @@ UFO_DEV double flip(double v, int bit) {
   return __hiloint2double(__double2hiint(v) ^ bit, __double2loint(v));
 }
 UFO_DEV double pick(bool first, double a, double b) { return first ? a : b; }
-
-// ---- opcode words of this kernel, built on the host (decode_pair)
-//   head  bits 0-7 variant, 8-15 exponent shift of div_shift, PF_* flags
-//   toff  first constant in the table row
-//   a     slices; first field in the coefficient cache (-1: none); observation
-//         index; first op of a segment in the public list
-//   b     general kicks: normal mask | skew mask << 16; end of the segment; with
-//         PF_THEN the first constant of a plain drift that follows the op
-struct PairOp {
-  int head, toff, a, b;
-};
-enum : int {
-  PF_NEG = 1 << 16,    // div_shift subtracts
-  PF_ACHRO = 1 << 17, PF_SPLITO = 1 << 18,
-  PF_X = 1 << 19, PF_Y = 1 << 20,  // the plane has the term (align, edge)
-  PF_CONST = 1 << 21, PF_PSER = 1 << 22,
-  PF_DIV = 1 << 23,    // the table holds [A, d, 1/d, A/d] for the inner drift
-  PF_FILL = 1 << 24,   // this op fills its cache fields
-  PF_THEN = 1 << 25,   // a plain drift follows, run with this op (strict list only)
-  // general teapots: the alignment shifts around them run with them (PF_X, PF_Y
-  // as in an align op), two dispatches fewer per magnet (FODO ring with errors,
-  // 1,000 particles, FMA 192 -> 183 us per turn, light-source ring 2,066 ->
-  // 1,907); their constants lie right before and after the element's, or
-  // (.._EDGE) beyond an empty edge's three
-  PF_PRE = 1 << 26, PF_POST = 1 << 27, PF_PRE_EDGE = 1 << 28, PF_POST_EDGE = 1 << 29
-};
-enum : int {
-  PV_SEGMENT = 0, PV_DRIFT, PV_DRIFT2, PV_DRIFT_DIV, PV_ALIGN, PV_EDGE, PV_EDGE_PSI, PV_THICKQ,
-  PV_THICKB, PV_CIRCLE, PV_OBSERVE, PV_LINEAR, PV_WIDE,
-  PV_KICK = 16,   // + pattern (0..3, see teapot in ops.cuh)
-  PV_TEAPOT = 20  // + pattern (0..3) + 4 * division form (0..2) + 12 * weak
-};
-constexpr int PAIR_SEGMENT = 16;
-// forms of the inner drift of a teapot: x += px L; x += (px A) / d with one
-// FMA (see div_shift); the same by Markstein's correction (divc)
-enum : int { DIV_NONE = 0, DIV_SHIFT = 1, DIV_GENERAL = 2, DIV_ANY = 3 };
-// cached fields of a thick element, per lane
-enum : int { TC_C = 0, TC_S, TC_K, TC_R, TC_Z, TC_D, TC_DP, TC_FIELDS };
 
 // Correctly rounded a / d for a small integer d with one FMA: q = RN(a r + u),
 // r = RN(1/d), u = +-a 2^-s (the exponent field moved, no FP64 instruction).

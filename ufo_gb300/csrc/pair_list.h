@@ -1,0 +1,363 @@
+// pair_list.h -- the two-lane kernel's opcode list and its host side: which form
+// an op takes, made from the public opcodes and constants.  Plain C++, so that a
+// CPU test can read what the kernel (pair.cuh) is going to walk.
+#pragma once
+#include <cmath>
+#include <cstring>
+#include <unordered_map>
+#include <vector>
+
+#include "../../include/ufo_gb300.h"
+#include "opcodes.h"
+
+namespace ufo {
+
+// ---- opcode words of this kernel, built on the host (decode_pair)
+//   head  bits 0-7 variant, 8-15 exponent shift of div_shift, PF_* flags
+//   toff  first constant in the table row
+//   a     slices; first field in the coefficient cache (-1: none); observation
+//         index; first op of a segment in the public list
+//   b     general kicks: normal mask | skew mask << 16; end of the segment; with
+//         PF_THEN the first constant of a plain drift that follows the op
+struct PairOp {
+  int head, toff, a, b;
+};
+enum : int {
+  PF_NEG = 1 << 16,    // div_shift subtracts
+  PF_ACHRO = 1 << 17, PF_SPLITO = 1 << 18,
+  PF_X = 1 << 19, PF_Y = 1 << 20,  // the plane has the term (align, edge)
+  PF_CONST = 1 << 21, PF_PSER = 1 << 22,
+  PF_DIV = 1 << 23,    // the table holds [A, d, 1/d, A/d] for the inner drift
+  PF_FILL = 1 << 24,   // this op fills its cache fields
+  PF_THEN = 1 << 25,   // a plain drift follows, run with this op (strict list only)
+  // general teapots: the alignment shifts around them run with them (PF_X, PF_Y
+  // as in an align op), two dispatches fewer per magnet (FODO ring with errors,
+  // 1,000 particles, FMA 192 -> 183 us per turn, light-source ring 2,066 ->
+  // 1,907); their constants lie right before and after the element's, or
+  // (.._EDGE) beyond an empty edge's three
+  PF_PRE = 1 << 26, PF_POST = 1 << 27, PF_PRE_EDGE = 1 << 28, PF_POST_EDGE = 1 << 29
+};
+enum : int {
+  PV_SEGMENT = 0, PV_DRIFT, PV_DRIFT2, PV_DRIFT_DIV, PV_ALIGN, PV_EDGE, PV_EDGE_PSI, PV_THICKQ,
+  PV_THICKB, PV_CIRCLE, PV_OBSERVE, PV_LINEAR, PV_WIDE,
+  PV_KICK = 16,   // + pattern (0..3, see teapot in ops.cuh)
+  PV_TEAPOT = 20  // + pattern (0..3) + 4 * division form (0..2) + 12 * weak
+};
+constexpr int PAIR_SEGMENT = 16;
+// forms of the inner drift of a teapot: x += px L; x += (px A) / d with one
+// FMA (see div_shift); the same by Markstein's correction (divc)
+enum : int { DIV_NONE = 0, DIV_SHIFT = 1, DIV_GENERAL = 2, DIV_ANY = 3 };
+// cached fields of a thick element, per lane
+enum : int { TC_C = 0, TC_S, TC_K, TC_R, TC_Z, TC_D, TC_DP, TC_FIELDS };
+
+// ------------------------------------------------ two-lane opcode list
+// The exponent shift of div_shift for the divisor d (RN(1/d) = r in the
+// table), or 0 when no power of two serves: with eps = (1/d - r) / ulp(r) and M
+// the significand of 1/d, the candidate k = +-2^-j must satisfy |k - eps| <
+// 1/(2 d') over operand significands up to 2/M (quotients below the next power
+// of two) and up to 2 halved (above it); 0.95 leaves room for the terms of
+// order 2^-53 that the bound drops.
+inline int shift_form(double d, double r, bool &negative) {
+  if (!(d > 1.0 && d < 1048576.0) || d != std::floor(d) || r != 1.0 / d) return 0;
+  long odd = static_cast<long>(d);
+  while (odd % 2 == 0) odd /= 2;
+  if (odd == 1) return 0;
+  int ez = 0;
+  const double m = 2.0 * std::frexp(r, &ez);  // r = m 2^(ez-1), m in [1, 2)
+  --ez;
+  const double eps = std::ldexp(std::fma(-d, r, 1.0) / d, 52 - ez);
+  negative = eps < 0.0;
+  const double bound = 0.95 / (2.0 * static_cast<double>(odd));
+  for (int j = 1; j <= 8; ++j) {
+    const double k = std::ldexp(negative ? -1.0 : 1.0, -j);
+    const double off = std::fabs(k - eps);
+    if (off * (2.0 / m) < bound && off < bound) return 52 + j - ez;
+  }
+  return 0;
+}
+
+// kick pattern of the interpreters (teapot in ops.cuh)
+inline int kick_pattern(int nn, int ns, int32_t mn) {
+  return ns != 0 ? 0 : (nn == 2 && mn == 2) ? 1 : (nn == 3 && mn == 4) ? 2 : mn == 0 ? 3 : 0;
+}
+
+// What the two-lane lists need to know of every row's constants, gathered in one
+// pass over the table row by row (op by op, each look misses the cache: 20,000
+// rows of 833 ops took 170 ms more at every new table).
+struct RowScan {
+  int strength = -1;     // where a short form's strength stands; -1: none
+  int division = -1;     // where an inner drift's [d, 1/d] stand; -1: none
+  bool plain = true;     // strengths whose half and negative are exact, in every row
+  bool same = true;      // the division is row 0's in every row
+  int twin = -1;         // an earlier op with the same cacheable constants in every row
+};
+
+inline bool plain_strength(double k) {
+  k = std::fabs(k);
+  return k == 0.0 || (k > 1e-280 && k < 1e280);
+}
+
+inline std::vector<RowScan> scan_rows(const int32_t *ops, int n_ops, const double *table, int64_t stride,
+                               int n_seeds) {
+  std::vector<RowScan> scan(static_cast<size_t>(n_ops));
+  std::vector<int> looked, twins;
+  std::unordered_multimap<uint64_t, int> seen;  // row 0's constants -> op
+  auto word = [&](int i) { return ops + static_cast<size_t>(i) * UFO_OP_WORDS; };
+  auto bytes = [&](int i) { return sizeof(double) * static_cast<size_t>(op_consts(word(i))); };
+  for (int i = 0; i < n_ops; ++i) {
+    const int32_t *w = word(i);
+    RowScan &s = scan[static_cast<size_t>(i)];
+    if (w[0] == OP_KICK ||
+        (w[0] == OP_TEAPOT && !(w[1] & (F_YOSHIDA | F_EXACT)))) {
+      const bool teapot = w[0] == OP_TEAPOT;
+      const bool div = teapot && w[3] > 1 && ((w[1] >> SH_FINNER) & 3) == DF_DIV;
+      const int pattern = kick_pattern(w[teapot ? 4 : 3], w[teapot ? 5 : 4], w[teapot ? 6 : 5]);
+      if (pattern == 1 || pattern == 2)
+        s.strength = w[2] + (!teapot ? 0 : w[3] <= 1 ? 1 : div ? 5 : 2);
+      if (div) s.division = w[2] + 2;
+      if (s.strength >= 0 || s.division >= 0) looked.push_back(i);
+    } else if (w[0] == OP_THICKQ || w[0] == OP_THICKB ||
+               (w[0] == OP_EDGE && (w[1] & F_RTPSI))) {
+      uint64_t h = 1469598103934665603ull ^ static_cast<uint64_t>(w[0] * 31 + w[1]);
+      for (int64_t k = 0; k < op_consts(w); ++k) {
+        uint64_t bits;
+        std::memcpy(&bits, table + w[2] + k, sizeof bits);
+        h = (h ^ bits) * 1099511628211ull;
+        h ^= h >> 29;
+      }
+      const auto range = seen.equal_range(h);
+      for (auto it = range.first; it != range.second && s.twin < 0; ++it) {
+        const int32_t *v = word(it->second);
+        if (v[0] == w[0] && v[1] == w[1] &&
+            std::memcmp(table + v[2], table + w[2], bytes(i)) == 0)
+          s.twin = it->second;
+      }
+      if (s.twin < 0)
+        seen.emplace(h, i);
+      else
+        twins.push_back(i);
+    }
+  }
+  for (int r = 0; r < n_seeds; ++r) {
+    const double *row = table + static_cast<int64_t>(r) * stride;
+    for (const int i : looked) {
+      RowScan &s = scan[static_cast<size_t>(i)];
+      if (s.strength >= 0) s.plain = s.plain && plain_strength(row[s.strength]);
+      if (s.division >= 0)
+        s.same = s.same && row[s.division] == table[s.division] &&
+                 row[s.division + 1] == table[s.division + 1];
+    }
+    for (size_t k = 0; r > 0 && k < twins.size();) {
+      const int i = twins[k];
+      RowScan &s = scan[static_cast<size_t>(i)];
+      if (std::memcmp(row + word(s.twin)[2], row + word(i)[2], bytes(i)) == 0) {
+        ++k;
+      } else {  // on its own from here
+        s.twin = -1;
+        twins[k] = twins.back();
+        twins.pop_back();
+      }
+    }
+  }
+  return scan;
+}
+
+// where a list's cache-filling ops start
+inline size_t pair_fill_at(int n_ops) { return 2 * static_cast<size_t>(n_ops) + 4; }
+
+// Translate a validated opcode list for the two-lane kernel; false when an op
+// has no two-lane form worth its name (Yoshida and exact-drift elements, which
+// would run as one-lane code on half-empty warps).  Structurally empty ops
+// (zero-angle edges) are left out: they matter to non-finite coordinates alone.
+// Thick elements and fringe edges with the same constants in every row share
+// their cache fields; at most `most_fields` are given out, and further elements
+// compute in every turn.  `fma_ready`: the general kicks carry the dense series
+// that the FMA kernel reads.
+inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
+                        const std::vector<RowScan> &scan, int most_fields, bool fold_drifts,
+                        std::vector<PairOp> &out, int &cache_fields, bool &fma_ready,
+                        bool &mostly_general) {
+  cache_fields = 0;
+  fma_ready = true;
+  int kicks = 0, general = 0;
+  std::vector<int> field_of(static_cast<size_t>(n_ops), -1);
+  size_t head = 0;  // the current segment's header
+  int64_t last_end = -1;  // where the constants of the last general teapot end
+  auto open = [&](int first) {
+    head = out.size();
+    out.push_back({PV_SEGMENT, 0, first, first});
+  };
+  open(0);
+  for (int i = 0; i < n_ops; ++i) {
+    const int32_t *w = ops + static_cast<size_t>(i) * UFO_OP_WORDS;
+    const int flags = w[1];
+    const int common = (flags & F_ACHRO) ? PF_ACHRO : 0;
+    PairOp op{PV_WIDE, w[2], i, 0};
+    int fields = 0;
+    bool keep = true;
+    switch (w[0]) {
+      case OP_NOP: keep = false; break;
+      case OP_DRIFT:
+        if (flags & F_EXACT) return false;
+        op.head = w[3] == DF_MUL ? PV_DRIFT
+                  : w[3] == DF_MUL2 ? PV_DRIFT2 : PV_DRIFT_DIV;
+        break;
+      case OP_KICK:
+      case OP_TEAPOT: {
+        const bool teapot = w[0] == OP_TEAPOT;
+        const int32_t *k = w + (teapot ? 4 : 3);  // nn, ns, mn, ms
+        const int pattern = (k[2] | k[3]) ? kick_pattern(k[0], k[1], k[2]) : 3;
+        if (pattern == 0 && !(flags & F_PSER)) fma_ready = false;
+        ++kicks;
+        general += pattern == 0;
+        if (teapot && (flags & (F_EXACT | F_YOSHIDA))) return false;
+        if (teapot && (((flags >> SH_FOUTER) & 3) != DF_MUL ||
+                       ((flags >> SH_FINNER) & 3) == DF_MUL2))
+          return false;
+        if ((k[2] >> 16) || (k[3] >> 16)) break;  // orders above 15
+        const bool div = teapot && w[3] > 1 && ((flags >> SH_FINNER) & 3) == DF_DIV;
+        // the half and negative strengths formed on constants must be exact
+        if (!scan[static_cast<size_t>(i)].plain) break;
+        op.a = teapot ? w[3] : i;
+        op.b = pattern == 0 ? k[2] | k[3] << 16 : 0;
+        if (!teapot) {
+          if (pattern == 3) keep = false;
+          op.head = (PV_KICK + pattern) | common;
+          break;
+        }
+        int form = DIV_NONE, shift = 0;
+        bool negative = false;
+        if (div) {
+          form = DIV_GENERAL;
+          const double *q = table + w[2] + 1;  // [A, d, 1/d, A/d]
+          if (scan[static_cast<size_t>(i)].same) shift = shift_form(q[1], q[2], negative);
+          if (shift) form = DIV_SHIFT;
+        }
+        op.head = (PV_TEAPOT + pattern + 4 * form + ((flags & F_WEAK) ? 12 : 0)) |
+                  shift << 8 | (shift && negative ? PF_NEG : 0) | (div ? PF_DIV : 0) |
+                  ((flags & F_SPLITO) ? PF_SPLITO : 0) | common |
+                  ((flags & F_PSER) ? PF_PSER : 0);
+        if (pattern == 0) {
+          // the shift before a general teapot runs with it: see PF_PRE
+          last_end = w[2] + op_consts(w);
+          const PairOp &before = out.back();
+          const int gap = w[2] - before.toff;
+          if (out.size() - 1 > head && (before.head & 0xff) == PV_ALIGN &&
+              !(before.head & PF_THEN) && (gap == 2 || gap == 5)) {
+            op.head |= PF_PRE | (gap == 5 ? PF_PRE_EDGE : 0) |
+                       (before.head & (PF_X | PF_Y));
+            out.pop_back();
+          }
+        }
+        break;
+      }
+      case OP_ALIGN:
+        op.head = PV_ALIGN | ((flags & F_AX) ? PF_X : 0) |
+                  ((flags & F_AY) ? PF_Y : 0);
+        {  // the shift after a general teapot
+          PairOp &before = out.back();
+          const int variant = (before.head & 0xff) - PV_TEAPOT;
+          const int planes = op.head & (PF_X | PF_Y);
+          const int64_t gap = w[2] - last_end;
+          if (out.size() - 1 > head && variant >= 0 && variant % 4 == 0 &&
+              !(before.head & PF_POST) && (gap == 0 || gap == 3) &&
+              (!(before.head & PF_PRE) ||
+               (before.head & (PF_X | PF_Y)) == planes)) {
+            before.head |= PF_POST | (gap == 3 ? PF_POST_EDGE : 0) | planes;
+            keep = false;
+          }
+        }
+        break;
+      case OP_EDGE:
+        keep = flags & (F_T1 | F_T2 | F_RTPSI);
+        op.head = ((flags & F_RTPSI) ? PV_EDGE_PSI : PV_EDGE) | common |
+                  ((flags & F_T1) ? PF_X : 0) | ((flags & F_T2) ? PF_Y : 0);
+        if (flags & F_RTPSI) {
+          if (!(flags & F_T2)) return false;
+          fields = 1;
+        }
+        break;
+      case OP_THICKQ:
+      case OP_THICKB:
+        op.head = (w[0] == OP_THICKQ ? PV_THICKQ : PV_THICKB) | common |
+                  ((flags & F_CONST) ? PF_CONST : 0);
+        fields = w[0] == OP_THICKQ ? TC_D : TC_FIELDS;
+        break;
+      case OP_APERTURE:
+        if (flags & F_CIRCLE) op.head = PV_CIRCLE;
+        break;
+      case OP_OBSERVE:
+        op.head = PV_OBSERVE;
+        op.a = w[3];
+        break;
+      case OP_LINEAR: op.head = PV_LINEAR; break;
+      default: break;  // wires, dynamic kicks: the one-lane code
+    }
+    if (fields) {
+      const int twin = scan[static_cast<size_t>(i)].twin;
+      const int field = twin >= 0 ? field_of[static_cast<size_t>(twin)] : -1;
+      op.a = field;
+      if (field < 0 && fields <= most_fields - cache_fields) {
+        op.a = cache_fields;
+        op.head |= PF_FILL;
+        cache_fields += fields;
+      }
+      field_of[static_cast<size_t>(i)] = op.a;
+    }
+    // A plain drift goes with the op before it (strict list): an op of its own
+    // costs its dispatch, about 200 cycles beside the 129 of its arithmetic.
+    PairOp &before = out.back();
+    const int variant = before.head & 0xff;
+    if (fold_drifts && keep && op.head == PV_DRIFT && out.size() - 1 > head &&
+        !(before.head & PF_THEN) &&
+        (variant == PV_DRIFT || variant == PV_ALIGN || variant == PV_EDGE ||
+         variant == PV_EDGE_PSI || variant == PV_THICKQ || variant == PV_THICKB ||
+         (variant >= PV_TEAPOT && (variant - PV_TEAPOT) % 4 != 0))) {
+      before.head |= PF_THEN;
+      before.b = op.toff;
+      keep = false;
+    }
+    if (keep) {
+      // an op without a two-lane form is a segment of its own
+      const bool wide = op.head == PV_WIDE;
+      const int kept = static_cast<int>(out.size() - 1 - head);
+      if (kept > 0 && (wide || out.back().head == PV_WIDE || kept == PAIR_SEGMENT))
+        open(i);
+      out.push_back(op);
+    }
+    out[head].b = i + 1;
+  }
+  if (out[head].b > out[head].a) open(n_ops);  // the end
+  out.push_back({PV_SEGMENT, 0, 0, 0});   // the kernel fetches two ops ahead
+  out.push_back({PV_SEGMENT, 0, 0, 0});
+  mostly_general = 2 * general > kicks;
+  return true;
+}
+
+// Both lists, at fixed places whatever the constants make of them (a captured
+// graph keeps their addresses): the second at `fma_at`, each padded to two
+// entries per op -- every op a segment of its own -- and the ends, and followed
+// by the ops that fill the cache (pair_fill walks those alone: one turn of three
+// particles through 1,600 ops 997 us with the whole list, 893 us).
+inline bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t stride,
+                        int n_seeds, int most_fields, std::vector<PairOp> &out, size_t &fma_at,
+                        int &cache_fields, bool &fma_ready, bool &mostly_general) {
+  out.clear();
+  const size_t fill_at = pair_fill_at(n_ops);
+  fma_at = fill_at + n_ops + 1;
+  const std::vector<RowScan> scan = scan_rows(ops, n_ops, table, stride, n_seeds);
+  for (const bool strict : {true, false}) {
+    const size_t start = out.size();
+    if (!decode_list(ops, n_ops, table, scan, most_fields, strict, out, cache_fields,
+                     fma_ready, mostly_general))
+      return false;
+    const size_t end = out.size();
+    out.resize(start + fill_at);
+    for (size_t i = start; i < end; ++i)
+      if (out[i].head & PF_FILL) out.push_back(out[i]);
+    out.resize(start + fma_at);  // an end at least
+  }
+  return true;
+}
+
+}  // namespace ufo

@@ -28,7 +28,6 @@
 #include <cstring>
 #include <mutex>
 #include <new>
-#include <unordered_map>
 #include <vector>
 
 #include "../../include/ufo_gb300.h"
@@ -823,83 +822,9 @@ int ensure_constants(int device) {
 
 constexpr int DEFAULT_WARPS = 16;  // resident warps per SM of the persistent grid
 
-int popc32(uint32_t v) { return __builtin_popcount(v); }
-
-bool mask_fits(int n, int32_t mask) {
-  if (n < 0 || n > 32) return false;
-  const uint32_t m = static_cast<uint32_t>(mask);
-  return n == 32 || (m >> n) == 0u;
-}
-
-// constants of the dense power series of a general kick (F_PSER): 2 per
-// order up to the highest coefficient; -1 if the flag is set without one
-int64_t pser_consts(int flags, int32_t mn, int32_t ms) {
-  if (!(flags & ufo::F_PSER)) return 0;
-  const uint32_t m = static_cast<uint32_t>(mn) | static_cast<uint32_t>(ms);
-  if (m == 0u) return -1;
-  return 2 * static_cast<int64_t>(32 - __builtin_clz(m));
-}
-
-int drift_consts(int form, bool exact) {
-  if (exact) return 1;
-  return form == ufo::DF_MUL ? 1 : form == ufo::DF_MUL2 ? 2 : form == ufo::DF_DIV ? 4 : -1;
-}
-
-// Number of table constants an op reads (exactly what the kernels read), or
-// -1 if the op's shape is invalid.  Every op must fit inside the stride so
-// that no kernel read leaves its seed's row.
-int64_t op_consts(const int32_t *w) {
-  const int kind = w[0], flags = w[1];
-  const bool exact = flags & ufo::F_EXACT;
-  switch (kind) {
-    case ufo::OP_NOP:
-    case ufo::OP_OBSERVE:
-      return 0;
-    case ufo::OP_DRIFT:
-      return drift_consts(w[3], exact);
-    case ufo::OP_KICK: {
-      if (!mask_fits(w[3], w[5]) || !mask_fits(w[4], w[6])) return -1;
-      const int64_t ps = pser_consts(flags, w[5], w[6]);
-      if (ps < 0) return -1;
-      return popc32(w[5]) + popc32(w[6]) + ps;
-    }
-    case ufo::OP_TEAPOT: {
-      const int64_t ps = pser_consts(flags, w[6], w[7]);
-      if (ps < 0) return -1;
-      if (flags & ufo::F_YOSHIDA) {  // [4 drifts][3 weights][kick][W][series]
-        if (exact || w[3] < 1 || !mask_fits(w[4], w[6]) || !mask_fits(w[5], w[7])) return -1;
-        return 7 + popc32(w[6]) + popc32(w[7]) + ((flags & ufo::F_WEAK) ? 1 : 0) + ps;
-      }
-      if (w[3] < 1 || !mask_fits(w[4], w[6]) || !mask_fits(w[5], w[7])) return -1;
-      if ((flags & ufo::F_PSER) && exact) return -1;
-      const int fo = (flags >> ufo::SH_FOUTER) & 3, fi = (flags >> ufo::SH_FINNER) & 3;
-      const int co = drift_consts(fo, exact), ci = w[3] > 1 ? drift_consts(fi, exact) : 0;
-      if (co < 0 || ci < 0) return -1;
-      return co + ci + popc32(w[6]) + popc32(w[7]) + ((flags & ufo::F_WEAK) ? 1 : 0) +
-             ((flags & ufo::F_SPLITO) ? 1 : 0) + ps;
-    }
-    case ufo::OP_ALIGN:
-      return 2;
-    case ufo::OP_EDGE:
-      return (flags & ufo::F_RTPSI) ? 6 : 3;
-    case ufo::OP_THICKQ:
-      return (flags & ufo::F_CONST) ? 7 : 2;
-    case ufo::OP_THICKB:
-      return (flags & ufo::F_CONST) ? 16 : 3;
-    case ufo::OP_WIRE:
-      return 3;
-    case ufo::OP_APERTURE:
-      if (flags & ufo::F_CIRCLE) return 1;
-      return w[3] >= 0 ? 2 * static_cast<int64_t>(w[3]) : -1;
-    case ufo::OP_DYNKICK:
-      if (w[3] < 0 || w[4] < 0 || w[3] > 32 || w[4] > 32 || w[5] < w[3] + w[4]) return -1;
-      return w[5];
-    case ufo::OP_LINEAR:
-      return 5;
-    default:
-      return -1;
-  }
-}
+using ufo::decode_pair;
+using ufo::op_consts;
+using ufo::pair_fill_at;
 
 // simulate an expression stack program (row 0 of the table; the opcodes are
 // the same in every row): every pop must find an operand and the depth must
@@ -983,315 +908,6 @@ int validate_ops(const int32_t *ops, int n_ops, int64_t stride, int n_dumps,
       return fail(UFO_E_ARG, "op %d: malformed dynamic-kick programs", i);
   }
   return UFO_OK;
-}
-
-// ------------------------------------------------ two-lane opcode list
-// The exponent shift of div_shift for the divisor d (RN(1/d) = r in the
-// table), or 0 when no power of two serves: with eps = (1/d - r) / ulp(r) and M
-// the significand of 1/d, the candidate k = +-2^-j must satisfy |k - eps| <
-// 1/(2 d') over operand significands up to 2/M (quotients below the next power
-// of two) and up to 2 halved (above it); 0.95 leaves room for the terms of
-// order 2^-53 that the bound drops.
-int shift_form(double d, double r, bool &negative) {
-  if (!(d > 1.0 && d < 1048576.0) || d != std::floor(d) || r != 1.0 / d) return 0;
-  long odd = static_cast<long>(d);
-  while (odd % 2 == 0) odd /= 2;
-  if (odd == 1) return 0;
-  int ez = 0;
-  const double m = 2.0 * std::frexp(r, &ez);  // r = m 2^(ez-1), m in [1, 2)
-  --ez;
-  const double eps = std::ldexp(std::fma(-d, r, 1.0) / d, 52 - ez);
-  negative = eps < 0.0;
-  const double bound = 0.95 / (2.0 * static_cast<double>(odd));
-  for (int j = 1; j <= 8; ++j) {
-    const double k = std::ldexp(negative ? -1.0 : 1.0, -j);
-    const double off = std::fabs(k - eps);
-    if (off * (2.0 / m) < bound && off < bound) return 52 + j - ez;
-  }
-  return 0;
-}
-
-// kick pattern of the interpreters (teapot in ops.cuh)
-int kick_pattern(int nn, int ns, int32_t mn) {
-  return ns != 0 ? 0 : (nn == 2 && mn == 2) ? 1 : (nn == 3 && mn == 4) ? 2 : mn == 0 ? 3 : 0;
-}
-
-// What the two-lane lists need to know of every row's constants, gathered in one
-// pass over the table row by row (op by op, each look misses the cache: 20,000
-// rows of 833 ops took 170 ms more at every new table).
-struct RowScan {
-  int strength = -1;     // where a short form's strength stands; -1: none
-  int division = -1;     // where an inner drift's [d, 1/d] stand; -1: none
-  bool plain = true;     // strengths whose half and negative are exact, in every row
-  bool same = true;      // the division is row 0's in every row
-  int twin = -1;         // an earlier op with the same cacheable constants in every row
-};
-
-bool plain_strength(double k) {
-  k = std::fabs(k);
-  return k == 0.0 || (k > 1e-280 && k < 1e280);
-}
-
-std::vector<RowScan> scan_rows(const int32_t *ops, int n_ops, const double *table, int64_t stride,
-                               int n_seeds) {
-  std::vector<RowScan> scan(static_cast<size_t>(n_ops));
-  std::vector<int> looked, twins;
-  std::unordered_multimap<uint64_t, int> seen;  // row 0's constants -> op
-  auto word = [&](int i) { return ops + static_cast<size_t>(i) * UFO_OP_WORDS; };
-  auto bytes = [&](int i) { return sizeof(double) * static_cast<size_t>(op_consts(word(i))); };
-  for (int i = 0; i < n_ops; ++i) {
-    const int32_t *w = word(i);
-    RowScan &s = scan[static_cast<size_t>(i)];
-    if (w[0] == ufo::OP_KICK ||
-        (w[0] == ufo::OP_TEAPOT && !(w[1] & (ufo::F_YOSHIDA | ufo::F_EXACT)))) {
-      const bool teapot = w[0] == ufo::OP_TEAPOT;
-      const bool div = teapot && w[3] > 1 && ((w[1] >> ufo::SH_FINNER) & 3) == ufo::DF_DIV;
-      const int pattern = kick_pattern(w[teapot ? 4 : 3], w[teapot ? 5 : 4], w[teapot ? 6 : 5]);
-      if (pattern == 1 || pattern == 2)
-        s.strength = w[2] + (!teapot ? 0 : w[3] <= 1 ? 1 : div ? 5 : 2);
-      if (div) s.division = w[2] + 2;
-      if (s.strength >= 0 || s.division >= 0) looked.push_back(i);
-    } else if (w[0] == ufo::OP_THICKQ || w[0] == ufo::OP_THICKB ||
-               (w[0] == ufo::OP_EDGE && (w[1] & ufo::F_RTPSI))) {
-      uint64_t h = 1469598103934665603ull ^ static_cast<uint64_t>(w[0] * 31 + w[1]);
-      for (int64_t k = 0; k < op_consts(w); ++k) {
-        uint64_t bits;
-        std::memcpy(&bits, table + w[2] + k, sizeof bits);
-        h = (h ^ bits) * 1099511628211ull;
-        h ^= h >> 29;
-      }
-      const auto range = seen.equal_range(h);
-      for (auto it = range.first; it != range.second && s.twin < 0; ++it) {
-        const int32_t *v = word(it->second);
-        if (v[0] == w[0] && v[1] == w[1] &&
-            std::memcmp(table + v[2], table + w[2], bytes(i)) == 0)
-          s.twin = it->second;
-      }
-      if (s.twin < 0)
-        seen.emplace(h, i);
-      else
-        twins.push_back(i);
-    }
-  }
-  for (int r = 0; r < n_seeds; ++r) {
-    const double *row = table + static_cast<int64_t>(r) * stride;
-    for (const int i : looked) {
-      RowScan &s = scan[static_cast<size_t>(i)];
-      if (s.strength >= 0) s.plain = s.plain && plain_strength(row[s.strength]);
-      if (s.division >= 0)
-        s.same = s.same && row[s.division] == table[s.division] &&
-                 row[s.division + 1] == table[s.division + 1];
-    }
-    for (size_t k = 0; r > 0 && k < twins.size();) {
-      const int i = twins[k];
-      RowScan &s = scan[static_cast<size_t>(i)];
-      if (std::memcmp(row + word(s.twin)[2], row + word(i)[2], bytes(i)) == 0) {
-        ++k;
-      } else {  // on its own from here
-        s.twin = -1;
-        twins[k] = twins.back();
-        twins.pop_back();
-      }
-    }
-  }
-  return scan;
-}
-
-// where a list's cache-filling ops start
-size_t pair_fill_at(int n_ops) { return 2 * static_cast<size_t>(n_ops) + 4; }
-
-// Translate a validated opcode list for the two-lane kernel; false when an op
-// has no two-lane form worth its name (Yoshida and exact-drift elements, which
-// would run as one-lane code on half-empty warps).  Structurally empty ops
-// (zero-angle edges) are left out: they matter to non-finite coordinates alone.
-// Thick elements and fringe edges with the same constants in every row share
-// their cache fields; at most `most_fields` are given out, and further elements
-// compute in every turn.  `fma_ready`: the general kicks carry the dense series
-// that the FMA kernel reads.
-bool decode_list(const int32_t *ops, int n_ops, const double *table,
-                 const std::vector<RowScan> &scan, int most_fields, bool fold_drifts, std::vector<ufo::PairOp> &out,
-                 int &cache_fields, bool &fma_ready, bool &mostly_general) {
-  cache_fields = 0;
-  fma_ready = true;
-  int kicks = 0, general = 0;
-  std::vector<int> field_of(static_cast<size_t>(n_ops), -1);
-  size_t head = 0;  // the current segment's header
-  int64_t last_end = -1;  // where the constants of the last general teapot end
-  auto open = [&](int first) {
-    head = out.size();
-    out.push_back({ufo::PV_SEGMENT, 0, first, first});
-  };
-  open(0);
-  for (int i = 0; i < n_ops; ++i) {
-    const int32_t *w = ops + static_cast<size_t>(i) * UFO_OP_WORDS;
-    const int flags = w[1];
-    const int common = (flags & ufo::F_ACHRO) ? ufo::PF_ACHRO : 0;
-    ufo::PairOp op{ufo::PV_WIDE, w[2], i, 0};
-    int fields = 0;
-    bool keep = true;
-    switch (w[0]) {
-      case ufo::OP_NOP: keep = false; break;
-      case ufo::OP_DRIFT:
-        if (flags & ufo::F_EXACT) return false;
-        op.head = w[3] == ufo::DF_MUL ? ufo::PV_DRIFT
-                  : w[3] == ufo::DF_MUL2 ? ufo::PV_DRIFT2 : ufo::PV_DRIFT_DIV;
-        break;
-      case ufo::OP_KICK:
-      case ufo::OP_TEAPOT: {
-        const bool teapot = w[0] == ufo::OP_TEAPOT;
-        const int32_t *k = w + (teapot ? 4 : 3);  // nn, ns, mn, ms
-        const int pattern = (k[2] | k[3]) ? kick_pattern(k[0], k[1], k[2]) : 3;
-        if (pattern == 0 && !(flags & ufo::F_PSER)) fma_ready = false;
-        ++kicks;
-        general += pattern == 0;
-        if (teapot && (flags & (ufo::F_EXACT | ufo::F_YOSHIDA))) return false;
-        if (teapot && (((flags >> ufo::SH_FOUTER) & 3) != ufo::DF_MUL ||
-                       ((flags >> ufo::SH_FINNER) & 3) == ufo::DF_MUL2))
-          return false;
-        if ((k[2] >> 16) || (k[3] >> 16)) break;  // orders above 15
-        const bool div = teapot && w[3] > 1 && ((flags >> ufo::SH_FINNER) & 3) == ufo::DF_DIV;
-        // the half and negative strengths formed on constants must be exact
-        if (!scan[static_cast<size_t>(i)].plain) break;
-        op.a = teapot ? w[3] : i;
-        op.b = pattern == 0 ? k[2] | k[3] << 16 : 0;
-        if (!teapot) {
-          if (pattern == 3) keep = false;
-          op.head = (ufo::PV_KICK + pattern) | common;
-          break;
-        }
-        int form = ufo::DIV_NONE, shift = 0;
-        bool negative = false;
-        if (div) {
-          form = ufo::DIV_GENERAL;
-          const double *q = table + w[2] + 1;  // [A, d, 1/d, A/d]
-          if (scan[static_cast<size_t>(i)].same) shift = shift_form(q[1], q[2], negative);
-          if (shift) form = ufo::DIV_SHIFT;
-        }
-        op.head = (ufo::PV_TEAPOT + pattern + 4 * form + ((flags & ufo::F_WEAK) ? 12 : 0)) |
-                  shift << 8 | (shift && negative ? ufo::PF_NEG : 0) | (div ? ufo::PF_DIV : 0) |
-                  ((flags & ufo::F_SPLITO) ? ufo::PF_SPLITO : 0) | common |
-                  ((flags & ufo::F_PSER) ? ufo::PF_PSER : 0);
-        if (pattern == 0) {
-          // the shift before a general teapot runs with it: see PF_PRE
-          last_end = w[2] + op_consts(w);
-          const ufo::PairOp &before = out.back();
-          const int gap = w[2] - before.toff;
-          if (out.size() - 1 > head && (before.head & 0xff) == ufo::PV_ALIGN &&
-              !(before.head & ufo::PF_THEN) && (gap == 2 || gap == 5)) {
-            op.head |= ufo::PF_PRE | (gap == 5 ? ufo::PF_PRE_EDGE : 0) |
-                       (before.head & (ufo::PF_X | ufo::PF_Y));
-            out.pop_back();
-          }
-        }
-        break;
-      }
-      case ufo::OP_ALIGN:
-        op.head = ufo::PV_ALIGN | ((flags & ufo::F_AX) ? ufo::PF_X : 0) |
-                  ((flags & ufo::F_AY) ? ufo::PF_Y : 0);
-        {  // the shift after a general teapot
-          ufo::PairOp &before = out.back();
-          const int variant = (before.head & 0xff) - ufo::PV_TEAPOT;
-          const int planes = op.head & (ufo::PF_X | ufo::PF_Y);
-          const int64_t gap = w[2] - last_end;
-          if (out.size() - 1 > head && variant >= 0 && variant % 4 == 0 &&
-              !(before.head & ufo::PF_POST) && (gap == 0 || gap == 3) &&
-              (!(before.head & ufo::PF_PRE) ||
-               (before.head & (ufo::PF_X | ufo::PF_Y)) == planes)) {
-            before.head |= ufo::PF_POST | (gap == 3 ? ufo::PF_POST_EDGE : 0) | planes;
-            keep = false;
-          }
-        }
-        break;
-      case ufo::OP_EDGE:
-        keep = flags & (ufo::F_T1 | ufo::F_T2 | ufo::F_RTPSI);
-        op.head = ((flags & ufo::F_RTPSI) ? ufo::PV_EDGE_PSI : ufo::PV_EDGE) | common |
-                  ((flags & ufo::F_T1) ? ufo::PF_X : 0) | ((flags & ufo::F_T2) ? ufo::PF_Y : 0);
-        if (flags & ufo::F_RTPSI) {
-          if (!(flags & ufo::F_T2)) return false;
-          fields = 1;
-        }
-        break;
-      case ufo::OP_THICKQ:
-      case ufo::OP_THICKB:
-        op.head = (w[0] == ufo::OP_THICKQ ? ufo::PV_THICKQ : ufo::PV_THICKB) | common |
-                  ((flags & ufo::F_CONST) ? ufo::PF_CONST : 0);
-        fields = w[0] == ufo::OP_THICKQ ? ufo::TC_D : ufo::TC_FIELDS;
-        break;
-      case ufo::OP_APERTURE:
-        if (flags & ufo::F_CIRCLE) op.head = ufo::PV_CIRCLE;
-        break;
-      case ufo::OP_OBSERVE:
-        op.head = ufo::PV_OBSERVE;
-        op.a = w[3];
-        break;
-      case ufo::OP_LINEAR: op.head = ufo::PV_LINEAR; break;
-      default: break;  // wires, dynamic kicks: the one-lane code
-    }
-    if (fields) {
-      const int twin = scan[static_cast<size_t>(i)].twin;
-      const int field = twin >= 0 ? field_of[static_cast<size_t>(twin)] : -1;
-      op.a = field;
-      if (field < 0 && fields <= most_fields - cache_fields) {
-        op.a = cache_fields;
-        op.head |= ufo::PF_FILL;
-        cache_fields += fields;
-      }
-      field_of[static_cast<size_t>(i)] = op.a;
-    }
-    // A plain drift goes with the op before it (strict list): an op of its own
-    // costs its dispatch, about 200 cycles beside the 129 of its arithmetic.
-    ufo::PairOp &before = out.back();
-    const int variant = before.head & 0xff;
-    if (fold_drifts && keep && op.head == ufo::PV_DRIFT && out.size() - 1 > head &&
-        !(before.head & ufo::PF_THEN) &&
-        (variant == ufo::PV_DRIFT || variant == ufo::PV_ALIGN || variant == ufo::PV_EDGE ||
-         variant == ufo::PV_EDGE_PSI || variant == ufo::PV_THICKQ || variant == ufo::PV_THICKB ||
-         (variant >= ufo::PV_TEAPOT && (variant - ufo::PV_TEAPOT) % 4 != 0))) {
-      before.head |= ufo::PF_THEN;
-      before.b = op.toff;
-      keep = false;
-    }
-    if (keep) {
-      // an op without a two-lane form is a segment of its own
-      const bool wide = op.head == ufo::PV_WIDE;
-      const int kept = static_cast<int>(out.size() - 1 - head);
-      if (kept > 0 && (wide || out.back().head == ufo::PV_WIDE || kept == ufo::PAIR_SEGMENT))
-        open(i);
-      out.push_back(op);
-    }
-    out[head].b = i + 1;
-  }
-  if (out[head].b > out[head].a) open(n_ops);  // the end
-  out.push_back({ufo::PV_SEGMENT, 0, 0, 0});   // the kernel fetches two ops ahead
-  out.push_back({ufo::PV_SEGMENT, 0, 0, 0});
-  mostly_general = 2 * general > kicks;
-  return true;
-}
-
-// Both lists, at fixed places whatever the constants make of them (a captured
-// graph keeps their addresses): the second at `fma_at`, each padded to two
-// entries per op -- every op a segment of its own -- and the ends, and followed
-// by the ops that fill the cache (pair_fill walks those alone: one turn of three
-// particles through 1,600 ops 997 us with the whole list, 893 us).
-bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t stride, int n_seeds,
-                 int most_fields, std::vector<ufo::PairOp> &out, size_t &fma_at,
-                 int &cache_fields, bool &fma_ready, bool &mostly_general) {
-  out.clear();
-  const size_t fill_at = pair_fill_at(n_ops);
-  fma_at = fill_at + n_ops + 1;
-  const std::vector<RowScan> scan = scan_rows(ops, n_ops, table, stride, n_seeds);
-  for (const bool strict : {true, false}) {
-    const size_t start = out.size();
-    if (!decode_list(ops, n_ops, table, scan, most_fields, strict, out, cache_fields,
-                     fma_ready, mostly_general))
-      return false;
-    const size_t end = out.size();
-    out.resize(start + fill_at);
-    for (size_t i = start; i < end; ++i)
-      if (out[i].head & ufo::PF_FILL) out.push_back(out[i]);
-    out.resize(start + fma_at);  // an end at least
-  }
-  return true;
 }
 
 // Chunk hand-out order of the compacting kernel: c -> (c * m) mod n_chunks
