@@ -1,0 +1,101 @@
+"""The two-lane kernel's opcode lists and launch plans on the CPU: what the
+kernel is going to walk stays within the coefficient cache and the table."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import helpers as H
+
+OP_DRIFT, OP_KICK, OP_TEAPOT, OP_ALIGN, OP_EDGE, OP_THICKQ, OP_THICKB = 1, 2, 3, 4, 5, 6, 7
+OP_APERTURE, OP_OBSERVE, OP_DYNKICK = 9, 10, 11
+PV_SEGMENT, PV_EDGE_PSI, PV_THICKQ, PV_THICKB, PV_OBSERVE, PV_WIDE = 0, 6, 7, 8, 10, 12
+PF_FILL = 1 << 24
+CACHED = {PV_THICKQ: 5, PV_THICKB: 7, PV_EDGE_PSI: 1}  # fields of the coefficient cache
+
+
+@pytest.fixture(scope='module')
+def host(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp('pair') / 'pair_list_host.so')
+    subprocess.run(['g++', '-std=c++17', '-O1', '-shared', '-fPIC', '-o', so,
+                    os.path.join(H.HERE, 'pair_list_host.cpp')], check=True)
+    return ctypes.CDLL(so)
+
+
+def decode(host, ops, table, most=2 ** 31 - 1):
+    """(strict list, FMA list, cache fields) of an opcode list and table."""
+    ops = np.ascontiguousarray(ops, np.int32).reshape(-1, 8)
+    table = np.ascontiguousarray(np.atleast_2d(table), np.float64)
+    out = np.zeros((8 * len(ops) + 64, 4), np.int32)
+    info = np.zeros(6, np.int64)
+    p = [a.ctypes.data_as(ctypes.c_void_p) for a in (ops, table, out, info)]
+    rc = host.pair_lists(p[0], len(ops), p[1], ctypes.c_int64(table.shape[1]), len(table),
+                         ctypes.c_int(most), p[2], ctypes.c_int64(out.size), p[3])
+    assert rc == 0 and info[0] == 1
+    out = out[:info[1]]
+    lists = []
+    for part in (out[:info[2]], out[info[2]:]):
+        part = part[:2 * len(ops) + 4]  # without the cache-filling ops
+        end = next(i for i, w in enumerate(part)
+                   if w[0] & 0xff == PV_SEGMENT and w[3] <= w[2])
+        lists.append(part[:end])
+    return lists[0], lists[1], int(info[3])
+
+
+def walk(lst, fields, stride, n_ops):
+    """Every entry reads constants of the row and, if cached, fields of the
+    cache; an op run by the one-lane code has its segment to itself; the
+    segments cover the opcode list."""
+    at, alone = 0, None
+    for head, toff, a, b in lst.tolist():
+        v = head & 0xff
+        assert 0 <= toff < stride
+        if v == PV_SEGMENT:
+            assert a == at and b > a
+            at, alone, count = b, None, 0
+            continue
+        count += 1
+        assert alone is None and (v != PV_WIDE or count == 1)
+        if v == PV_WIDE:
+            alone = True
+        if v in CACHED:
+            assert 0 <= a and a + CACHED[v] <= fields
+    assert at == n_ops
+
+
+def thick_quads(k1):
+    """A list of thick quadrupoles (constants k1, length), one row per row of k1."""
+    k1 = np.atleast_2d(k1)
+    n = k1.shape[1]
+    ops = [[OP_THICKQ, 0, 2 * i, 0, 0, 0, 0, 0] for i in range(n)]
+    table = np.zeros((len(k1), 2 * n))
+    table[:, 0::2], table[:, 1::2] = k1, 0.3
+    return ops, table
+
+
+def test_thick_elements_without_room_in_the_cache_run_one_lane(host):
+    """A captured launch keeps the cache's size.  Elements that shared an entry
+    and no longer do have none: they go through the one-lane code instead of
+    reading an entry that is not there."""
+    ops, table = thick_quads([[1.1] * 4] * 3)
+    strict, fma, fields = decode(host, ops, table)
+    assert fields == 5
+    apart = table.copy()
+    apart[1, 4] = 1.2  # the third quadrupole differs in one row
+    strict, fma, again = decode(host, ops, apart, most=fields)
+    assert again == fields
+    for lst in (strict, fma):
+        walk(lst, fields, table.shape[1], len(ops))
+        kinds = [h & 0xff for h in lst[:, 0]]
+        assert kinds.count(PV_THICKQ) == 3 and kinds.count(PV_WIDE) == 1
+        assert sum(bool(h & PF_FILL) for h in lst[:, 0]) == 1
+    # bends and fringe edges take what is left, or nothing
+    ops = [[OP_THICKQ, 0, 0, 0, 0, 0, 0, 0], [OP_THICKB, 0, 2, 0, 0, 0, 0, 0],
+           [OP_EDGE, 1 << 3 | 1 << 5, 5, 0, 0, 0, 0, 0], [OP_EDGE, 1 << 3 | 1 << 5, 11, 0, 0, 0, 0, 0]]
+    table = np.linspace(0.1, 1.0, 17)
+    for most in range(16):
+        strict, _, fields = decode(host, ops, table, most)
+        assert fields <= most
+        walk(strict, fields, 17, 4)

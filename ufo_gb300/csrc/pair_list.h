@@ -15,7 +15,7 @@ namespace ufo {
 // ---- opcode words of this kernel, built on the host (decode_pair)
 //   head  bits 0-7 variant, 8-15 exponent shift of div_shift, PF_* flags
 //   toff  first constant in the table row
-//   a     slices; first field in the coefficient cache (-1: none); observation
+//   a     slices; first field in the coefficient cache; observation
 //         index; first op of a segment in the public list
 //   b     general kicks: normal mask | skew mask << 16; end of the segment; with
 //         PF_THEN the first constant of a plain drift that follows the op
@@ -170,8 +170,9 @@ inline size_t pair_fill_at(int n_ops) { return 2 * static_cast<size_t>(n_ops) + 
 // would run as one-lane code on half-empty warps).  Structurally empty ops
 // (zero-angle edges) are left out: they matter to non-finite coordinates alone.
 // Thick elements and fringe edges with the same constants in every row share
-// their cache fields; at most `most_fields` are given out, and further elements
-// compute in every turn.  `fma_ready`: the general kicks carry the dense series
+// their cache fields; at most `most_fields` are given out, and an element that
+// gets none goes through the one-lane code, in a segment of its own.
+// `fma_ready`: the general kicks carry the dense series
 // that the FMA kernel reads.
 inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
                         const std::vector<RowScan> &scan, int most_fields, bool fold_drifts,
@@ -303,6 +304,7 @@ inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
         cache_fields += fields;
       }
       field_of[static_cast<size_t>(i)] = op.a;
+      if (op.a < 0) op = {PV_WIDE, w[2], i, 0};  // no room: by the one-lane code
     }
     // A plain drift goes with the op before it (strict list): an op of its own
     // costs its dispatch, about 200 cycles beside the 129 of its arithmetic.
