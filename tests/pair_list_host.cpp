@@ -1,6 +1,4 @@
 // The two-lane kernel's host side behind a C interface, for tests on the CPU.
-#include <algorithm>
-
 #include "../ufo_gb300/csrc/pair_list.h"
 
 extern "C" {
@@ -24,6 +22,16 @@ int pair_lists(const int32_t *ops, int n_ops, const double *table, int64_t strid
   if (static_cast<int64_t>(list.size()) * 4 > capacity) return -1;
   std::memcpy(out, list.data(), sizeof(ufo::PairOp) * list.size());
   return 0;
+}
+
+// groups, slices per group, turns per slice, warps per SM
+void pair_slices(int64_t n, int turns, int n_ops, int sm_count, int most_warps,
+                 int64_t most_groups, int64_t *out) {
+  const ufo::SlicePlan p = ufo::slice_plan(n, turns, n_ops, sm_count, most_warps, most_groups);
+  out[0] = p.groups;
+  out[1] = p.count;
+  out[2] = p.turns;
+  out[3] = p.warps_per_sm;
 }
 
 }  // extern "C"

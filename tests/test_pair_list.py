@@ -99,3 +99,24 @@ def test_thick_elements_without_room_in_the_cache_run_one_lane(host):
         strict, _, fields = decode(host, ops, table, most)
         assert fields <= most
         walk(strict, fields, 17, 4)
+
+
+def slices(host, n, turns, n_ops, sms=152):
+    out = np.zeros(4, np.int64)
+    host.pair_slices(ctypes.c_int64(n), turns, n_ops, sms, 16, ctypes.c_int64(sms * 512),
+                     out.ctypes.data_as(ctypes.c_void_p))
+    return out.tolist()
+
+
+@pytest.mark.parametrize('n_ops', [0, 1, 16, 128, 8192, 1_000_000])
+@pytest.mark.parametrize('turns', [1, 2, 3, 1000, 2 ** 30, 2 ** 31 - 2, 2 ** 31 - 1])
+def test_slices_cover_every_turn_count(host, turns, n_ops):
+    """Every slice but the last is whole and the last is not empty, up to the
+    turn counts that stand for "until all are lost"."""
+    for n in (1, 152 * 8 * 16, 152 * 8 * 16 + 17, 38_912, 65_536):
+        groups, count, q, warps = slices(host, n, turns, n_ops)
+        if not groups:
+            continue
+        assert turns >= 2 and groups == (n + 15) // 16 and warps in (8, 12, 16)
+        assert count >= 1 and q >= 1 and (count - 1) * q < turns <= count * q
+        assert groups * count < 2 ** 63

@@ -2,6 +2,7 @@
 // an op takes, made from the public opcodes and constants.  Plain C++, so that a
 // CPU test can read what the kernel (pair.cuh) is going to walk.
 #pragma once
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <unordered_map>
@@ -360,6 +361,39 @@ inline bool decode_pair(const int32_t *ops, int n_ops, const double *table, int6
     out.resize(start + fma_at);  // an end at least
   }
   return true;
+}
+
+// Time slices (Slices in pair.cuh) for a two-lane launch of equal turns with
+// more groups of 16 particles than 8 warps per SM: as many warps as fill every
+// sub-partition evenly (a multiple of 4 per SM) and leave groups in hand.  Below
+// that a sub-partition's first and second warp hide each other's latency, so an
+// uneven second one costs nothing.  Measured (us per turn, strict, without ->
+// with): FODO ring 65,536 particles 434 -> 379, light-source ring 4,991 -> 4,259,
+// thick ring 1,948 -> 1,777, 30,000 particles of the FODO ring 182 -> 175.  The
+// one-lane kernel keeps whole runs: the 12 warps per SM that leave it groups in
+// hand cost it more than the even end gains (FMA, light-source ring 1,511 ->
+// 1,685).
+struct SlicePlan {
+  int groups = 0;  // 0: whole runs
+  int count = 0, turns = 0;  // slices per group, turns per slice
+  int warps_per_sm = 0;
+};
+
+inline SlicePlan slice_plan(int64_t n, int turns, int n_ops, int sm_count, int most_warps,
+                            int64_t most_groups) {
+  SlicePlan s;
+  const int64_t groups = (n + 15) / 16;
+  const int64_t w = std::min<int64_t>(most_warps, (groups - 1) / sm_count) / 4 * 4;
+  if (turns < 2 || w < 8 || groups > most_groups) return s;
+  s.groups = static_cast<int>(groups);
+  // slice length: a launch ends within about half a slice (a share of Q / 2T),
+  // and each slice costs about 5 us of exchange against some 0.6 us per op and
+  // turn: the sum is least near Q = sqrt(16 T / ops)
+  s.turns = std::max(1, static_cast<int>(std::sqrt(16.0 * turns / std::max(1, n_ops))));
+  // in 64 bits: turns near INT_MAX mean "until all are lost"
+  s.count = static_cast<int>((static_cast<int64_t>(turns) + s.turns - 1) / s.turns);
+  s.warps_per_sm = static_cast<int>(w);
+  return s;
 }
 
 }  // namespace ufo

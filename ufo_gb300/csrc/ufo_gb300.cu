@@ -1124,34 +1124,21 @@ void ensure_cache(const ufo_prog *prog, int64_t lanes, cudaStream_t stream) {
   prog->cache_lanes = lanes;
 }
 
-// Time slices (Slices in pair.cuh) for a two-lane launch of equal turns with
-// more groups than 8 warps per SM: as many warps as fill every sub-partition
-// evenly (a multiple of 4 per SM) and leave groups in hand.  Below that a
-// sub-partition's first and second warp hide each other's latency, so an uneven
-// second one costs nothing.  Measured (us per turn, strict, without -> with):
-// FODO ring 65,536 particles 434 -> 379, light-source ring 4,991 -> 4,259, thick
-// ring 1,948 -> 1,777, 30,000 particles of the FODO ring 182 -> 175.  The
-// one-lane kernel keeps whole runs: the 12 warps per SM that leave it groups in
-// hand cost it more than the even end gains (FMA, light-source ring 1,511 ->
-// 1,685).  Particles of a dynamic-aperture scan are lost early (the lane refill
-// serves them), and uneven turn counts run longest first.
+// Time slices for a two-lane launch (slice_plan has the rule).  Particles of a
+// dynamic-aperture scan are lost early (the lane refill serves them), and uneven
+// turn counts run longest first.
 ufo::Slices plan_slices(const ufo_ctx *ctx, const ufo::TrackArgs &a, int &warps_per_sm) {
   ufo::Slices s{};
-  const int64_t groups = (a.n + 15) / 16;
-  const int64_t most = std::min(16, 2 * warps_per_sm);
-  const int64_t w = std::min(most, (groups - 1) / ctx->sm_count) / 4 * 4;
-  const int64_t slots = static_cast<int64_t>(ctx->sm_count) * ufo::CTA_MAX_WARPS * 32;
-  if (a.mode != UFO_MODE_TRACK || a.pturns || !a.lost || !a.final_state || a.turns < 2 || w < 8 ||
-      groups > slots)
-    return s;
+  if (a.mode != UFO_MODE_TRACK || a.pturns || !a.lost || !a.final_state) return s;
+  const ufo::SlicePlan plan =
+      ufo::slice_plan(a.n, a.turns, a.n_ops, ctx->sm_count, std::min(16, 2 * warps_per_sm),
+                      static_cast<int64_t>(ctx->sm_count) * ufo::CTA_MAX_WARPS * 32);
+  if (!plan.groups) return s;
   s.claims = ctx->pool_seq;  // one word per lane of the largest compacting grid
-  s.groups = static_cast<int>(groups);
-  // slice length: a launch ends within about half a slice (a share of Q / 2T),
-  // and each slice costs about 5 us of exchange against some 0.6 us per op and
-  // turn: the sum is least near Q = sqrt(16 T / ops)
-  s.turns = std::max(1, static_cast<int>(std::sqrt(16.0 * a.turns / std::max(1, a.n_ops))));
-  s.count = (a.turns + s.turns - 1) / s.turns;
-  warps_per_sm = static_cast<int>(w);
+  s.groups = plan.groups;
+  s.count = plan.count;
+  s.turns = plan.turns;
+  warps_per_sm = plan.warps_per_sm;
   return s;
 }
 
