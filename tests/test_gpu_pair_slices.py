@@ -30,3 +30,23 @@ def test_launch_ends_when_every_particle_is_lost(turns, fma):
                  for f in (0, capi.UFO_TRACK_PLAIN))
     assert np.array_equal(got[1], want[1]) and 150 < got[1].max() <= 200
     assert np.array_equal(got[2], want[2], equal_nan=True)
+
+
+@pytest.mark.parametrize('turns', [2, 37, 4000])
+def test_finished_groups_are_passed_over_and_the_others_run_on(turns):
+    """A group of 16 whose particles are all lost is handed out no more; groups
+    with one survivor, in any of its places, run every turn."""
+    import ufo_gb300 as u
+    from ufo_gb300 import capi, compiler as C
+    ctx = u.context(0)
+    line = u.Line('r', [u.Quadrupole('q', length=0.2, k1=0.0, slices=4),
+                        u.Drift('d', length=0.8), u.Aperture('a', window='x*x + y*y < 1e-4')])
+    dp = capi.DeviceProgram(ctx, C.compile_line(line, u.KICK, where=[-1]))
+    n = 152 * 16 * 16 + 3
+    coords = growing(n, 60, np.random.default_rng(turns))
+    alive = np.arange(0, n, 83)  # every fifth group or so, in changing places
+    coords[alive, 1] = 0.0
+    got, want = (capi.track(ctx, dp, coords, turns, capi.UFO_MODE_TRACK, f, slots=0)
+                 for f in (0, capi.UFO_TRACK_PLAIN))
+    assert np.array_equal(got[1], want[1]) and np.all(got[1][alive] == turns)
+    assert np.array_equal(got[2], want[2], equal_nan=True)

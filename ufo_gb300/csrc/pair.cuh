@@ -825,9 +825,11 @@ __global__ void __launch_bounds__(32, 16) track_pair_kernel(const __grid_constan
 // run (high half).  Whoever raises the low half from 0 runs the group; a warp
 // that finds it raised leaves the slice to that runner, which goes on until the
 // count is back at 0.  So no warp waits for another, and every slice runs once,
-// in order.  The last slice runs to the end whatever its length.
+// in order.  The last slice runs to the end whatever its length.  A group whose
+// particles are all finished keeps its count raised, so its other slices are
+// passed over; the last group to finish moves the work counter past the end.
 struct Slices {
-  unsigned long long *claims;  // [groups], zero at launch
+  unsigned long long *claims;  // [groups], then the groups finished; zero at launch
   int groups, count, turns;    // slices per group, turns per slice
 };
 
@@ -862,6 +864,14 @@ UFO_DEV bool slice_more(const Slices &s, int group, int &done) {
   old = __shfl_sync(0xffffffffu, old, 0);
   ++done;
   return (old & 0xffffffffull) > 1;
+}
+
+// Every particle of a group has finished.
+UFO_DEV void slice_finish(const Slices &s, unsigned long long *queue) {
+  if ((threadIdx.x & 31) != 0) return;
+  const unsigned long long total = static_cast<unsigned long long>(s.groups) * s.count;
+  if (atomicAdd(s.claims + s.groups, 1ull) + 1 == static_cast<unsigned long long>(s.groups))
+    atomicMax(queue, total);
 }
 
 constexpr uint32_t SLICE_RUNNING = 0x80000000u;
@@ -932,6 +942,10 @@ __global__ void __launch_bounds__(32, 16)
           a.lost[p] = static_cast<uint32_t>(sh.turn[lane]) | (idle ? 0u : SLICE_RUNNING);
       }
       __syncwarp();
+      if (__all_sync(PAIR_ALL, idle)) {
+        slice_finish(s, a.queue);
+        break;
+      }
     } while (slice_more(s, group, done));
   }
 }

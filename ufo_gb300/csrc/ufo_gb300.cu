@@ -988,7 +988,7 @@ int launch_kernels(ufo::TrackArgs &a, bool full, bool pair, const ufo::Slices &s
            : ufo::track_kernel_cta<false, false><<<g, tpb, smem, stream>>>(a);
   } else if (slices.groups) {
     UFO_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), stream));
-    UFO_CUDA(cudaMemsetAsync(slices.claims, 0, sizeof(unsigned long long) * slices.groups, stream));
+    UFO_CUDA(cudaMemsetAsync(slices.claims, 0, sizeof(unsigned long long) * (slices.groups + 1), stream));
     const unsigned g = static_cast<unsigned>(sm_count * warps_per_sm);
     if (fma)
       ufo::track_pair_sliced<true><<<g, 32, 0, stream>>>(a, slices);
@@ -1132,9 +1132,10 @@ ufo::Slices plan_slices(const ufo_ctx *ctx, const ufo::TrackArgs &a, int &warps_
   if (a.mode != UFO_MODE_TRACK || a.pturns || !a.lost || !a.final_state) return s;
   const ufo::SlicePlan plan =
       ufo::slice_plan(a.n, a.turns, a.n_ops, ctx->sm_count, std::min(16, 2 * warps_per_sm),
-                      static_cast<int64_t>(ctx->sm_count) * ufo::CTA_MAX_WARPS * 32);
+                      static_cast<int64_t>(ctx->sm_count) * ufo::CTA_MAX_WARPS * 32 - 1);
   if (!plan.groups) return s;
-  s.claims = ctx->pool_seq;  // one word per lane of the largest compacting grid
+  // one word per lane of the largest compacting grid: the groups' and one more
+  s.claims = ctx->pool_seq;
   s.groups = plan.groups;
   s.count = plan.count;
   s.turns = plan.turns;
