@@ -1,0 +1,38 @@
+"""Edges of the differentiation kernels' inputs."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def forward(ops, tab, z0, tangent, n_ops=None, turns=1):
+    """ufo_diff_forward on device buffers; ``ops`` a device tensor."""
+    import torch
+    from ufo_gb300 import capi
+    dev = torch.device('cuda', 0)
+    n = len(z0)
+    tab = torch.as_tensor(np.atleast_2d(tab), device=dev)
+    z = torch.as_tensor(np.ascontiguousarray(z0, np.float64), device=dev)
+    o = torch.ones(n, dtype=torch.float64, device=dev)
+    out = torch.zeros((n, 20), dtype=torch.float64, device=dev)
+    rc = capi.load().ufo_diff_forward(
+        capi.ptr(ops.data_ptr()), ops.numel() // 8 if n_ops is None else n_ops,
+        capi.ptr(tab.data_ptr()), ctypes.c_int64(tab.shape[1]), None, 0, 0, n,
+        capi.ptr(z.data_ptr()), capi.ptr(o.data_ptr()), turns, turns, int(tangent), None,
+        capi.ptr(out.data_ptr()), capi.ptr(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize('tangent', [False, True])
+def test_an_empty_opcode_list_is_the_identity(tangent):
+    import torch
+    z0 = np.arange(20.0).reshape(5, 4)
+    ops = torch.zeros(8, dtype=torch.int32, device='cuda:0')
+    out = forward(ops, np.zeros(1), z0, tangent, n_ops=0, turns=3)
+    assert np.array_equal(out[:, :4], z0)
+    if tangent:
+        assert np.array_equal(out[:, 4:], np.tile(np.eye(4).ravel(), (5, 1)))

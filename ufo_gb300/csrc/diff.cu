@@ -731,7 +731,7 @@ __device__ __forceinline__ DOp fetch(const DOp *p) {
 template <bool TAPE>
 __device__ void turn_forward_pair(Half &h, const DiffArgs &a, const double *T0, double o,
                                   bool even, bool write, double *tape) {
-  DOp next = fetch(a.ops);
+  DOp next = a.n_ops > 0 ? fetch(a.ops) : DOp{};
   for (int i = 0; i < a.n_ops; ++i) {
     const DOp op = next;
     if (i + 1 < a.n_ops) next = fetch(a.ops + i + 1);
@@ -1107,7 +1107,7 @@ template <bool TAPE>
 __device__ void turn_forward_oct(Oct &s, const DiffArgs &a, const double *T0, double o,
                                  const OctLane &l, double *tape) {
   const bool even = l.even;
-  DOp next = fetch(a.ops);
+  DOp next = a.n_ops > 0 ? fetch(a.ops) : DOp{};
   for (int i = 0; i < a.n_ops; ++i) {
     const DOp op = next;
     if (i + 1 < a.n_ops) next = fetch(a.ops + i + 1);
