@@ -36,3 +36,24 @@ def test_an_empty_opcode_list_is_the_identity(tangent):
     assert np.array_equal(out[:, :4], z0)
     if tangent:
         assert np.array_equal(out[:, 4:], np.tile(np.eye(4).ravel(), (5, 1)))
+
+
+@pytest.mark.parametrize('tangent', [False, True])
+def test_the_opcode_list_needs_no_more_than_int_alignment(tangent):
+    """A list that starts 4, 8 or 12 bytes off a 16-byte boundary, as a slice of a
+    caller's array may."""
+    import torch
+    D_DRIFT, D_ALIGN = 1, 4
+    words = [[D_DRIFT, 0, 0, 0, 0, -1, 0, 0], [D_ALIGN, 0, 1, 0, 0, -1, 0, 0],
+             [D_DRIFT, 0, 3, 0, 0, -1, 0, 0]]
+    tab = [0.5, 1e-3, -2e-3, 0.25]
+    z0 = np.arange(28.0).reshape(7, 4)
+    want = z0.copy()
+    want[:, 0::2] = (z0[:, 0::2] + 0.5 * z0[:, 1::2] - np.array(tab[1:3])) + 0.25 * z0[:, 1::2]
+    for off in range(4):
+        store = torch.zeros(24 + off, dtype=torch.int32, device='cuda:0')
+        store[off:] = torch.tensor(words, dtype=torch.int32).flatten().to(store.device)
+        ops = store[off:]
+        assert ops.data_ptr() % 16 == 4 * off
+        out = forward(ops, tab, z0, tangent)
+        assert np.allclose(out[:, :4], want, rtol=1e-15, atol=1e-15)

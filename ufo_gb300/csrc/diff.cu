@@ -720,10 +720,12 @@ __device__ __forceinline__ void kick_elem_pair(Half &h, const double *c, bool tp
   }
 }
 
+// An opcode ahead of its use.  The list is the caller's, aligned like any int32
+// array: word by word.
 __device__ __forceinline__ DOp fetch(const DOp *p) {
-  const int4 v = __ldg(reinterpret_cast<const int4 *>(p));
-  const int4 w = __ldg(reinterpret_cast<const int4 *>(p) + 1);
-  return {v.x, v.y, v.z, v.w, w.x, w.y, w.z, w.w};
+  const int *w = reinterpret_cast<const int *>(p);
+  return {__ldg(w),     __ldg(w + 1), __ldg(w + 2), __ldg(w + 3),
+          __ldg(w + 4), __ldg(w + 5), __ldg(w + 6), __ldg(w + 7)};
 }
 
 // one turn forward of the pair; with TAPE the rich tape is written from `tape`
