@@ -120,3 +120,11 @@ def test_slices_cover_every_turn_count(host, turns, n_ops):
         assert turns >= 2 and groups == (n + 15) // 16 and warps in (8, 12, 16)
         assert count >= 1 and q >= 1 and (count - 1) * q < turns <= count * q
         assert groups * count < 2 ** 63
+
+
+def test_slices_end_where_whole_runs_refill_their_lanes(host):
+    """Up to 32 groups of 16 per SM."""
+    assert slices(host, 152 * 32 * 16, 1000, 128)[0] == 152 * 32
+    assert slices(host, 152 * 32 * 16 + 1, 1000, 128)[0] == 0
+    assert slices(host, 152 * 8 * 16, 1000, 128)[0] == 0
+    assert slices(host, 152 * 8 * 16 + 1, 1000, 128)[0] == 152 * 8 + 1

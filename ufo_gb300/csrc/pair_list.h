@@ -373,6 +373,14 @@ inline bool decode_pair(const int32_t *ops, int n_ops, const double *table, int6
 // one-lane kernel keeps whole runs: the 12 warps per SM that leave it groups in
 // hand cost it more than the even end gains (FMA, light-source ring 1,511 ->
 // 1,685).
+// At most 32 groups per SM.  A slice's group keeps its lanes, lost or not, while
+// a lane of a whole run takes the next particle: beams of which a part is lost
+// run longer in slices, and up to here (where the one-lane kernel holds them all
+// at once and refills nothing either) never longer than on that kernel.  Light-
+// source ring, 30 turns (ms: slices, whole runs, one-lane kernel): 77,824
+// particles of which 14 % survive 141, 79, 183, none lost 151, 150, 180; 262,144
+// particles 469, 122, 210 and 510, 524, 629; thick ring, 40 turns, 262,144
+// particles, 3 % survive 120, 52, 224.
 struct SlicePlan {
   int groups = 0;  // 0: whole runs
   int count = 0, turns = 0;  // slices per group, turns per slice
@@ -384,7 +392,7 @@ inline SlicePlan slice_plan(int64_t n, int turns, int n_ops, int sm_count, int m
   SlicePlan s;
   const int64_t groups = (n + 15) / 16;
   const int64_t w = std::min<int64_t>(most_warps, (groups - 1) / sm_count) / 4 * 4;
-  if (turns < 2 || w < 8 || groups > most_groups) return s;
+  if (turns < 2 || w < 8 || groups > std::min<int64_t>(most_groups, 32 * sm_count)) return s;
   s.groups = static_cast<int>(groups);
   // slice length: a launch ends within about half a slice (a share of Q / 2T),
   // and each slice costs about 5 us of exchange against some 0.6 us per op and
