@@ -128,3 +128,15 @@ def test_slices_end_where_whole_runs_refill_their_lanes(host):
     assert slices(host, 152 * 32 * 16 + 1, 1000, 128)[0] == 0
     assert slices(host, 152 * 8 * 16, 1000, 128)[0] == 0
     assert slices(host, 152 * 8 * 16 + 1, 1000, 128)[0] == 152 * 8 + 1
+
+
+def test_ops_without_constants_read_none(host):
+    """The kernel loads the first constant of the op ahead: an op that has none may
+    stand at the end of the row (offset = stride), where there is none to load."""
+    for kind, words in ((0, [0] * 5), (OP_OBSERVE, [0] * 5), (OP_APERTURE, [0] * 5),
+                        (OP_DYNKICK, [0] * 5), (OP_KICK, [1, 1, 0, 0, 0])):
+        ops = [[OP_DRIFT, 0, 0, 0, 0, 0, 0, 0], [kind, 0, 1, *words], [OP_DRIFT, 0, 0, 0, 0, 0, 0, 0]]
+        strict, fma, fields = decode(host, ops, [0.5])
+        for lst in (strict, fma):
+            walk(lst, fields, 1, 3)
+            assert sum((h & 0xff) == PV_OBSERVE for h in lst[:, 0]) == (kind == OP_OBSERVE)

@@ -320,6 +320,8 @@ inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
       before.b = op.toff;
       keep = false;
     }
+    // the kernel loads the constant at toff with the op, read or not
+    if (op_consts(w) == 0) op.toff = 0;
     if (keep) {
       // an op without a two-lane form is a segment of its own
       const bool wide = op.head == PV_WIDE;
