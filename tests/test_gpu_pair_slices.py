@@ -50,3 +50,28 @@ def test_finished_groups_are_passed_over_and_the_others_run_on(turns):
                  for f in (0, capi.UFO_TRACK_PLAIN))
     assert np.array_equal(got[1], want[1]) and np.all(got[1][alive] == turns)
     assert np.array_equal(got[2], want[2], equal_nan=True)
+
+
+@pytest.mark.parametrize('slices', [4, 7, 8, 13, 15, 29])
+def test_constant_divisions_round_subnormal_quotients_correctly(slices):
+    """Inner drifts divide by slices - 1; the smallest operands' quotients, ties
+    among them, are IEEE division's."""
+    import ufo_gb300 as u
+    from ufo_gb300 import capi, compiler as C
+    ctx = u.context(0)
+    line = u.Line('r', [u.Sextupole('s', length=4.0, k2=0.0, slices=slices)])
+    dp = capi.DeviceProgram(ctx, C.compile_line(line, u.KICK, where=[-1]))
+    n = 4000
+    rng = np.random.default_rng(slices)
+    p = rng.choice([-1.0, 1.0], n) * rng.integers(0, 2000, n) * 2.0 ** -1074
+    p[::3] *= 2.0 ** rng.integers(0, 60, len(p[::3]))
+    coords = np.zeros((n, 6))
+    coords[:, 1], coords[:, 3] = p, p[::-1]
+    _, _, got = capi.track(ctx, dp, coords, 1, capi.UFO_MODE_TRACK, 0, slots=0)
+    outer = 4.0 / (2 * (1 + slices))
+    inner = 4.0 - 2 * outer
+    want = p * outer
+    for _ in range(slices - 1):
+        want = want + (p * inner) / float(slices - 1)
+    want = want + p * outer
+    assert np.array_equal(got[:, 0], want) and np.array_equal(got[:, 2], want[::-1])

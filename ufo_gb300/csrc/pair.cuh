@@ -77,17 +77,15 @@ UFO_DEV double pick(bool first, double a, double b) { return first ? a : b; }
 // the odd part of d: 2N - (2i+1) d' is odd), so any u closer to a eps ulp(r)
 // than that gives the correctly rounded quotient; the host admits the form
 // when a power of two is (d' = 3: eps = 1/3, 1/4 serves; d' = 7: eps = 2/7,
-// 1/4 serves; d' = 5 has none and keeps the general form).  Zeros and
-// subnormal a take u = 0, which is as good there (the quotient is a multiple of
-// 2^-1074 off by far less than 1/(2 d') of it); `bad` collects operands whose
-// exponent the shift would take out of range.
+// 1/4 serves; d' = 5 has none and keeps the general form).  A zero takes u = 0;
+// `bad` collects operands whose exponent the shift would take out of range, and
+// the subnormal ones, whose quotient by an even d may be a tie (9 2^-1074 / 6).
 UFO_DEV double div_shift(double a, double r, int shift_hi, int sign, bool &bad) {
-  const int hi = __double2hiint(a);
-  const unsigned t = (static_cast<unsigned>(hi) & 0x7fffffffu) - 0x00100000u;
-  bad = bad || t < 0x07000000u;
-  const bool tiny = static_cast<int>(t) < 0;
-  const double u = __hiloint2double(tiny ? 0 : (hi - shift_hi) ^ sign,
-                                    tiny ? 0 : __double2loint(a));
+  const int hi = __double2hiint(a), lo = __double2loint(a);
+  const unsigned mag = static_cast<unsigned>(hi) & 0x7fffffffu;
+  const bool zero = (mag | static_cast<unsigned>(lo)) == 0;
+  bad = bad || (!zero && mag < 0x07100000u);
+  const double u = __hiloint2double(zero ? 0 : (hi - shift_hi) ^ sign, lo);
   return fma_(a, r, u);
 }
 
