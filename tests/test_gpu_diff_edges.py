@@ -57,3 +57,16 @@ def test_the_opcode_list_needs_no_more_than_int_alignment(tangent):
         assert ops.data_ptr() % 16 == 4 * off
         out = forward(ops, tab, z0, tangent)
         assert np.allclose(out[:, :4], want, rtol=1e-15, atol=1e-15)
+
+
+@pytest.mark.parametrize('tangent', [False, True])
+def test_weak_focusing_leaves_the_vertical_plane_alone(tangent):
+    """A bend's weak focusing acts on x; an infinite y keeps its finite slope."""
+    import ufo_gb300 as u
+    from ufo_gb300 import diff
+    line = u.Line('l', [u.Sbend('b', length=1.0, angle=0.1, slices=3), u.Drift('d', length=0.5)])
+    eng = diff.DiffEngine(diff.DiffProgram(line, u.KICK, []))
+    z0 = np.array([[1e-3, 1e-4, np.inf, 2e-4], [1e-3, 1e-4, -1e-3, 2e-4]])
+    out, _ = eng.forward(z0, np.ones(2), 2, tangent=tangent)
+    assert np.array_equal(out[0, :2], out[1, :2]) and out[0, 2] == np.inf
+    assert out[0, 3] == out[1, 3] == 2e-4

@@ -691,8 +691,9 @@ __device__ __forceinline__ void kick_elem_pair(Half &h, const double *c, bool tp
 #pragma unroll
   for (int n = 0; n < M; ++n) cf[n] = __ldg(src + n);
   const double Lo = __ldg(c), Li = __ldg(c + 1), W = __ldg(c + 2), Lx = __ldg(c + 5);
-  const double so = even ? neg(oo) : oo, sw = even ? neg(W) : 0.0;
-  const bool weak = tp && nonzero(W);
+  const double so = even ? neg(oo) : oo, sw = neg(W);
+  // the x plane's alone: 0 times an infinite y would be NaN
+  const bool weak = tp && even && nonzero(W);
   if (tp) h.u = fma(h.pu, Lo, h.u);
   for (int sl = 0; sl < N; ++sl) {
     const double w = other(h.u);
@@ -796,7 +797,7 @@ __device__ void turn_forward_pair(Half &h, const DiffArgs &a, const double *T0, 
             tape += 4 * TLANES;
           }
           h.pu = fma(even ? neg(oo) : oo, s0, h.pu);
-          if (tp && nonzero(W)) h.pu = fma(even ? neg(W) : 0.0, h.u, h.pu);
+          if (tp && even && nonzero(W)) h.pu = fma(neg(W), h.u, h.pu);
           if (tp) h.u = fma(h.pu, sl < N - 1 ? Li : Lx, h.u);
         }
         break;
@@ -830,8 +831,8 @@ __device__ __forceinline__ void rev_part_pair(Half &bh, const DiffArgs &a, const
   }
   tape -= N * 4 * TLANES;
   const double Lo = __ldg(c), Li = __ldg(c + 1), W = __ldg(c + 2), Lx = __ldg(c + 5);
-  const double sw = even ? neg(W) : 0.0;
-  const bool weak = tp && nonzero(W);
+  const double sw = neg(W);
+  const bool weak = tp && even && nonzero(W);
 #pragma unroll
   for (int q = 0; q < N; ++q) {  // slice N-1-q
     if (tp) bh.pu = fma(bh.u, q == 0 && last ? Lx : Li, bh.pu);
@@ -1070,8 +1071,8 @@ __device__ __forceinline__ void kick_elem_oct(Oct &s, const double *c, int M, bo
 #pragma unroll
   for (int n = 0; n < R; ++n) cf[n] = __ldg(c + KHDR + (even ? 0 : M) + n);
   const double Lo = __ldg(c), Li = __ldg(c + 1), W = __ldg(c + 2), Lx = __ldg(c + 5);
-  const double so = even ? neg(oo) : oo, sw = even ? neg(W) : 0.0;
-  const bool weak = tp && nonzero(W);
+  const double so = even ? neg(oo) : oo, sw = neg(W);
+  const bool weak = tp && even && nonzero(W);
   if (tp) oct_drift(s, Lo);
   for (int sl = 0; sl < N; ++sl) {
     if (TAPE) {
@@ -1205,8 +1206,8 @@ __device__ void turn_reverse_oct(Oct &b, const DiffArgs &a, const double *T0, do
         const bool tp = op.kind == D_TEAPOT;
         const int N = tp ? op.N : 1;
         const double Lo = __ldg(c), Li = __ldg(c + 1), W = __ldg(c + 2), Lx = __ldg(c + 5);
-        const double sw = even ? neg(W) : 0.0;
-        const bool weak = tp && nonzero(W);
+        const double sw = neg(W);
+        const bool weak = tp && even && nonzero(W);
         const int pm = op.pslot >= 0 ? op.pm : -1;
         const double *coef = c + KHDR + (even ? 0 : op.M);
         double g0 = 0.0, g1 = 0.0;
