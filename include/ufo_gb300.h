@@ -70,9 +70,13 @@ void ufo_ctx_destroy(ufo_ctx *ctx);
  * `n_dumps` observation points per turn.  Replaces the kernel build of
  * ufo/track.py:84-118 (cl.Program(...).build).
  * A program with thick elements or chromatic fringe edges keeps a device cache of
- * their momentum-dependent coefficients: allocated by its first launch (or graph
- * creation) outside a stream capture, at most 4 GiB, freed with the program, and
- * shared like the context's counters.  A launch without it gives the same results
+ * their momentum-dependent coefficients, shared like the context's counters.
+ * The first launch or graph creation outside a stream capture allocates it and a
+ * larger launch a larger one (cudaMalloc inside ufo_track_device).  Outgrown
+ * caches are kept, so that nothing waits for the launches that use them, until
+ * all together would pass 4 GiB (then they are freed, which waits), the program
+ * gets a table that needs more entries, or it is destroyed.  While a graph holds
+ * a cache none is freed.  A launch that finds no cache gives the same results
  * from the one-lane kernel. */
 int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *table,
                     int64_t stride, int n_seeds, int n_dumps, ufo_prog **out);

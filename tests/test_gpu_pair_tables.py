@@ -68,3 +68,89 @@ def test_captured_thick_batch_takes_tables_that_share_other_entries(captured):
         seen.append(want[0])
     assert np.isfinite(seen[0]).all() and not np.array_equal(seen[0], seen[1])
     assert np.array_equal(seen[0], seen[2])
+
+
+def test_a_callers_own_capture_may_come_first():
+    """The first launch of a thick program in the caller's capture, where nothing
+    can be allocated, then larger launches, a second capture that holds the cache
+    they left, and new tables."""
+    import torch
+    rng = np.random.default_rng(4)
+    magnets = [e for e in alba().flatten() if type(e).__name__ in ('Quadrupole', 'Sbend')][:12]
+    rows = np.array([[e.k1 for e in magnets]] * 3)
+    b, table = thick_batch(rows)
+    b.upload()
+    want = plain(b)
+    stream = torch.cuda.Stream()
+    graphs = []
+    for _ in range(2):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            b.launch(stream=stream.cuda_stream, graph=False)
+        graphs.append(g)
+        b._dev['final'].zero_()
+        g.replay()
+        assert same(b.download(), want)
+        b._dev['final'].zero_()
+        b.launch(graph=False)
+        assert same(b.download(), want)
+    other = rows * (1 + 1e-3 * rng.standard_normal(rows.shape))
+    b.dprog.set_table(table(other))
+    want = plain(b)
+    for g in graphs:
+        b._dev['final'].zero_()
+        g.replay()
+        assert same(b.download(), want)
+
+
+def test_a_first_launch_beside_a_capture_leaves_it_alone():
+    """A thick program's first launch allocates; a capture of the same thread on
+    another stream, in the mode that forbids that, goes on."""
+    import torch
+    b, _ = thick_batch(np.full((3, 1), 1.4))
+    b.upload()
+    x = torch.zeros(8, device='cuda:0')
+    torch.cuda.synchronize()
+    side, work = torch.cuda.Stream(), torch.cuda.Stream()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=side, capture_error_mode='global'):
+        x += 1
+        b.launch(stream=work.cuda_stream, graph=False)
+        x += 1
+    work.synchronize()
+    g.replay()
+    got = b.download()
+    assert float(x.sum()) == 16.0
+    assert same(got, plain(b))
+
+
+def test_graphs_outlive_larger_launches_and_one_another():
+    """Caches grow past a live graph, and when the last graph is gone a table may
+    need more entries again."""
+    from ufo_gb300 import capi
+    rng = np.random.default_rng(5)
+    magnets = [e for e in alba().flatten() if type(e).__name__ in ('Quadrupole', 'Sbend')]
+    equal = np.array([[e.k1 for e in magnets]] * 3)
+    individual = equal * (1 + 1e-3 * rng.standard_normal(equal.shape))
+    b, table = thick_batch(equal)
+    b.upload()
+    b.capture()
+    for rows in (equal, individual, equal):
+        b.dprog.set_table(table(rows))
+        want = plain(b)
+        b.launch()
+        assert same(b.download(), want)
+        for n in (3000, 40_000, 80_000):  # whole runs, slices, whole runs again
+            c = np.tile(b.coords, (-(-n // 60), 1))[:n]
+            out = [capi.track(b.ctx, b.dprog, c, 2, capi.UFO_MODE_TRACK, f, slots=0)[1:]
+                   for f in (0, capi.UFO_TRACK_PLAIN)]
+            assert same(*out), n
+        b.launch()
+        assert same(b.download(), want)
+    b.destroy_graph()
+    b.dprog.set_table(table(individual))
+    want = plain(b)
+    b.capture()
+    for graph in (True, False):
+        b.launch(graph=graph)
+        assert same(b.download(), want)

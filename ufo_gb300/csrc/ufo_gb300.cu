@@ -26,6 +26,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -771,7 +772,14 @@ struct ufo_prog {
   int cache_fields;            // doubles per lane of the coefficient cache
   mutable double *cache;       // [cache_fields][cache_lanes]
   mutable int64_t cache_lanes;
-  mutable bool captured;       // a graph may hold the cache: its layout stays
+  mutable std::vector<double *> old_caches;  // outgrown ones, which launches may still use
+  mutable size_t cache_bytes;  // of all of them
+  // who may run a launch again that holds a cache: graphs of ufo_graph_create
+  // that live, and the caller's own captures.  Meanwhile no cache is freed and
+  // cache_fields stays.
+  std::shared_ptr<std::atomic<int>> graphs;
+  mutable bool captured;
+  bool cache_held() const { return captured || graphs->load() > 0; }
 };
 
 namespace {
@@ -1087,41 +1095,62 @@ bool use_pair(const ufo_ctx *ctx, const ufo_prog *prog, int64_t n, int mode, int
   return (n + 15) / 16 <= most * static_cast<int64_t>(ctx->sm_count);
 }
 
-// The program's coefficient cache for a two-lane launch of `lanes` lanes, grown
-// when needed and until a graph holds it.  Without memory for it (or under the
-// caller's own stream capture, which allows no allocation) the launch takes the
-// one-lane kernel.
 constexpr size_t CACHE_MOST = size_t{4} << 30;
 
-void ensure_cache(const ufo_prog *prog, int64_t lanes, cudaStream_t stream) {
-  if (!prog->cache_fields) return;
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) {
-    cudaGetLastError();
-    return;
+void free_caches(const ufo_prog *prog) {  // waits for the launches that use them
+  cudaFree(prog->cache);
+  for (double *old : prog->old_caches) cudaFree(old);
+  prog->old_caches.clear();
+  prog->cache = nullptr;
+  prog->cache_lanes = 0;
+  prog->cache_bytes = 0;
+}
+
+bool is_capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream beside a capture
+    return true;
   }
-  if (capturing != cudaStreamCaptureStatusNone) prog->captured = true;
-  if (prog->cache_lanes >= lanes || prog->captured) return;
+  return status != cudaStreamCaptureStatusNone;
+}
+
+// The program's coefficient cache for a two-lane launch of `lanes` lanes, grown
+// when needed.  An outgrown one is kept, so that nothing waits for the launches
+// and graphs that use it; only where all together would pass 4 GiB are they
+// freed, if no graph holds one.  Without memory for it (or under the caller's
+// own stream capture, which allows no allocation) the launch takes the one-lane
+// kernel.
+void ensure_cache(const ufo_prog *prog, int64_t lanes, cudaStream_t stream) {
+  if (!prog->cache_fields || prog->cache_lanes >= lanes || is_capturing(stream)) return;
   // lanes of the largest grid where that is cheap, so that it grows once
   const size_t per_lane = sizeof(double) * static_cast<size_t>(prog->cache_fields);
   const int64_t most = static_cast<int64_t>(prog->ctx->sm_count) * 16 * 32;
   if (per_lane * most <= CACHE_MOST / 8) lanes = std::max(lanes, most);
   const size_t bytes = per_lane * lanes;
   if (bytes > CACHE_MOST) return;
-  double *buf = nullptr;
-  if (cudaMalloc(&buf, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    return;
+  if (prog->cache_bytes + bytes > CACHE_MOST) {
+    if (prog->cache_held()) return;
+    free_caches(prog);
   }
+  // a capture on another stream forbids this thread to allocate, unless it says
+  // that the allocation is none of the capture's
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  double *buf = nullptr;
+  cudaError_t e = cudaMalloc(&buf, bytes);
   // zeros: lanes without a particle read finite coefficients
-  if (cudaMemsetAsync(buf, 0, bytes, stream) != cudaSuccess) {
+  if (e == cudaSuccess) e = cudaMemsetAsync(buf, 0, bytes, stream);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) {
     cudaGetLastError();
     cudaFree(buf);
     return;
   }
-  cudaFree(prog->cache);  // waits for launches that use it
+  if (prog->cache) prog->old_caches.push_back(prog->cache);
   prog->cache = buf;
   prog->cache_lanes = lanes;
+  prog->cache_bytes += bytes;
 }
 
 // Time slices for a two-lane launch (slice_plan has the rule).  Particles of a
@@ -1148,41 +1177,64 @@ int64_t cache_lanes_for(const ufo_ctx *ctx, const ufo::Slices &s, const ufo::Tra
   return 32 * (s.groups ? s.groups : pair_warps(a, ctx->sm_count, ctx->warps_per_sm));
 }
 
-int launch_track(ufo_ctx *ctx, const ufo_prog *prog, const double *d_coords, const int32_t *d_seed,
-                 const int32_t *d_pturns, int64_t n, int turns, int mode, int flags, int64_t slots,
-                 int every, double *d_tracks, uint32_t *d_lost, double *d_final,
+// The kernel of a launch: two-lane or one-lane, in slices or whole, and its cache.
+struct Route {
+  bool pair = false;
+  ufo::Slices slices{};
+  int warps_per_sm = 0;
+};
+
+Route plan_route(const ufo_ctx *ctx, const ufo_prog *prog, ufo::TrackArgs &a,
                  cudaStream_t stream) {
-  if (n <= 0) return UFO_OK;
+  Route r;
+  r.warps_per_sm = ctx->warps_per_sm;
+  r.pair = use_pair(ctx, prog, a.n, a.mode, a.flags, a.pturns != nullptr);
+  if (!r.pair) return r;
+  r.slices = plan_slices(ctx, a, r.warps_per_sm);
+  a.pair_ops = prog->pair_ops + ((a.flags & UFO_TRACK_FMA) ? prog->pair_fma_at : 0);
+  a.pair_fills = a.pair_ops + pair_fill_at(prog->n_ops);
+  if (!prog->cache_fields) return r;
+  int64_t lanes = cache_lanes_for(ctx, r.slices, a);
+  ensure_cache(prog, lanes, stream);
+  if (prog->cache_lanes < lanes && r.slices.groups) {  // fewer lanes without slices
+    r.slices = ufo::Slices{};
+    r.warps_per_sm = ctx->warps_per_sm;
+    lanes = cache_lanes_for(ctx, r.slices, a);
+    ensure_cache(prog, lanes, stream);
+  }
+  r.pair = prog->cache_lanes >= lanes;
+  if (!r.pair) r.slices = ufo::Slices{};
+  a.cache = r.pair ? prog->cache : nullptr;
+  a.cache_lanes = r.pair ? prog->cache_lanes : 0;
+  return r;
+}
+
+// `holds_cache`, of a capture whose graph the library keeps: set when the launch
+// uses the program's cache.
+int launch_track(ufo_ctx *ctx, const ufo_prog *prog, ufo::TrackArgs &a, cudaStream_t stream,
+                 bool *holds_cache = nullptr) {
+  if (a.n <= 0) return UFO_OK;
+  const Route r = plan_route(ctx, prog, a, stream);
+  if (a.cache && holds_cache)
+    *holds_cache = true;
+  else if (a.cache && is_capturing(stream))
+    prog->captured = true;
+  const int rc = launch_kernels(a, prog->full, r.pair, r.slices, ctx->sm_count, r.warps_per_sm,
+                                stream);
+  if (rc == UFO_OK) ctx->launches.fetch_add(1);
+  return rc;
+}
+
+ufo::TrackArgs track_args(const ufo_ctx *ctx, const ufo_prog *prog, const double *d_coords,
+                          const int32_t *d_seed, const int32_t *d_pturns, int64_t n, int turns,
+                          int mode, int flags, int64_t slots, int every, double *d_tracks,
+                          uint32_t *d_lost, double *d_final) {
   ufo::TrackArgs a = make_args(prog->ops, prog->n_ops, prog->table, prog->stride, prog->n_seeds,
                                prog->n_dumps, d_coords, d_seed, d_pturns, n, turns, mode, flags,
                                slots, every, d_tracks, d_lost, d_final, ctx->queue);
   a.pool = ctx->pool;
   a.pool_seq = ctx->pool_seq;
-  bool pair = use_pair(ctx, prog, n, mode, flags, d_pturns != nullptr);
-  int warps_per_sm = ctx->warps_per_sm;  // of the launch
-  ufo::Slices slices{};
-  if (pair) {
-    slices = plan_slices(ctx, a, warps_per_sm);
-    a.pair_ops = prog->pair_ops + ((flags & UFO_TRACK_FMA) ? prog->pair_fma_at : 0);
-    a.pair_fills = a.pair_ops + pair_fill_at(prog->n_ops);
-    if (prog->cache_fields) {
-      int64_t lanes = cache_lanes_for(ctx, slices, a);
-      ensure_cache(prog, lanes, stream);
-      if (prog->cache_lanes < lanes && slices.groups) {  // fewer lanes without slices
-        slices = ufo::Slices{};
-        warps_per_sm = ctx->warps_per_sm;
-        lanes = cache_lanes_for(ctx, slices, a);
-        ensure_cache(prog, lanes, stream);
-      }
-      pair = prog->cache_lanes >= lanes;
-      a.cache = prog->cache;
-      a.cache_lanes = prog->cache_lanes;
-    }
-  }
-  const int rc =
-      launch_kernels(a, prog->full, pair, slices, ctx->sm_count, warps_per_sm, stream);
-  if (rc == UFO_OK) ctx->launches.fetch_add(1);
-  return rc;
+  return a;
 }
 
 int check_track_args(ufo_ctx *ctx, const ufo_prog *prog, int64_t n, int turns, int mode,
@@ -1372,6 +1424,8 @@ int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *t
   p->pair_ops = nullptr;
   p->cache = nullptr;
   p->cache_lanes = 0;
+  p->cache_bytes = 0;
+  p->graphs = std::make_shared<std::atomic<int>>(0);
   p->captured = false;
   const bool pair =
       decode_pair(ops, n_ops, table, stride, n_seeds, INT_MAX, p->host_pair_ops, p->pair_fma_at,
@@ -1418,15 +1472,15 @@ int ufo_prog_set_table(ufo_prog *prog, const double *table, int n_seeds) {
     int fields = 0;
     std::vector<ufo::PairOp> ops2;
     decode_pair(prog->host_ops.data(), prog->n_ops, table, prog->stride, n_seeds,
-                prog->captured ? prog->cache_fields : INT_MAX, ops2, prog->pair_fma_at, fields,
+                prog->cache_held() ? prog->cache_fields : INT_MAX, ops2, prog->pair_fma_at, fields,
                 prog->pair_fma, prog->pair_general);
     if (std::memcmp(ops2.data(), prog->host_pair_ops.data(), sizeof(ufo::PairOp) * ops2.size())) {
       UFO_CUDA(cudaMemcpyAsync(prog->pair_ops, ops2.data(), sizeof(ufo::PairOp) * ops2.size(),
                                cudaMemcpyHostToDevice, prog->ctx->stream));
       UFO_CUDA(cudaStreamSynchronize(prog->ctx->stream));
       prog->host_pair_ops.swap(ops2);
-      if (fields > prog->cache_fields) {  // grown at the next launch
-        prog->cache_lanes = 0;
+      if (fields > prog->cache_fields) {  // allocated again by the next launch
+        free_caches(prog);
         prog->cache_fields = fields;
       }
     }
@@ -1445,7 +1499,7 @@ void ufo_prog_destroy(ufo_prog *prog) {
   cudaFree(prog->ops);
   cudaFree(prog->table);
   cudaFree(prog->pair_ops);
-  cudaFree(prog->cache);
+  free_caches(prog);
   delete prog;
 }
 
@@ -1458,8 +1512,9 @@ int ufo_track_device(ufo_ctx *ctx, const ufo_prog *prog, const double *d_coords,
   if (n > 0 && !d_coords) return fail(UFO_E_ARG, "null coordinates");
   UFO_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-  return launch_track(ctx, prog, d_coords, d_seed, d_pturns, n, turns, mode, flags, slots, every,
-                      d_tracks, d_lost, d_final, st);
+  ufo::TrackArgs a = track_args(ctx, prog, d_coords, d_seed, d_pturns, n, turns, mode, flags,
+                                slots, every, d_tracks, d_lost, d_final);
+  return launch_track(ctx, prog, a, st);
 }
 
 int ufo_track(ufo_ctx *ctx, const ufo_prog *prog, const double *coords, const int32_t *seed,
@@ -1505,8 +1560,9 @@ int ufo_track(ufo_ctx *ctx, const ufo_prog *prog, const double *coords, const in
     cleanup();
     return cuda_fail(e, "upload");
   }
-  rc = launch_track(ctx, prog, d_coords, d_seed, d_pturns, n, turns, mode, flags, slots, every,
-                    d_tracks, d_lost, d_final, st);
+  ufo::TrackArgs a = track_args(ctx, prog, d_coords, d_seed, d_pturns, n, turns, mode, flags,
+                                slots, every, d_tracks, d_lost, d_final);
+  rc = launch_track(ctx, prog, a, st);
   if (rc) {
     cleanup();
     return rc;
@@ -1621,6 +1677,7 @@ struct ufo_graph {
   int device;  // copied: destruction must not touch the context
   cudaGraph_t graph;
   cudaGraphExec_t exec;
+  std::shared_ptr<std::atomic<int>> cache_holders;  // of the program, if it holds its cache
 };
 
 extern "C" int ufo_closed_orbit(ufo_ctx *ctx, const ufo_prog *prog, const double *start,
@@ -1714,19 +1771,17 @@ extern "C" int ufo_graph_create(ufo_ctx *ctx, const ufo_prog *prog, const double
   if (n <= 0) return fail(UFO_E_ARG, "empty launch");
   if (!d_coords) return fail(UFO_E_ARG, "null coordinates");
   UFO_CUDA(cudaSetDevice(ctx->device));
-  if (use_pair(ctx, prog, n, mode, flags, d_pturns != nullptr)) {  // nothing may be allocated under capture
-    // enough for a launch with and without time slices
-    ensure_cache(prog, 32 * ((n + 15) / 16), ctx->stream);
-    ensure_cache(prog, 32 * std::min((n + 15) / 16, int64_t{16} * ctx->sm_count), ctx->stream);
-    UFO_CUDA(cudaStreamSynchronize(ctx->stream));
-  }
+  ufo::TrackArgs a = track_args(ctx, prog, d_coords, d_seed, d_pturns, n, turns, mode, flags,
+                                slots, every, d_tracks, d_lost, d_final);
+  plan_route(ctx, prog, a, ctx->stream);  // the cache: nothing may be allocated under capture
+  UFO_CUDA(cudaStreamSynchronize(ctx->stream));
+  bool holds_cache = false;
   cudaStream_t cap;
   UFO_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    rc = launch_track(ctx, prog, d_coords, d_seed, d_pturns, n, turns, mode, flags, slots, every,
-                      d_tracks, d_lost, d_final, cap);
+    rc = launch_track(ctx, prog, a, cap, &holds_cache);
     e = cudaStreamEndCapture(cap, &graph);
   }
   cudaStreamDestroy(cap);
@@ -1751,6 +1806,10 @@ extern "C" int ufo_graph_create(ufo_ctx *ctx, const ufo_prog *prog, const double
   g->device = ctx->device;
   g->graph = graph;
   g->exec = exec;
+  if (holds_cache) {
+    g->cache_holders = prog->graphs;
+    g->cache_holders->fetch_add(1);
+  }
   *out = g;
   return UFO_OK;
 }
@@ -1770,5 +1829,6 @@ extern "C" void ufo_graph_destroy(ufo_graph *g) {
   cudaDeviceSynchronize();
   cudaGraphExecDestroy(g->exec);
   cudaGraphDestroy(g->graph);
+  if (g->cache_holders) g->cache_holders->fetch_sub(1);
   delete g;
 }
