@@ -597,7 +597,10 @@ def bench_c3(args):
         coords = inputs[order]
         # the compacting kernel at StableAperture's resident warps per SM
         cw = args.c3_compact_warps or u.StableAperture.COMPACT_WARPS_PER_SM
-        ctx.set_tuning(cw if kind == 'compact' else 16)
+        if kind == 'compact':
+            ctx.set_tuning(cw)
+        else:
+            ctx.reset_tuning()
         for _ in range(args.warmup):
             launch(coords, kind)
         torch.cuda.synchronize()
@@ -621,7 +624,7 @@ def bench_c3(args):
     for order in ('sorted', 'shuffled', 'amplitude'):
         for kind in kinds:
             runs[(order, kind)] = timed(order, kind, args.steps)
-    ctx.set_tuning(16)
+    ctx.reset_tuning()
     ms_p, launches, lost_p = runs[('sorted', 'compact')]
     ms_pers = runs[('sorted', 'persistent')][0]
     ms_plain = runs[('sorted', 'plain')][0]
@@ -736,8 +739,10 @@ def c3_measure(ctx, stream, mode, reps=2):
 
     def timed(m, extra, k):
         # the compacting kernel with StableAperture's resident warps per SM
-        ctx.set_tuning(u.StableAperture.COMPACT_WARPS_PER_SM
-                       if extra & capi.UFO_TRACK_COMPACT else 16)
+        if extra & capi.UFO_TRACK_COMPACT:
+            ctx.set_tuning(u.StableAperture.COMPACT_WARPS_PER_SM)
+        else:
+            ctx.reset_tuning()
         launch(m, extra)  # warm-up
         torch.cuda.synchronize()
         l0 = ctx.launches()
@@ -760,7 +765,7 @@ def c3_measure(ctx, stream, mode, reps=2):
         ms, launches, lo = timed(mode, extra, reps)
         identical &= bool(np.array_equal(lo, lost_strict))
         variants[name] = {'value': pet / (ms / 1e3), 'ms': ms, 'launches': launches}
-    ctx.set_tuning(16)
+    ctx.reset_tuning()
     sa = u.StableAperture(ring, flags=u.KICK | (u.FMA if mode == 'fma' else 0) |
                           u.DOUBLE_PRECISION, turns=T, particles=n,
                           parameters=['x', 'px', 'y', 'py', 'dp'], context=ctx)

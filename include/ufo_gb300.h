@@ -168,10 +168,13 @@ int ufo_track_noalloc(const int32_t *ops, int n_ops, const double *d_table, int6
 int ufo_closed_orbit(ufo_ctx *ctx, const ufo_prog *prog, const double *start,
                      const int32_t *seed, int64_t n, int iterations, double *orbits);
 
-/* Resident warps per SM of the persistent grid (default 16; the two-lane kernel,
- * whose warps hold half the particles, takes twice as many, at most 16, and 8 for
- * a dynamic-aperture scan at the default); set by the autotuner (ufo_gb300/batch.py: autotune).  No reference counterpart. */
+/* Resident warps per SM of the persistent grid, 1 to 32; set by the autotuner
+ * (ufo_gb300/batch.py: autotune).  The two-lane kernel, whose warps hold half the
+ * particles, takes twice as many, at most 16.  Until it is called, and again
+ * after ufo_ctx_reset_tuning, the library chooses: 16, and 8 two-lane warps for a
+ * dynamic-aperture scan.  No reference counterpart. */
 int ufo_ctx_set_tuning(ufo_ctx *ctx, int warps_per_sm);
+int ufo_ctx_reset_tuning(ufo_ctx *ctx);
 
 /* One tracking launch (work-counter reset + persistent kernel over all
  * particles of all seeds) captured into a CUDA graph and replayed on the same

@@ -75,3 +75,27 @@ def test_constant_divisions_round_subnormal_quotients_correctly(slices):
         want = want + (p * inner) / float(slices - 1)
     want = want + p * outer
     assert np.array_equal(got[:, 0], want) and np.array_equal(got[:, 2], want[::-1])
+
+
+@pytest.mark.parametrize('fma', [False, True])
+def test_scans_are_the_same_at_every_tuning(fma):
+    """Dynamic-aperture scans with the library's choice of resident warps, and
+    tuned, where a full launch of general magnets goes by its size."""
+    import ufo_gb300 as u
+    from ufo_gb300 import capi, compiler as C, workloads as W
+    ctx = u.context(0)
+    prog = C.compile_line(W.c3_ring(u), u.KICK | (u.FMA if fma else 0), where=[-1])
+    dp = capi.DeviceProgram(ctx, prog)
+    grid = W.c3_grid(128, 128)
+    tf = capi.UFO_TRACK_FMA if fma else 0
+    want = capi.track(ctx, dp, grid, 12, capi.UFO_MODE_SA, tf | capi.UFO_TRACK_PLAIN, slots=0)
+    ctx.reset_tuning()
+    try:
+        for warps in (None, 1, 7, 16, 32):
+            if warps:
+                ctx.set_tuning(warps)
+            got = capi.track(ctx, dp, grid, 12, capi.UFO_MODE_SA, tf, slots=0)
+            assert np.array_equal(got[1], want[1]), warps
+            assert np.array_equal(got[2], want[2], equal_nan=True), warps
+    finally:
+        ctx.reset_tuning()

@@ -53,6 +53,7 @@ SIGNATURES = {
     'ufo_fp64_peak': [P, P],
     'ufo_fp64_probe': [P, ctypes.c_int, ctypes.c_int, ctypes.c_int, P],
     'ufo_ctx_set_tuning': [P, ctypes.c_int],
+    'ufo_ctx_reset_tuning': [P],
     'ufo_closed_orbit': [P, P, P, P, I64, ctypes.c_int, P],
     'ufo_graph_create': [P, P, P, P, P, I64, ctypes.c_int, ctypes.c_int, ctypes.c_int, I64,
                          ctypes.c_int, P, P, P, P],
@@ -122,11 +123,19 @@ class Context:
         self.device = device
 
     warps_per_sm = 16  # resident warps per SM of the persistent grid (library default)
+    tuned = False      # set by set_tuning; until then the library chooses per launch
 
     def set_tuning(self, warps_per_sm):
         """ufo_ctx_set_tuning, remembered so that callers can restore it."""
         check(load().ufo_ctx_set_tuning(self.handle, int(warps_per_sm)))
         self.warps_per_sm = int(warps_per_sm)
+        self.tuned = True
+
+    def reset_tuning(self):
+        """Back to the library's choice (ufo_ctx_reset_tuning)."""
+        check(load().ufo_ctx_reset_tuning(self.handle))
+        self.warps_per_sm = Context.warps_per_sm
+        self.tuned = False
 
     def launches(self):
         n = ctypes.c_int64()

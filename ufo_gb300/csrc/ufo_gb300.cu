@@ -744,6 +744,7 @@ struct ufo_ctx {
   int device;
   int sm_count;
   int warps_per_sm;  // resident warps per SM of the persistent grid
+  bool tuned;        // set by the caller
   cudaStream_t stream;
   unsigned long long *queue;
   ufo::Parked *pool;               // the compacting kernel's particle pool
@@ -943,17 +944,21 @@ unsigned long long spread_multiplier(int64_t n_particles) {
   return m;
 }
 
-// Warps of the two-lane kernel: 16 particles each; the tuning counts warps of
-// the one-lane kernel, so twice as many, at most the 16 per SM that the
-// registers allow.  A dynamic-aperture scan at the default tuning gets 8 per SM:
-// most of its particles are lost in the first turns, and lanes that refill from
-// a longer queue stay fuller (49,152 particles of the FODO ring with errors, 64
-// turns, 15 % survive: FMA 25 ms with 16, 16 ms with 8; strict 132 and 79 ms),
-// while two warps per sub-partition still fill most of the FP64 pipe.
-int64_t pair_warps(const ufo::TrackArgs &a, int sm_count, int warps_per_sm) {
-  const int64_t per_sm = a.mode == UFO_MODE_SA && warps_per_sm == DEFAULT_WARPS
-                             ? 8 : std::min(16, 2 * warps_per_sm);
-  return std::min((a.n + 15) / 16, sm_count * per_sm);
+// Resident warps per SM of the two-lane kernel, 16 particles each: the tuning
+// counts warps of the one-lane kernel, so twice as many, at most the 16 that the
+// registers allow.  A dynamic-aperture scan that nobody tuned gets 8: most of its
+// particles are lost in the first turns, and lanes that refill from a longer
+// queue stay fuller, while two warps per sub-partition still fill most of the
+// FP64 pipe (FODO ring with errors, 49,152 particles, ms with 16 and with 8: 128
+// turns FMA, 15 % survive 48.8 and 31.1, 31 % 60.5 and 34.4, 46 % 60.6 and 57.9,
+// 66 % 61.6 and 62.2; 32 turns strict, 17 % 71.7 and 45.2, 72 % 132 and 117;
+// 196,608 particles and 12,288 within 6 % either way).
+int pair_warps_per_sm(int mode, int warps_per_sm, bool tuned) {
+  return mode == UFO_MODE_SA && !tuned ? 8 : std::min(16, 2 * warps_per_sm);
+}
+
+int64_t pair_warps(int64_t n, int sm_count, int pair_per_sm) {
+  return std::min<int64_t>((n + 15) / 16, static_cast<int64_t>(sm_count) * pair_per_sm);
 }
 
 // The launch shared by every entry point: fill the kernel arguments and start
@@ -1004,7 +1009,7 @@ int launch_kernels(ufo::TrackArgs &a, bool full, bool pair, const ufo::Slices &s
       ufo::track_pair_sliced<false><<<g, 32, 0, stream>>>(a, slices);
   } else if (pair) {
     UFO_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), stream));
-    const unsigned g = static_cast<unsigned>(pair_warps(a, sm_count, warps_per_sm));
+    const unsigned g = static_cast<unsigned>(pair_warps(a.n, sm_count, warps_per_sm));
     if (fma)
       ufo::track_pair_kernel<true><<<g, 32, 0, stream>>>(a);
     else
@@ -1081,7 +1086,11 @@ ufo::TrackArgs make_args(const ufo::Op *ops, int n_ops, const double *table, int
 //   20,000 (8.2 warps per SM) 699 -> 615, 24,000 (9.9) 705 -> 770; ring with
 //   errors on every magnet 1,000 346 -> 192, 33,000 (13.6) 442 -> 439, 38,900
 //   (16) 477 -> 516.
-//  Dynamic-aperture scans of such a ring: always (pair_warps).
+//  Dynamic-aperture scans of such a ring that nobody tuned: always.  Where few
+//  survive the refill of twice as many, half-size warps wins (196,608 particles,
+//  128 turns, ms: 15 % survive 87.5 -> 64.9); where most do it costs up to 5 %
+//  (31 % 119 -> 123, 66 % 225 -> 236), which a launch cannot know beforehand.  A
+//  tuned scan (StableAperture's second phase, of survivors) goes by its size.
 //  Uneven turn counts on such a ring: always.  The last, longest particles run
 //   in few warps, and twice as many half-size warps leave the queue more evenly:
 //   error seeds of 64 to 256 turns, 39,873 particles 132 -> 110 ms, 85,102
@@ -1090,7 +1099,7 @@ bool use_pair(const ufo_ctx *ctx, const ufo_prog *prog, int64_t n, int mode, int
               bool uneven) {
   if (!prog->pair_ops || ((flags & UFO_TRACK_FMA) && !prog->pair_fma) || (flags & (UFO_TRACK_PLAIN | UFO_TRACK_COMPACT))) return false;
   if (!(flags & UFO_TRACK_FMA) && !prog->pair_general) return true;
-  if (prog->pair_general && (uneven || mode == UFO_MODE_SA)) return true;
+  if (prog->pair_general && (uneven || (mode == UFO_MODE_SA && !ctx->tuned))) return true;
   const int most = !prog->pair_general ? 9 : (flags & UFO_TRACK_FMA) ? 14 : 12;
   return (n + 15) / 16 <= most * static_cast<int64_t>(ctx->sm_count);
 }
@@ -1160,7 +1169,7 @@ ufo::Slices plan_slices(const ufo_ctx *ctx, const ufo::TrackArgs &a, int &warps_
   ufo::Slices s{};
   if (a.mode != UFO_MODE_TRACK || a.pturns || !a.lost || !a.final_state) return s;
   const ufo::SlicePlan plan =
-      ufo::slice_plan(a.n, a.turns, a.n_ops, ctx->sm_count, std::min(16, 2 * warps_per_sm),
+      ufo::slice_plan(a.n, a.turns, a.n_ops, ctx->sm_count, warps_per_sm,
                       static_cast<int64_t>(ctx->sm_count) * ufo::CTA_MAX_WARPS * 32 - 1);
   if (!plan.groups) return s;
   // one word per lane of the largest compacting grid: the groups' and one more
@@ -1172,12 +1181,8 @@ ufo::Slices plan_slices(const ufo_ctx *ctx, const ufo::TrackArgs &a, int &warps_
   return s;
 }
 
-// lanes of the coefficient cache: per group where groups move between warps
-int64_t cache_lanes_for(const ufo_ctx *ctx, const ufo::Slices &s, const ufo::TrackArgs &a) {
-  return 32 * (s.groups ? s.groups : pair_warps(a, ctx->sm_count, ctx->warps_per_sm));
-}
-
-// The kernel of a launch: two-lane or one-lane, in slices or whole, and its cache.
+// The kernel of a launch: two-lane or one-lane, in slices or whole, the resident
+// warps per SM, and the cache.
 struct Route {
   bool pair = false;
   ufo::Slices slices{};
@@ -1188,24 +1193,29 @@ Route plan_route(const ufo_ctx *ctx, const ufo_prog *prog, ufo::TrackArgs &a,
                  cudaStream_t stream) {
   Route r;
   r.warps_per_sm = ctx->warps_per_sm;
-  r.pair = use_pair(ctx, prog, a.n, a.mode, a.flags, a.pturns != nullptr);
-  if (!r.pair) return r;
-  r.slices = plan_slices(ctx, a, r.warps_per_sm);
+  if (!use_pair(ctx, prog, a.n, a.mode, a.flags, a.pturns != nullptr)) return r;
+  const int whole = pair_warps_per_sm(a.mode, ctx->warps_per_sm, ctx->tuned);
+  int warps = whole;
+  ufo::Slices slices = plan_slices(ctx, a, warps);
+  if (prog->cache_fields) {
+    // lanes of the coefficient cache: per group where groups move between warps
+    int64_t lanes = 32 * (slices.groups ? slices.groups : pair_warps(a.n, ctx->sm_count, whole));
+    ensure_cache(prog, lanes, stream);
+    if (prog->cache_lanes < lanes && slices.groups) {  // fewer lanes without slices
+      slices = ufo::Slices{};
+      warps = whole;
+      lanes = 32 * pair_warps(a.n, ctx->sm_count, whole);
+      ensure_cache(prog, lanes, stream);
+    }
+    if (prog->cache_lanes < lanes) return r;
+    a.cache = prog->cache;
+    a.cache_lanes = prog->cache_lanes;
+  }
+  r.pair = true;
+  r.slices = slices;
+  r.warps_per_sm = warps;
   a.pair_ops = prog->pair_ops + ((a.flags & UFO_TRACK_FMA) ? prog->pair_fma_at : 0);
   a.pair_fills = a.pair_ops + pair_fill_at(prog->n_ops);
-  if (!prog->cache_fields) return r;
-  int64_t lanes = cache_lanes_for(ctx, r.slices, a);
-  ensure_cache(prog, lanes, stream);
-  if (prog->cache_lanes < lanes && r.slices.groups) {  // fewer lanes without slices
-    r.slices = ufo::Slices{};
-    r.warps_per_sm = ctx->warps_per_sm;
-    lanes = cache_lanes_for(ctx, r.slices, a);
-    ensure_cache(prog, lanes, stream);
-  }
-  r.pair = prog->cache_lanes >= lanes;
-  if (!r.pair) r.slices = ufo::Slices{};
-  a.cache = r.pair ? prog->cache : nullptr;
-  a.cache_lanes = r.pair ? prog->cache_lanes : 0;
   return r;
 }
 
@@ -1278,6 +1288,7 @@ int ufo_ctx_create(int device, ufo_ctx **out) {
   if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaGetDeviceProperties"); }
   c->sm_count = prop.multiProcessorCount;
   c->warps_per_sm = DEFAULT_WARPS;
+  c->tuned = false;
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaStreamCreate"); }
   e = cudaMalloc(&c->queue, 64);
@@ -1754,6 +1765,14 @@ extern "C" int ufo_ctx_set_tuning(ufo_ctx *ctx, int warps_per_sm) {
   if (warps_per_sm < 1 || warps_per_sm > 32)
     return fail(UFO_E_ARG, "warps_per_sm %d outside [1, 32]", warps_per_sm);
   ctx->warps_per_sm = warps_per_sm;
+  ctx->tuned = true;
+  return UFO_OK;
+}
+
+extern "C" int ufo_ctx_reset_tuning(ufo_ctx *ctx) {
+  if (!ctx) return fail(UFO_E_ARG, "null context");
+  ctx->warps_per_sm = DEFAULT_WARPS;
+  ctx->tuned = false;
   return UFO_OK;
 }
 

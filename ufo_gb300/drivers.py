@@ -13,6 +13,7 @@ Arithmetic is FP64 whatever the flags say; DOUBLE_PRECISION only selects the
 dtype of ``parameters`` and of the outputs, as in the reference.  ``threads``
 is accepted and ignored: the kernels size their own grid.
 """
+import contextlib
 import copy
 
 import numpy as np
@@ -209,6 +210,24 @@ def _sm_count(device):
     return torch.cuda.get_device_properties(device).multi_processor_count
 
 
+@contextlib.contextmanager
+def _tuned(ctx, warps=None):
+    """``warps`` resident warps per SM for the launches inside (None: the
+    library's choice), then the context's own state again."""
+    before, tuned = ctx.warps_per_sm, getattr(ctx, 'tuned', warps is not None)
+    if warps is not None:
+        ctx.set_tuning(warps)
+    elif tuned:
+        ctx.reset_tuning()
+    try:
+        yield
+    finally:
+        if tuned:
+            ctx.set_tuning(before)
+        elif warps is not None:
+            ctx.reset_tuning()
+
+
 class StableAperture:
     """Turns survived per particle (ufo/sa.py:18-145): lost at the end of the
     first turn with |x| > 1 or |y| > 1 or isnan(x); ``lost`` holds that turn,
@@ -269,13 +288,9 @@ class StableAperture:
             compact = True
         flags = _track_flags(self.flags)
         if compact is True:
-            before = self.ctx.warps_per_sm
-            self.ctx.set_tuning(self.COMPACT_WARPS_PER_SM)
-            try:
+            with _tuned(self.ctx, self.COMPACT_WARPS_PER_SM):
                 _, lost, final = capi.track(self.ctx, dprog, coords, T, capi.UFO_MODE_SA,
                                             flags | capi.UFO_TRACK_COMPACT, seed=seed, slots=0)
-            finally:
-                self.ctx.set_tuning(before)
             self.lost = lost
             self.final = final
             return
@@ -286,23 +301,20 @@ class StableAperture:
             self.final = final
             return
         T1 = max(1, T // 8)
-        _, lost, final = capi.track(self.ctx, dprog, coords, T1, capi.UFO_MODE_SA, flags,
-                                    seed=seed, slots=0)
+        with _tuned(self.ctx):  # the context may be tuned to another workload
+            _, lost, final = capi.track(self.ctx, dprog, coords, T1, capi.UFO_MODE_SA, flags,
+                                        seed=seed, slots=0)
         alive = np.nonzero(lost >= T1)[0]
         self.survivors_after_first_phase = len(alive)
         if len(alive) and T > T1:
             sms = _sm_count(self.ctx.device)
             warps = int(min(16, max(2, round(len(alive) / (0.9 * 32 * sms)))))
             self.second_phase_warps_per_sm = warps
-            before = self.ctx.warps_per_sm
-            self.ctx.set_tuning(warps)
-            try:
+            with _tuned(self.ctx, warps):
                 _, lost2, final2 = capi.track(
                     self.ctx, dprog, np.ascontiguousarray(final[alive]), T - T1,
                     capi.UFO_MODE_SA, flags,
                     seed=None if seed is None else np.ascontiguousarray(seed[alive]), slots=0)
-            finally:
-                self.ctx.set_tuning(before)
             lost = lost.copy()
             lost[alive] = T1 + lost2
             final = final.copy()
