@@ -4,24 +4,34 @@
 extern "C" {
 
 // The lists of decode_pair, four words per entry.  info: accepted, entries,
-// start of the FMA list, cache fields, FMA lists usable, most kicks general.
+// start of the FMA list, cache fields, FMA lists usable, most kicks general,
+// entries run by the one-lane code in the strict and the FMA list.
 int pair_lists(const int32_t *ops, int n_ops, const double *table, int64_t stride, int n_seeds,
                int most_fields, int32_t *out, int64_t capacity, int64_t *info) {
-  std::vector<ufo::PairOp> list;
-  size_t fma_at = 0;
-  int fields = 0;
-  bool fma = false, general = false;
-  const bool ok = ufo::decode_pair(ops, n_ops, table, stride, n_seeds, most_fields, list, fma_at,
-                                   fields, fma, general);
-  info[0] = ok;
-  info[1] = static_cast<int64_t>(list.size());
-  info[2] = static_cast<int64_t>(fma_at);
-  info[3] = fields;
-  info[4] = fma;
-  info[5] = general;
-  if (static_cast<int64_t>(list.size()) * 4 > capacity) return -1;
-  std::memcpy(out, list.data(), sizeof(ufo::PairOp) * list.size());
+  ufo::PairLists p;
+  info[0] = ufo::decode_pair(ops, n_ops, table, stride, n_seeds, most_fields, p);
+  info[1] = static_cast<int64_t>(p.ops.size());
+  info[2] = static_cast<int64_t>(p.fma_at);
+  info[3] = p.cache_fields;
+  info[4] = p.fma_ready;
+  info[5] = p.general;
+  info[6] = p.wide[0];
+  info[7] = p.wide[1];
+  if (static_cast<int64_t>(p.ops.size()) * 4 > capacity) return -1;
+  std::memcpy(out, p.ops.data(), sizeof(ufo::PairOp) * p.ops.size());
   return 0;
+}
+
+// Whether a launch of n particles of such lists takes the two-lane kernel.
+int pair_use(int n_ops, int wide, int thick, int general, int64_t n, int sm_count, int fma,
+             int uneven, int scan) {
+  ufo::PairLists p;
+  p.n_ops = n_ops;
+  p.wide[0] = p.wide[1] = wide;
+  p.thick = thick != 0;
+  p.general = general != 0;
+  p.fma_ready = true;
+  return ufo::pair_pays(p, {n, sm_count, fma != 0, uneven != 0, scan != 0});
 }
 
 // groups, slices per group, turns per slice, warps per SM

@@ -29,18 +29,19 @@ def decode(host, ops, table, most=2 ** 31 - 1):
     ops = np.ascontiguousarray(ops, np.int32).reshape(-1, 8)
     table = np.ascontiguousarray(np.atleast_2d(table), np.float64)
     out = np.zeros((8 * len(ops) + 64, 4), np.int32)
-    info = np.zeros(6, np.int64)
+    info = np.zeros(8, np.int64)
     p = [a.ctypes.data_as(ctypes.c_void_p) for a in (ops, table, out, info)]
     rc = host.pair_lists(p[0], len(ops), p[1], ctypes.c_int64(table.shape[1]), len(table),
                          ctypes.c_int(most), p[2], ctypes.c_int64(out.size), p[3])
     assert rc == 0 and info[0] == 1
     out = out[:info[1]]
     lists = []
-    for part in (out[:info[2]], out[info[2]:]):
+    for part, wide in ((out[:info[2]], info[6]), (out[info[2]:], info[7])):
         part = part[:2 * len(ops) + 4]  # without the cache-filling ops
         end = next(i for i, w in enumerate(part)
                    if w[0] & 0xff == PV_SEGMENT and w[3] <= w[2])
         lists.append(part[:end])
+        assert wide == sum((h & 0xff) == PV_WIDE for h in lists[-1][:, 0])
     return lists[0], lists[1], int(info[3])
 
 
@@ -140,3 +141,26 @@ def test_ops_without_constants_read_none(host):
         for lst in (strict, fma):
             walk(lst, fields, 1, 3)
             assert sum((h & 0xff) == PV_OBSERVE for h in lst[:, 0]) == (kind == OP_OBSERVE)
+
+
+def use(host, n, ops=200, wide=0, thick=False, general=False, fma=False, uneven=False, scan=False):
+    return bool(host.pair_use(ops, wide, int(thick), int(general), ctypes.c_int64(n), 152, int(fma),
+                              int(uneven), int(scan)))
+
+
+@pytest.mark.parametrize('fma', [False, True])
+@pytest.mark.parametrize('general', [False, True])
+def test_ops_without_a_two_lane_form_bound_the_two_lane_kernel(host, general, fma):
+    """The larger the launch, the fewer of them; without any the sizes alone decide."""
+    sizes = (1, 1000, 152 * 5 * 16, 152 * 8 * 16, 152 * 9 * 16, 65_536, 1_000_000)
+    for extra in ({}, {'uneven': True}, {'scan': True}):
+        most = []
+        for n in sizes:
+            took = [use(host, n, 400, w, general=general, fma=fma, **extra) for w in range(401)]
+            assert took == sorted(took, reverse=True)  # no more once there are too many
+            most.append(sum(took))
+        assert all(a >= b for a, b in zip(most, most[1:]))
+        assert 40 <= most[0] <= 81 and most[-1] <= 13
+    assert use(host, 10 ** 6) and not use(host, 10 ** 6, fma=True)
+    for n in sizes:  # thick rings: up to a fifth at any size
+        assert use(host, n, 200, 40, thick=True) and not use(host, n, 200, 41, thick=True)

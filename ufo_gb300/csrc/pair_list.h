@@ -163,25 +163,36 @@ inline std::vector<RowScan> scan_rows(const int32_t *ops, int n_ops, const doubl
   return scan;
 }
 
+struct PairLists {
+  std::vector<PairOp> ops;  // the strict list, then at fma_at the FMA one
+  size_t fma_at = 0;
+  int n_ops = 0;            // public ops
+  int cache_fields = 0;     // doubles per lane of the coefficient cache
+  int wide[2] = {0, 0};     // entries run by the one-lane code, per list
+  bool fma_ready = false;   // general kicks carry the series that FMA launches read
+  bool general = false;     // most kicks are general
+  bool thick = false;       // most magnets are thick
+};
+
 // where a list's cache-filling ops start
 inline size_t pair_fill_at(int n_ops) { return 2 * static_cast<size_t>(n_ops) + 4; }
 
 // Translate a validated opcode list for the two-lane kernel; false when an op
-// has no two-lane form worth its name (Yoshida and exact-drift elements, which
-// would run as one-lane code on half-empty warps).  Structurally empty ops
+// is a Yoshida or exact-drift element, which would run as one-lane code on
+// half-empty warps (a program has them everywhere or nowhere; pair_pays bounds
+// the share of the other ops without a two-lane form).  Structurally empty ops
 // (zero-angle edges) are left out: they matter to non-finite coordinates alone.
 // Thick elements and fringe edges with the same constants in every row share
 // their cache fields; at most `most_fields` are given out, and an element that
 // gets none goes through the one-lane code, in a segment of its own.
-// `fma_ready`: the general kicks carry the dense series
-// that the FMA kernel reads.
 inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
                         const std::vector<RowScan> &scan, int most_fields, bool fold_drifts,
-                        std::vector<PairOp> &out, int &cache_fields, bool &fma_ready,
-                        bool &mostly_general) {
-  cache_fields = 0;
-  fma_ready = true;
-  int kicks = 0, general = 0;
+                        PairLists &lists) {
+  std::vector<PairOp> &out = lists.ops;
+  int &cache_fields = lists.cache_fields, &wides = lists.wide[fold_drifts ? 0 : 1];
+  cache_fields = wides = 0;
+  lists.fma_ready = true;
+  int kicks = 0, general = 0, thick = 0;
   std::vector<int> field_of(static_cast<size_t>(n_ops), -1);
   size_t head = 0;  // the current segment's header
   int64_t last_end = -1;  // where the constants of the last general teapot end
@@ -209,7 +220,7 @@ inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
         const bool teapot = w[0] == OP_TEAPOT;
         const int32_t *k = w + (teapot ? 4 : 3);  // nn, ns, mn, ms
         const int pattern = (k[2] | k[3]) ? kick_pattern(k[0], k[1], k[2]) : 3;
-        if (pattern == 0 && !(flags & F_PSER)) fma_ready = false;
+        if (pattern == 0 && !(flags & F_PSER)) lists.fma_ready = false;
         ++kicks;
         general += pattern == 0;
         if (teapot && (flags & (F_EXACT | F_YOSHIDA))) return false;
@@ -284,6 +295,7 @@ inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
         op.head = (w[0] == OP_THICKQ ? PV_THICKQ : PV_THICKB) | common |
                   ((flags & F_CONST) ? PF_CONST : 0);
         fields = w[0] == OP_THICKQ ? TC_D : TC_FIELDS;
+        ++thick;
         break;
       case OP_APERTURE:
         if (flags & F_CIRCLE) op.head = PV_CIRCLE;
@@ -329,13 +341,15 @@ inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
       if (kept > 0 && (wide || out.back().head == PV_WIDE || kept == PAIR_SEGMENT))
         open(i);
       out.push_back(op);
+      wides += wide;
     }
     out[head].b = i + 1;
   }
   if (out[head].b > out[head].a) open(n_ops);  // the end
   out.push_back({PV_SEGMENT, 0, 0, 0});   // the kernel fetches two ops ahead
   out.push_back({PV_SEGMENT, 0, 0, 0});
-  mostly_general = 2 * general > kicks;
+  lists.general = 2 * general > kicks;
+  lists.thick = thick > kicks;
   return true;
 }
 
@@ -345,26 +359,90 @@ inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
 // by the ops that fill the cache (pair_fill walks those alone: one turn of three
 // particles through 1,600 ops 997 us with the whole list, 893 us).
 inline bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t stride,
-                        int n_seeds, int most_fields, std::vector<PairOp> &out, size_t &fma_at,
-                        int &cache_fields, bool &fma_ready, bool &mostly_general) {
+                        int n_seeds, int most_fields, PairLists &lists) {
+  std::vector<PairOp> &out = lists.ops;
   out.clear();
   const size_t fill_at = pair_fill_at(n_ops);
-  fma_at = fill_at + n_ops + 1;
+  lists.n_ops = n_ops;
+  lists.fma_at = fill_at + n_ops + 1;
   const std::vector<RowScan> scan = scan_rows(ops, n_ops, table, stride, n_seeds);
   for (const bool strict : {true, false}) {
     const size_t start = out.size();
-    if (!decode_list(ops, n_ops, table, scan, most_fields, strict, out, cache_fields,
-                     fma_ready, mostly_general))
-      return false;
+    if (!decode_list(ops, n_ops, table, scan, most_fields, strict, lists)) return false;
     const size_t end = out.size();
     out.resize(start + fill_at);
     for (size_t i = start; i < end; ++i)
       if (out[i].head & PF_FILL) out.push_back(out[i]);
-    out.resize(start + fma_at);  // an end at least
+    out.resize(start + lists.fma_at);  // an end at least
   }
   return true;
 }
 
+// Which launches take the two-lane kernel (measured on one GB300, us per turn,
+// one-lane kernel -> two-lane kernel; 152 SMs, 16 particles per warp):
+//  strict arithmetic: always.  Its operations come in pairs of planes, so the
+//   two-lane form issues no more of them at any size, and the constant division
+//   and the coefficient cache shorten it: FODO ring (128 elements) 1,024
+//   particles 167 -> 61, 65,536 particles 475 -> 382; light-source ring (1,024)
+//   65,536 particles 5,352 -> 4,273; thick 768-element ring, 1,000 particles
+//   1,355 -> 318, 65,536 particles 4,481 -> 1,765.
+//   A ring with general error kicks on most magnets (a coefficient enters one
+//   lane's sum, so half its products are idle) gains up to 12 warps per SM:
+//   light-source ring with errors 1,000 particles 15,590 -> 8,480, 30,000 even.
+//  FMA: up to 9 warps per SM, 14 where most kicks are general.  The sextupole
+//   form and the composed linear elements cost the two-lane code more
+//   instructions (6 for 5, 8 for 5 per 32 particles), so the one-lane kernel
+//   wins once its pipe is full: light-source ring 333 particles 652 -> 345,
+//   20,000 (8.2 warps per SM) 699 -> 615, 24,000 (9.9) 705 -> 770; ring with
+//   errors on every magnet 1,000 346 -> 192, 33,000 (13.6) 442 -> 439, 38,900
+//   (16) 477 -> 516.
+//  Dynamic-aperture scans of such a ring that nobody tuned: always.  Where few
+//  survive the refill of twice as many, half-size warps wins (196,608 particles,
+//  128 turns, ms: 15 % survive 87.5 -> 64.9); where most do it costs up to 5 %
+//  (31 % 119 -> 123, 66 % 225 -> 236), which a launch cannot know beforehand.  A
+//  tuned scan (StableAperture's second phase, of survivors) goes by its size.
+//  Uneven turn counts on such a ring: always.  The last, longest particles run
+//   in few warps, and twice as many half-size warps leave the queue more evenly:
+//   error seeds of 64 to 256 turns, 39,873 particles 132 -> 110 ms, 85,102
+//   particles 223 -> 167 ms, 15,978 the same.
+//  Few ops without a two-lane form (wires, general apertures, dynamic kicks,
+//   orders above 15, elements without room in the cache): each is a segment that
+//   both lanes of a pair compute in full, twice the FP64 instructions of the one-
+//   lane kernel.  The share that still pays falls with the warps per SM (FODO
+//   ring with a rectangular aperture, or a wire, after every k-th magnet, strict;
+//   share of ops, particles): 14 %, 12,000 270 -> 227, 278 -> 260; 8 %, 16,000
+//   236 -> 171, 245 -> 212; 8 %, 30,000 299 -> 301, 339 -> 402; 2 %, 65,536
+//   490 -> 434, 523 -> 492; but 25 %, 65,536 675 -> 1,034, 1,210 -> 1,929.  FMA 5 %,
+//   16,000 65 -> 49, 67 -> 58, 20,000 65 -> 73, 70 -> 84.  General magnets and
+//   thick elements, the longer part of their turn, bear more: errors on every
+//   magnet, FMA 17 %, 16,000 584 -> 511, 24,000 613 -> 761; thick ring 24 %, 16,000
+//   2,397 -> 1,856, 65,536 5,248 -> 4,900.
+struct PairUse {
+  int64_t n;
+  int sm_count;
+  bool fma, uneven, untuned_scan;
+};
+
+// the least ops per op without a two-lane form; 0: none may be
+inline int least_ops_per_wide(const PairLists &p, const PairUse &u, int64_t groups) {
+  if (p.thick) return 5;
+  if (p.general) return groups <= 8 * static_cast<int64_t>(u.sm_count) ? 5 : 32;
+  if (groups <= 5 * static_cast<int64_t>(u.sm_count)) return u.fma ? 8 : 6;
+  if (groups <= 8 * static_cast<int64_t>(u.sm_count)) return u.fma ? 12 : 10;
+  return u.fma ? 0 : 32;
+}
+
+inline bool pair_pays(const PairLists &p, const PairUse &u) {
+  if (u.fma && !p.fma_ready) return false;
+  const int64_t groups = (u.n + 15) / 16;
+  const int64_t wide = p.wide[u.fma ? 1 : 0];
+  const int per_wide = least_ops_per_wide(p, u, groups);
+  if (wide && (!per_wide || p.n_ops < per_wide * wide)) return false;
+  if (!u.fma && !p.general) return true;
+  if (p.general && (u.uneven || u.untuned_scan)) return true;
+  const int most = !p.general ? 9 : u.fma ? 14 : 12;
+  return groups <= most * static_cast<int64_t>(u.sm_count);
+}
 // Time slices (Slices in pair.cuh) for a two-lane launch of equal turns with
 // more groups of 16 particles than 8 warps per SM: as many warps as fill every
 // sub-partition evenly (a multiple of 4 per SM) and leave groups in hand.  Below

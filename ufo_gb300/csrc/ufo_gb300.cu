@@ -763,13 +763,9 @@ struct ufo_prog {
   int n_dumps;
   bool full;  // needs the full interpreter (thick, wire, exact, ...)
   std::vector<int32_t> host_ops;  // for validating replacement tables
-  // two-lane kernel (pair.cuh): the strict list, then at pair_fma_at the FMA one;
-  // null when an op has no two-lane form
+  // two-lane kernel (pair.cuh): the lists on the device, null when there are none
   ufo::PairOp *pair_ops;
-  std::vector<ufo::PairOp> host_pair_ops;
-  size_t pair_fma_at;
-  bool pair_fma;               // also for FMA launches
-  bool pair_general;           // most kicks are general
+  ufo::PairLists lists;
   int cache_fields;            // doubles per lane of the coefficient cache
   mutable double *cache;       // [cache_fields][cache_lanes]
   mutable int64_t cache_lanes;
@@ -1068,40 +1064,12 @@ ufo::TrackArgs make_args(const ufo::Op *ops, int n_ops, const double *table, int
   return a;
 }
 
-// Which launches take the two-lane kernel (measured on one GB300, us per turn,
-// one-lane kernel -> two-lane kernel; 152 SMs, 16 particles per warp):
-//  strict arithmetic: always.  Its operations come in pairs of planes, so the
-//   two-lane form issues no more of them at any size, and the constant division
-//   and the coefficient cache shorten it: FODO ring (128 elements) 1,024
-//   particles 167 -> 69, 65,536 particles 475 -> 434; light-source ring (1,024)
-//   65,536 particles 5,352 -> 4,991; thick 768-element ring, 1,000 particles
-//   1,355 -> 357, 65,536 particles 4,481 -> 1,948.
-//   A ring with general error kicks on most magnets (a coefficient enters one
-//   lane's sum, so half its products are idle) gains up to 12 warps per SM:
-//   light-source ring with errors 1,000 particles 15,590 -> 8,480, 30,000 even.
-//  FMA: up to 9 warps per SM, 14 where most kicks are general.  The sextupole
-//   form and the composed linear elements cost the two-lane code more
-//   instructions (6 for 5, 8 for 5 per 32 particles), so the one-lane kernel
-//   wins once its pipe is full: light-source ring 333 particles 652 -> 345,
-//   20,000 (8.2 warps per SM) 699 -> 615, 24,000 (9.9) 705 -> 770; ring with
-//   errors on every magnet 1,000 346 -> 192, 33,000 (13.6) 442 -> 439, 38,900
-//   (16) 477 -> 516.
-//  Dynamic-aperture scans of such a ring that nobody tuned: always.  Where few
-//  survive the refill of twice as many, half-size warps wins (196,608 particles,
-//  128 turns, ms: 15 % survive 87.5 -> 64.9); where most do it costs up to 5 %
-//  (31 % 119 -> 123, 66 % 225 -> 236), which a launch cannot know beforehand.  A
-//  tuned scan (StableAperture's second phase, of survivors) goes by its size.
-//  Uneven turn counts on such a ring: always.  The last, longest particles run
-//   in few warps, and twice as many half-size warps leave the queue more evenly:
-//   error seeds of 64 to 256 turns, 39,873 particles 132 -> 110 ms, 85,102
-//   particles 223 -> 167 ms, 15,978 the same.
+// the two-lane kernel for this launch: pair_pays has the rule
 bool use_pair(const ufo_ctx *ctx, const ufo_prog *prog, int64_t n, int mode, int flags,
               bool uneven) {
-  if (!prog->pair_ops || ((flags & UFO_TRACK_FMA) && !prog->pair_fma) || (flags & (UFO_TRACK_PLAIN | UFO_TRACK_COMPACT))) return false;
-  if (!(flags & UFO_TRACK_FMA) && !prog->pair_general) return true;
-  if (prog->pair_general && (uneven || (mode == UFO_MODE_SA && !ctx->tuned))) return true;
-  const int most = !prog->pair_general ? 9 : (flags & UFO_TRACK_FMA) ? 14 : 12;
-  return (n + 15) / 16 <= most * static_cast<int64_t>(ctx->sm_count);
+  if (!prog->pair_ops || (flags & (UFO_TRACK_PLAIN | UFO_TRACK_COMPACT))) return false;
+  const bool scan = mode == UFO_MODE_SA && !ctx->tuned;
+  return ufo::pair_pays(prog->lists, {n, ctx->sm_count, (flags & UFO_TRACK_FMA) != 0, uneven, scan});
 }
 
 constexpr size_t CACHE_MOST = size_t{4} << 30;
@@ -1214,7 +1182,7 @@ Route plan_route(const ufo_ctx *ctx, const ufo_prog *prog, ufo::TrackArgs &a,
   r.pair = true;
   r.slices = slices;
   r.warps_per_sm = warps;
-  a.pair_ops = prog->pair_ops + ((a.flags & UFO_TRACK_FMA) ? prog->pair_fma_at : 0);
+  a.pair_ops = prog->pair_ops + ((a.flags & UFO_TRACK_FMA) ? prog->lists.fma_at : 0);
   a.pair_fills = a.pair_ops + pair_fill_at(prog->n_ops);
   return r;
 }
@@ -1438,10 +1406,9 @@ int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *t
   p->cache_bytes = 0;
   p->graphs = std::make_shared<std::atomic<int>>(0);
   p->captured = false;
-  const bool pair =
-      decode_pair(ops, n_ops, table, stride, n_seeds, INT_MAX, p->host_pair_ops, p->pair_fma_at,
-                  p->cache_fields, p->pair_fma, p->pair_general);
-  const size_t pb = sizeof(ufo::PairOp) * p->host_pair_ops.size();
+  const bool pair = decode_pair(ops, n_ops, table, stride, n_seeds, INT_MAX, p->lists);
+  p->cache_fields = p->lists.cache_fields;
+  const size_t pb = sizeof(ufo::PairOp) * p->lists.ops.size();
   const size_t ob = sizeof(ufo::Op) * (n_ops > 0 ? n_ops : 1);
   const size_t tb = sizeof(double) * static_cast<size_t>(stride) * n_seeds;
   if (cudaMalloc(&p->ops, ob) != cudaSuccess || cudaMalloc(&p->table, tb) != cudaSuccess ||
@@ -1456,7 +1423,7 @@ int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *t
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(p->table, table, tb, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess && pair)
-    e = cudaMemcpyAsync(p->pair_ops, p->host_pair_ops.data(), pb, cudaMemcpyHostToDevice,
+    e = cudaMemcpyAsync(p->pair_ops, p->lists.ops.data(), pb, cudaMemcpyHostToDevice,
                         ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
@@ -1480,20 +1447,19 @@ int ufo_prog_set_table(ufo_prog *prog, const double *table, int n_seeds) {
   const size_t tb = sizeof(double) * static_cast<size_t>(prog->stride) * n_seeds;
   if (prog->pair_ops) {
     // new constants may share other cache fields or admit another division form
-    int fields = 0;
-    std::vector<ufo::PairOp> ops2;
+    ufo::PairLists next;
     decode_pair(prog->host_ops.data(), prog->n_ops, table, prog->stride, n_seeds,
-                prog->cache_held() ? prog->cache_fields : INT_MAX, ops2, prog->pair_fma_at, fields,
-                prog->pair_fma, prog->pair_general);
-    if (std::memcmp(ops2.data(), prog->host_pair_ops.data(), sizeof(ufo::PairOp) * ops2.size())) {
-      UFO_CUDA(cudaMemcpyAsync(prog->pair_ops, ops2.data(), sizeof(ufo::PairOp) * ops2.size(),
-                               cudaMemcpyHostToDevice, prog->ctx->stream));
+                prog->cache_held() ? prog->cache_fields : INT_MAX, next);
+    const size_t pb = sizeof(ufo::PairOp) * next.ops.size();
+    if (std::memcmp(next.ops.data(), prog->lists.ops.data(), pb)) {
+      UFO_CUDA(cudaMemcpyAsync(prog->pair_ops, next.ops.data(), pb, cudaMemcpyHostToDevice,
+                               prog->ctx->stream));
       UFO_CUDA(cudaStreamSynchronize(prog->ctx->stream));
-      prog->host_pair_ops.swap(ops2);
-      if (fields > prog->cache_fields) {  // allocated again by the next launch
+      if (next.cache_fields > prog->cache_fields) {  // allocated again by the next launch
         free_caches(prog);
-        prog->cache_fields = fields;
+        prog->cache_fields = next.cache_fields;
       }
+      std::swap(prog->lists, next);
     }
   }
   UFO_CUDA(cudaMemcpyAsync(prog->table, table, tb, cudaMemcpyHostToDevice, prog->ctx->stream));
@@ -1730,7 +1696,13 @@ extern "C" int ufo_closed_orbit(ufo_ctx *ctx, const ufo_prog *prog, const double
   // (no orbit waits for another's shrink), then four.  The one-thread search
   // wins back where its warps fill the GPU (n > 64 per SM), except that it
   // recomputes the thick elements' functions in every turn.
-  bool pair = prog->pair_ops && (prog->cache_fields || n <= 64 * static_cast<int64_t>(ctx->sm_count));
+  // Ops without a two-lane form are computed in full by all eight lanes of an
+  // orbit; a quarter of a FODO ring's (wires, 50 steps) still leaves 9,728 orbits
+  // 56 ms against 63.  Above that, one warp per sub-partition, where the number
+  // of turns in a row is all that counts.
+  const int64_t sms = ctx->sm_count;
+  bool pair = prog->pair_ops && (prog->cache_fields || n <= 64 * sms) &&
+              (4 * prog->lists.wide[0] <= prog->n_ops || n <= 16 * sms);
   const int per_warp = n <= 4 * static_cast<int64_t>(ctx->sm_count) ? 1 : 4;
   const int64_t warps = std::min((n + per_warp - 1) / per_warp,
                                  16 * static_cast<int64_t>(ctx->sm_count));
