@@ -164,3 +164,14 @@ def test_ops_without_a_two_lane_form_bound_the_two_lane_kernel(host, general, fm
     assert use(host, 10 ** 6) and not use(host, 10 ** 6, fma=True)
     for n in sizes:  # thick rings: up to a fifth at any size
         assert use(host, n, 200, 40, thick=True) and not use(host, n, 200, 41, thick=True)
+
+
+def test_uneven_fused_launches_end_where_whole_warps_win(host):
+    """General magnets, particles with their own turn counts: the two-lane kernel
+    up to 44 warps per SM (107,008 particles), strict at any size."""
+    n = 152 * 44 * 16
+    assert use(host, n, general=True, fma=True, uneven=True)
+    assert not use(host, n + 1, general=True, fma=True, uneven=True)
+    assert not use(host, 1_145_971, general=True, fma=True, uneven=True)
+    assert use(host, 1_145_971, general=True, uneven=True)
+    assert use(host, 1_145_971, general=True, fma=True, scan=True)

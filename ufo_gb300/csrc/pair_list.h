@@ -401,10 +401,12 @@ inline bool decode_pair(const int32_t *ops, int n_ops, const double *table, int6
 //  128 turns, ms: 15 % survive 87.5 -> 64.9); where most do it costs up to 5 %
 //  (31 % 119 -> 123, 66 % 225 -> 236), which a launch cannot know beforehand.  A
 //  tuned scan (StableAperture's second phase, of survivors) goes by its size.
-//  Uneven turn counts on such a ring: always.  The last, longest particles run
-//   in few warps, and twice as many half-size warps leave the queue more evenly:
-//   error seeds of 64 to 256 turns, 39,873 particles 132 -> 110 ms, 85,102
-//   particles 223 -> 167 ms, 15,978 the same.
+//  Uneven turn counts on such a ring: strict always; FMA up to 44 warps per SM.
+//   The last, longest particles run in few warps, and twice as many half-size
+//   warps leave the queue more evenly: error seeds of 64 to 256 turns, ms, 39,967
+//   particles 122 -> 99, 79,967 185 -> 148, 99,966 205 -> 189, but 119,968 219 ->
+//   222 and 159,879 295 -> 307; of 1,000 to 4,096 turns / 32, 1,145,971 particles
+//   1,013 -> 1,082 (strict 5,892 -> 5,887).
 //  Few ops without a two-lane form (wires, general apertures, dynamic kicks,
 //   orders above 15, elements without room in the cache): each is a segment that
 //   both lanes of a pair compute in full, twice the FP64 instructions of the one-
@@ -439,8 +441,8 @@ inline bool pair_pays(const PairLists &p, const PairUse &u) {
   const int per_wide = least_ops_per_wide(p, u, groups);
   if (wide && (!per_wide || p.n_ops < per_wide * wide)) return false;
   if (!u.fma && !p.general) return true;
-  if (p.general && (u.uneven || u.untuned_scan)) return true;
-  const int most = !p.general ? 9 : u.fma ? 14 : 12;
+  if (p.general && (u.untuned_scan || (u.uneven && !u.fma))) return true;
+  const int most = !p.general ? 9 : !u.fma ? 12 : u.uneven ? 44 : 14;
   return groups <= most * static_cast<int64_t>(u.sm_count);
 }
 // Time slices (Slices in pair.cuh) for a two-lane launch of equal turns with
