@@ -9,7 +9,12 @@ extern "C" {
 int pair_lists(const int32_t *ops, int n_ops, const double *table, int64_t stride, int n_seeds,
                int most_fields, int32_t *out, int64_t capacity, int64_t *info) {
   ufo::PairLists p;
-  info[0] = ufo::decode_pair(ops, n_ops, table, stride, n_seeds, most_fields, p);
+  std::vector<ufo::RowCheck> checks;
+  std::vector<unsigned char> bad;
+  std::vector<ufo::RowScan> scan = ufo::scan_first_row(ops, n_ops, table, checks);
+  ufo::check_rows(checks, table, stride, n_seeds, bad);
+  ufo::apply_checks(checks, bad, scan);
+  info[0] = ufo::decode_pair(ops, n_ops, table, scan, most_fields, p);
   info[1] = static_cast<int64_t>(p.ops.size());
   info[2] = static_cast<int64_t>(p.fma_at);
   info[3] = p.cache_fields;

@@ -154,3 +154,50 @@ def test_graphs_outlive_larger_launches_and_one_another():
     for graph in (True, False):
         b.launch(graph=graph)
         assert same(b.download(), want)
+
+
+@pytest.mark.parametrize('rows', [2, 3000])
+@pytest.mark.parametrize('what', ['strength', 'division', 'entry'])
+def test_one_row_apart_is_seen_in_small_and_large_tables(rows, what):
+    """Tables are looked through on the host or, when large, on the GPU: a last
+    row whose strengths, inner-drift divisions or thick constants stand apart from
+    the first row's changes the lists, at creation and with a new table."""
+    import types
+    import ufo_gb300 as u
+    from ufo_gb300 import capi, compiler as C
+    ctx = u.context(0)
+    q = u.Quadrupole('q', length=0.3, k1=1.1, slices=4)
+    s = u.Sextupole('s', length=0.2, k2=30.0, slices=4)
+    v = u.Quadrupole('v', length=0.3, k1=-1.1, slices=4)
+    line = u.Line('r', [u.Drift('d', length=0.5), q, u.Drift('e', length=0.4), s, v] * 20)
+    prog = C.compile_line(line, 0 if what == 'entry' else u.KICK, where=[])
+    table = np.repeat(prog.table, rows, axis=0)
+    apart = table.copy()
+    for op in prog.ops:
+        kind, off = int(op[0]), int(op[2])
+        if what == 'entry' and kind == C.OP_THICKQ:
+            apart[-1, off] *= 1.0 + 1e-3 * (off % 7)
+        if what != 'entry' and kind == C.OP_TEAPOT:
+            if what == 'strength':
+                apart[-1, off + 5] = 1e-300
+            else:  # [A, d, 1/d, A/d] of the inner drift
+                apart[-1, off + 2:off + 5] = 5.0, 1 / 5.0, apart[-1, off + 1] / 5.0
+    coords = beam(200)
+    seed = np.where(np.arange(200) % 2, rows - 1, 0).astype(np.int32)
+
+    def check(dp):
+        out = [capi.track(ctx, dp, coords, 3, capi.UFO_MODE_TRACK, f, seed=seed, slots=0)[1:]
+               for f in (0, capi.UFO_TRACK_PLAIN)]
+        assert same(*out)
+        return out[0][1]
+
+    def program(tab):
+        return capi.DeviceProgram(ctx, types.SimpleNamespace(ops=prog.ops, table=tab, n_dumps=0))
+    dp = program(table)
+    first = check(dp)
+    dp.set_table(apart)
+    second = check(dp)
+    assert np.isfinite(first).all() and not np.array_equal(first, second)
+    assert np.array_equal(check(program(apart)), second)
+    dp.set_table(table)
+    assert np.array_equal(check(dp), first)

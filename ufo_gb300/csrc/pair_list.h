@@ -11,6 +11,12 @@
 #include "../../include/ufo_gb300.h"
 #include "opcodes.h"
 
+#ifdef __CUDACC__
+#define UFO_HOST_DEV __host__ __device__ inline
+#else
+#define UFO_HOST_DEV inline
+#endif
+
 namespace ufo {
 
 // ---- opcode words of this kernel, built on the host (decode_pair)
@@ -82,29 +88,46 @@ inline int kick_pattern(int nn, int ns, int32_t mn) {
   return ns != 0 ? 0 : (nn == 2 && mn == 2) ? 1 : (nn == 3 && mn == 4) ? 2 : mn == 0 ? 3 : 0;
 }
 
-// What the two-lane lists need to know of every row's constants, gathered in one
-// pass over the table row by row (op by op, each look misses the cache: 20,000
-// rows of 833 ops took 170 ms more at every new table).
+// What the two-lane lists need to know of every row's constants.
 struct RowScan {
-  int strength = -1;     // where a short form's strength stands; -1: none
-  int division = -1;     // where an inner drift's [d, 1/d] stand; -1: none
   bool plain = true;     // strengths whose half and negative are exact, in every row
-  bool same = true;      // the division is row 0's in every row
+  bool same = true;      // an inner drift's division is row 0's in every row
   int twin = -1;         // an earlier op with the same cacheable constants in every row
 };
 
-inline bool plain_strength(double k) {
-  k = std::fabs(k);
+// What is to hold in every row for a part of an op's RowScan to stand.  The rows
+// are looked through by the host, or by the GPU once the table is there
+// (check_rows_kernel).
+struct RowCheck {
+  enum : int { PLAIN = 0, SAME, TWIN };
+  int kind, op;
+  int a, b, n;  // TWIN: n constants at a and at b; else the constant at a
+};
+
+UFO_HOST_DEV bool plain_strength(double k) {
+  k = fabs(k);
   return k == 0.0 || (k > 1e-280 && k < 1e280);
 }
 
-inline std::vector<RowScan> scan_rows(const int32_t *ops, int n_ops, const double *table, int64_t stride,
-                               int n_seeds) {
+UFO_HOST_DEV bool same_bits(double x, double y) {
+  union { double d; uint64_t u; } p{x}, q{y};
+  return p.u == q.u;
+}
+
+UFO_HOST_DEV bool check_row(const RowCheck &c, const double *row, const double *row0) {
+  if (c.kind == RowCheck::PLAIN) return plain_strength(row[c.a]);
+  if (c.kind == RowCheck::SAME) return row[c.a] == row0[c.a] && row[c.a + 1] == row0[c.a + 1];
+  bool same = true;
+  for (int k = 0; k < c.n; ++k) same = same && same_bits(row[c.a + k], row[c.b + k]);
+  return same;
+}
+
+// The scan as the first row has it, and what to check in the rows.
+inline std::vector<RowScan> scan_first_row(const int32_t *ops, int n_ops, const double *row0,
+                                           std::vector<RowCheck> &checks) {
   std::vector<RowScan> scan(static_cast<size_t>(n_ops));
-  std::vector<int> looked, twins;
-  std::unordered_multimap<uint64_t, int> seen;  // row 0's constants -> op
+  std::unordered_multimap<uint64_t, int> seen;  // constants -> op
   auto word = [&](int i) { return ops + static_cast<size_t>(i) * UFO_OP_WORDS; };
-  auto bytes = [&](int i) { return sizeof(double) * static_cast<size_t>(op_consts(word(i))); };
   for (int i = 0; i < n_ops; ++i) {
     const int32_t *w = word(i);
     RowScan &s = scan[static_cast<size_t>(i)];
@@ -113,16 +136,18 @@ inline std::vector<RowScan> scan_rows(const int32_t *ops, int n_ops, const doubl
       const bool teapot = w[0] == OP_TEAPOT;
       const bool div = teapot && w[3] > 1 && ((w[1] >> SH_FINNER) & 3) == DF_DIV;
       const int pattern = kick_pattern(w[teapot ? 4 : 3], w[teapot ? 5 : 4], w[teapot ? 6 : 5]);
-      if (pattern == 1 || pattern == 2)
-        s.strength = w[2] + (!teapot ? 0 : w[3] <= 1 ? 1 : div ? 5 : 2);
-      if (div) s.division = w[2] + 2;
-      if (s.strength >= 0 || s.division >= 0) looked.push_back(i);
+      if (pattern == 1 || pattern == 2) {  // a short form's strength
+        const int at = w[2] + (!teapot ? 0 : w[3] <= 1 ? 1 : div ? 5 : 2);
+        checks.push_back({RowCheck::PLAIN, i, at, 0, 1});
+      }
+      if (div) checks.push_back({RowCheck::SAME, i, w[2] + 2, 0, 2});  // [d, 1/d]
     } else if (w[0] == OP_THICKQ || w[0] == OP_THICKB ||
                (w[0] == OP_EDGE && (w[1] & F_RTPSI))) {
+      const int n = static_cast<int>(op_consts(w));
       uint64_t h = 1469598103934665603ull ^ static_cast<uint64_t>(w[0] * 31 + w[1]);
-      for (int64_t k = 0; k < op_consts(w); ++k) {
+      for (int k = 0; k < n; ++k) {
         uint64_t bits;
-        std::memcpy(&bits, table + w[2] + k, sizeof bits);
+        std::memcpy(&bits, row0 + w[2] + k, sizeof bits);
         h = (h ^ bits) * 1099511628211ull;
         h ^= h >> 29;
       }
@@ -130,37 +155,37 @@ inline std::vector<RowScan> scan_rows(const int32_t *ops, int n_ops, const doubl
       for (auto it = range.first; it != range.second && s.twin < 0; ++it) {
         const int32_t *v = word(it->second);
         if (v[0] == w[0] && v[1] == w[1] &&
-            std::memcmp(table + v[2], table + w[2], bytes(i)) == 0)
+            check_row({RowCheck::TWIN, i, v[2], w[2], n}, row0, row0))
           s.twin = it->second;
       }
       if (s.twin < 0)
         seen.emplace(h, i);
       else
-        twins.push_back(i);
-    }
-  }
-  for (int r = 0; r < n_seeds; ++r) {
-    const double *row = table + static_cast<int64_t>(r) * stride;
-    for (const int i : looked) {
-      RowScan &s = scan[static_cast<size_t>(i)];
-      if (s.strength >= 0) s.plain = s.plain && plain_strength(row[s.strength]);
-      if (s.division >= 0)
-        s.same = s.same && row[s.division] == table[s.division] &&
-                 row[s.division + 1] == table[s.division + 1];
-    }
-    for (size_t k = 0; r > 0 && k < twins.size();) {
-      const int i = twins[k];
-      RowScan &s = scan[static_cast<size_t>(i)];
-      if (std::memcmp(row + word(s.twin)[2], row + word(i)[2], bytes(i)) == 0) {
-        ++k;
-      } else {  // on its own from here
-        s.twin = -1;
-        twins[k] = twins.back();
-        twins.pop_back();
-      }
+        checks.push_back({RowCheck::TWIN, i, word(s.twin)[2], w[2], n});
     }
   }
   return scan;
+}
+
+// Row by row (check by check, each look misses the cache: 20,000 rows of 833 ops
+// took 170 ms more); `bad`: one byte per check, set where a row fails it.
+inline void check_rows(const std::vector<RowCheck> &checks, const double *table, int64_t stride,
+                       int n_seeds, std::vector<unsigned char> &bad) {
+  bad.assign(checks.size(), 0);
+  for (int r = 0; r < n_seeds; ++r)
+    for (size_t k = 0; k < checks.size(); ++k)
+      if (!bad[k]) bad[k] = !check_row(checks[k], table + static_cast<int64_t>(r) * stride, table);
+}
+
+inline void apply_checks(const std::vector<RowCheck> &checks,
+                         const std::vector<unsigned char> &bad, std::vector<RowScan> &scan) {
+  for (size_t k = 0; k < checks.size(); ++k) {
+    if (!bad[k]) continue;
+    RowScan &s = scan[static_cast<size_t>(checks[k].op)];
+    if (checks[k].kind == RowCheck::PLAIN) s.plain = false;
+    if (checks[k].kind == RowCheck::SAME) s.same = false;
+    if (checks[k].kind == RowCheck::TWIN) s.twin = -1;
+  }
 }
 
 struct PairLists {
@@ -185,7 +210,7 @@ inline size_t pair_fill_at(int n_ops) { return 2 * static_cast<size_t>(n_ops) + 
 // Thick elements and fringe edges with the same constants in every row share
 // their cache fields; at most `most_fields` are given out, and an element that
 // gets none goes through the one-lane code, in a segment of its own.
-inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
+inline bool decode_list(const int32_t *ops, int n_ops, const double *row0,
                         const std::vector<RowScan> &scan, int most_fields, bool fold_drifts,
                         PairLists &lists) {
   std::vector<PairOp> &out = lists.ops;
@@ -242,7 +267,7 @@ inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
         bool negative = false;
         if (div) {
           form = DIV_GENERAL;
-          const double *q = table + w[2] + 1;  // [A, d, 1/d, A/d]
+          const double *q = row0 + w[2] + 1;  // [A, d, 1/d, A/d]
           if (scan[static_cast<size_t>(i)].same) shift = shift_form(q[1], q[2], negative);
           if (shift) form = DIV_SHIFT;
         }
@@ -358,17 +383,16 @@ inline bool decode_list(const int32_t *ops, int n_ops, const double *table,
 // entries per op -- every op a segment of its own -- and the ends, and followed
 // by the ops that fill the cache (pair_fill walks those alone: one turn of three
 // particles through 1,600 ops 997 us with the whole list, 893 us).
-inline bool decode_pair(const int32_t *ops, int n_ops, const double *table, int64_t stride,
-                        int n_seeds, int most_fields, PairLists &lists) {
+inline bool decode_pair(const int32_t *ops, int n_ops, const double *row0,
+                        const std::vector<RowScan> &scan, int most_fields, PairLists &lists) {
   std::vector<PairOp> &out = lists.ops;
   out.clear();
   const size_t fill_at = pair_fill_at(n_ops);
   lists.n_ops = n_ops;
   lists.fma_at = fill_at + n_ops + 1;
-  const std::vector<RowScan> scan = scan_rows(ops, n_ops, table, stride, n_seeds);
   for (const bool strict : {true, false}) {
     const size_t start = out.size();
-    if (!decode_list(ops, n_ops, table, scan, most_fields, strict, lists)) return false;
+    if (!decode_list(ops, n_ops, row0, scan, most_fields, strict, lists)) return false;
     const size_t end = out.size();
     out.resize(start + fill_at);
     for (size_t i = start; i < end; ++i)

@@ -700,6 +700,17 @@ __global__ void __launch_bounds__(32) co_amoeba_kernel(TrackArgs a, const double
   for (int j = 0; j < 4; ++j) out[j] = sx[ilo][j];
 }
 
+// The checks of a table's rows (RowCheck), a block per row at a time: neighbouring
+// threads look at neighbouring constants, and the bytes are set, never cleared.
+// Bound by the table's one read.
+__global__ void __launch_bounds__(128)
+    check_rows_kernel(const double *table, int64_t stride, int n_seeds, const RowCheck *checks,
+                      int n_checks, unsigned char *bad) {
+  for (int r = blockIdx.x; r < n_seeds; r += gridDim.x)
+    for (int k = threadIdx.x; k < n_checks; k += blockDim.x)
+      if (!check_row(checks[k], table + r * stride, table)) bad[k] = 1;
+}
+
 // FP64 pipe peak probe: 8 independent DFMA chains per thread
 __global__ void __launch_bounds__(256) dfma_peak_kernel(double *out, int iters, double b, double c) {
   double a[8];
@@ -762,6 +773,7 @@ struct ufo_prog {
   int n_seeds;
   int n_dumps;
   bool full;  // needs the full interpreter (thick, wire, exact, ...)
+  unsigned char *check_buf;  // scan_table's, once a table was large enough
   std::vector<int32_t> host_ops;  // for validating replacement tables
   // two-lane kernel (pair.cuh): the lists on the device, null when there are none
   ufo::PairOp *pair_ops;
@@ -912,6 +924,42 @@ int validate_ops(const int32_t *ops, int n_ops, int64_t stride, int n_dumps,
     if (w[0] == ufo::OP_DYNKICK && table && !dynkick_ok(table + w[2], w[3] + w[4], w[5]))
       return fail(UFO_E_ARG, "op %d: malformed dynamic-kick programs", i);
   }
+  return UFO_OK;
+}
+
+// The lists' scan of a table that is on the device.  Many rows are looked through
+// there: on the host they cost a table of 20,000 rows x 1,928 constants as much
+// again as its upload.
+constexpr size_t DEVICE_CHECKS = 16384;  // rows x checks from which the GPU is quicker
+
+int scan_table(ufo_prog *prog, const double *table, std::vector<ufo::RowScan> &scan) {
+  std::vector<ufo::RowCheck> checks;
+  scan = ufo::scan_first_row(prog->host_ops.data(), prog->n_ops, table, checks);
+  std::vector<unsigned char> bad(checks.size(), 0);
+  // on the device: the checks (at most two per op), then a byte for each
+  const size_t cb = sizeof(ufo::RowCheck) * checks.size();
+  const size_t most = (sizeof(ufo::RowCheck) + 1) * 2 * static_cast<size_t>(prog->n_ops);
+  bool here = checks.size() * prog->n_seeds < DEVICE_CHECKS;
+  if (!here && !prog->check_buf && cudaMalloc(&prog->check_buf, most) != cudaSuccess) {
+    cudaGetLastError();
+    prog->check_buf = nullptr;
+    here = true;
+  }
+  if (here) {
+    ufo::check_rows(checks, table, prog->stride, prog->n_seeds, bad);
+  } else {
+    unsigned char *buf = prog->check_buf;
+    cudaStream_t st = prog->ctx->stream;
+    UFO_CUDA(cudaMemcpyAsync(buf, checks.data(), cb, cudaMemcpyHostToDevice, st));
+    UFO_CUDA(cudaMemsetAsync(buf + cb, 0, bad.size(), st));
+    ufo::check_rows_kernel<<<std::min(prog->n_seeds, 65535), 128, 0, st>>>(
+        prog->table, prog->stride, prog->n_seeds, reinterpret_cast<const ufo::RowCheck *>(buf),
+        static_cast<int>(checks.size()), buf + cb);
+    UFO_CUDA(cudaGetLastError());
+    UFO_CUDA(cudaMemcpyAsync(bad.data(), buf + cb, bad.size(), cudaMemcpyDeviceToHost, st));
+    UFO_CUDA(cudaStreamSynchronize(st));
+  }
+  ufo::apply_checks(checks, bad, scan);
   return UFO_OK;
 }
 
@@ -1401,38 +1449,43 @@ int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *t
   p->ops = nullptr;
   p->table = nullptr;
   p->pair_ops = nullptr;
+  p->check_buf = nullptr;
+  p->cache_fields = 0;
   p->cache = nullptr;
   p->cache_lanes = 0;
   p->cache_bytes = 0;
   p->graphs = std::make_shared<std::atomic<int>>(0);
   p->captured = false;
-  const bool pair = decode_pair(ops, n_ops, table, stride, n_seeds, INT_MAX, p->lists);
-  p->cache_fields = p->lists.cache_fields;
-  const size_t pb = sizeof(ufo::PairOp) * p->lists.ops.size();
   const size_t ob = sizeof(ufo::Op) * (n_ops > 0 ? n_ops : 1);
   const size_t tb = sizeof(double) * static_cast<size_t>(stride) * n_seeds;
-  if (cudaMalloc(&p->ops, ob) != cudaSuccess || cudaMalloc(&p->table, tb) != cudaSuccess ||
-      (pair && cudaMalloc(&p->pair_ops, pb) != cudaSuccess)) {
+  auto drop = [&](int code) {
     cudaFree(p->ops);
     cudaFree(p->table);
+    cudaFree(p->pair_ops);
+    cudaFree(p->check_buf);
     delete p;
-    return fail(UFO_E_NOMEM, "cudaMalloc(program %zu + %zu bytes)", ob, tb);
-  }
+    return code;
+  };
+  if (cudaMalloc(&p->ops, ob) != cudaSuccess || cudaMalloc(&p->table, tb) != cudaSuccess)
+    return drop(fail(UFO_E_NOMEM, "cudaMalloc(program %zu + %zu bytes)", ob, tb));
   cudaError_t e = cudaMemcpyAsync(p->ops, ops, sizeof(ufo::Op) * n_ops, cudaMemcpyHostToDevice,
                                   ctx->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(p->table, table, tb, cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess && pair)
+  if (e != cudaSuccess) return drop(cuda_fail(e, "program upload"));
+  std::vector<ufo::RowScan> scan;
+  rc = scan_table(p, table, scan);
+  if (rc) return drop(rc);
+  if (decode_pair(ops, n_ops, table, scan, INT_MAX, p->lists)) {
+    p->cache_fields = p->lists.cache_fields;
+    const size_t pb = sizeof(ufo::PairOp) * p->lists.ops.size();
+    if (cudaMalloc(&p->pair_ops, pb) != cudaSuccess)
+      return drop(fail(UFO_E_NOMEM, "cudaMalloc(two-lane lists of %zu bytes)", pb));
     e = cudaMemcpyAsync(p->pair_ops, p->lists.ops.data(), pb, cudaMemcpyHostToDevice,
                         ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  if (e != cudaSuccess) {
-    cudaFree(p->ops);
-    cudaFree(p->table);
-    cudaFree(p->pair_ops);
-    delete p;
-    return cuda_fail(e, "program upload");
   }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e != cudaSuccess) return drop(cuda_fail(e, "program upload"));
   *out = p;
   return UFO_OK;
 }
@@ -1440,21 +1493,25 @@ int ufo_prog_create(ufo_ctx *ctx, const int32_t *ops, int n_ops, const double *t
 int ufo_prog_set_table(ufo_prog *prog, const double *table, int n_seeds) {
   if (!prog || !table) return fail(UFO_E_ARG, "null argument");
   if (n_seeds != prog->n_seeds) return fail(UFO_E_ARG, "seed count changed");
-  const int rc = validate_rows(prog->host_ops.data(), prog->n_ops, prog->stride, prog->n_dumps,
-                               table, n_seeds);
+  int rc = validate_rows(prog->host_ops.data(), prog->n_ops, prog->stride, prog->n_dumps, table,
+                         n_seeds);
   if (rc) return rc;
   UFO_CUDA(cudaSetDevice(prog->ctx->device));
   const size_t tb = sizeof(double) * static_cast<size_t>(prog->stride) * n_seeds;
+  cudaStream_t st = prog->ctx->stream;
+  UFO_CUDA(cudaMemcpyAsync(prog->table, table, tb, cudaMemcpyHostToDevice, st));
   if (prog->pair_ops) {
     // new constants may share other cache fields or admit another division form
+    std::vector<ufo::RowScan> scan;
+    rc = scan_table(prog, table, scan);
+    if (rc) return rc;
     ufo::PairLists next;
-    decode_pair(prog->host_ops.data(), prog->n_ops, table, prog->stride, n_seeds,
+    decode_pair(prog->host_ops.data(), prog->n_ops, table, scan,
                 prog->cache_held() ? prog->cache_fields : INT_MAX, next);
     const size_t pb = sizeof(ufo::PairOp) * next.ops.size();
     if (std::memcmp(next.ops.data(), prog->lists.ops.data(), pb)) {
-      UFO_CUDA(cudaMemcpyAsync(prog->pair_ops, next.ops.data(), pb, cudaMemcpyHostToDevice,
-                               prog->ctx->stream));
-      UFO_CUDA(cudaStreamSynchronize(prog->ctx->stream));
+      UFO_CUDA(cudaMemcpyAsync(prog->pair_ops, next.ops.data(), pb, cudaMemcpyHostToDevice, st));
+      UFO_CUDA(cudaStreamSynchronize(st));
       if (next.cache_fields > prog->cache_fields) {  // allocated again by the next launch
         free_caches(prog);
         prog->cache_fields = next.cache_fields;
@@ -1462,8 +1519,7 @@ int ufo_prog_set_table(ufo_prog *prog, const double *table, int n_seeds) {
       std::swap(prog->lists, next);
     }
   }
-  UFO_CUDA(cudaMemcpyAsync(prog->table, table, tb, cudaMemcpyHostToDevice, prog->ctx->stream));
-  UFO_CUDA(cudaStreamSynchronize(prog->ctx->stream));
+  UFO_CUDA(cudaStreamSynchronize(st));
   return UFO_OK;
 }
 
@@ -1476,6 +1532,7 @@ void ufo_prog_destroy(ufo_prog *prog) {
   cudaFree(prog->ops);
   cudaFree(prog->table);
   cudaFree(prog->pair_ops);
+  cudaFree(prog->check_buf);
   free_caches(prog);
   delete prog;
 }
