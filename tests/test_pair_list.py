@@ -162,8 +162,9 @@ def test_ops_without_a_two_lane_form_bound_the_two_lane_kernel(host, general, fm
         assert all(a >= b for a, b in zip(most, most[1:]))
         assert 40 <= most[0] <= 81 and most[-1] <= 13
     assert use(host, 10 ** 6) and not use(host, 10 ** 6, fma=True)
-    for n in sizes:  # thick rings: up to a fifth at any size
-        assert use(host, n, 200, 40, thick=True) and not use(host, n, 200, 41, thick=True)
+    for n in sizes:  # thick rings: up to a quarter, then a fifth at any size
+        most = 50 if n <= 152 * 8 * 16 else 40
+        assert use(host, n, 200, most, thick=True) and not use(host, n, 200, most + 1, thick=True)
 
 
 def test_uneven_fused_launches_end_where_whole_warps_win(host):

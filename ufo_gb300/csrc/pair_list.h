@@ -441,8 +441,8 @@ inline bool decode_pair(const int32_t *ops, int n_ops, const double *row0,
 //   490 -> 434, 523 -> 492; but 25 %, 65,536 675 -> 1,034, 1,210 -> 1,929.  FMA 5 %,
 //   16,000 65 -> 49, 67 -> 58, 20,000 65 -> 73, 70 -> 84.  General magnets and
 //   thick elements, the longer part of their turn, bear more: errors on every
-//   magnet, FMA 17 %, 16,000 584 -> 511, 24,000 613 -> 761; thick ring 24 %, 16,000
-//   2,397 -> 1,856, 65,536 5,248 -> 4,900.
+//   magnet, FMA 17 %, 16,000 584 -> 511, 24,000 613 -> 761; thick ring 24 %, 1,000
+//   2,246 -> 1,558, 16,000 2,397 -> 1,856, 24,000 2,554 -> 2,641.
 struct PairUse {
   int64_t n;
   int sm_count;
@@ -451,10 +451,11 @@ struct PairUse {
 
 // the least ops per op without a two-lane form; 0: none may be
 inline int least_ops_per_wide(const PairLists &p, const PairUse &u, int64_t groups) {
-  if (p.thick) return 5;
-  if (p.general) return groups <= 8 * static_cast<int64_t>(u.sm_count) ? 5 : 32;
-  if (groups <= 5 * static_cast<int64_t>(u.sm_count)) return u.fma ? 8 : 6;
-  if (groups <= 8 * static_cast<int64_t>(u.sm_count)) return u.fma ? 12 : 10;
+  const int64_t sms = u.sm_count;
+  if (p.thick) return groups <= 8 * sms ? 4 : 5;
+  if (p.general) return groups <= 8 * sms ? 5 : 32;
+  if (groups <= 5 * sms) return u.fma ? 8 : 6;
+  if (groups <= 8 * sms) return u.fma ? 12 : 10;
   return u.fma ? 0 : 32;
 }
 
