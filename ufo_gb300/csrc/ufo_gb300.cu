@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(32) co_amoeba_kernel(TrackArgs a, const double
 
 // The checks of a table's rows (RowCheck), a block per row at a time: neighbouring
 // threads look at neighbouring constants, and the bytes are set, never cleared.
-// Bound by the table's one read.
+// Bound by the table's one read (20,000 rows x 1,928 constants, 308 MB, 109 us).
 __global__ void __launch_bounds__(128)
     check_rows_kernel(const double *table, int64_t stride, int n_seeds, const RowCheck *checks,
                       int n_checks, unsigned char *bad) {
