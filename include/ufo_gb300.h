@@ -172,7 +172,7 @@ int ufo_closed_orbit(ufo_ctx *ctx, const ufo_prog *prog, const double *start,
  * (ufo_gb300/batch.py: autotune).  The two-lane kernel, whose warps hold half the
  * particles, takes twice as many, at most 16.  Until it is called, and again
  * after ufo_ctx_reset_tuning, the library chooses: 16, and 8 two-lane warps for a
- * dynamic-aperture scan.  No reference counterpart. */
+ * larger dynamic-aperture scan.  No reference counterpart. */
 int ufo_ctx_set_tuning(ufo_ctx *ctx, int warps_per_sm);
 int ufo_ctx_reset_tuning(ufo_ctx *ctx);
 

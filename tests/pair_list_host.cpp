@@ -39,6 +39,10 @@ int pair_use(int n_ops, int wide, int thick, int general, int64_t n, int sm_coun
   return ufo::pair_pays(p, {n, sm_count, fma != 0, uneven != 0, scan != 0});
 }
 
+int pair_resident(int64_t n, int sm_count, int tuning, int scan) {
+  return ufo::pair_warps_per_sm(n, sm_count, tuning, scan != 0);
+}
+
 // groups, slices per group, turns per slice, warps per SM
 void pair_slices(int64_t n, int turns, int n_ops, int sm_count, int most_warps,
                  int64_t most_groups, int64_t *out) {

@@ -176,3 +176,14 @@ def test_uneven_fused_launches_end_where_whole_warps_win(host):
     assert not use(host, 1_145_971, general=True, fma=True, uneven=True)
     assert use(host, 1_145_971, general=True, uneven=True)
     assert use(host, 1_145_971, general=True, fma=True, scan=True)
+
+
+def test_scans_refill_from_a_queue_only_where_it_is_long(host):
+    """Untuned scans: all resident up to 10 warps per SM, then 8; tuned launches
+    and plain tracking get what they ask for, at most 16."""
+    def warps(n, tuning=16, scan=False):
+        return host.pair_resident(ctypes.c_int64(n), 152, tuning, int(scan))
+    full = 152 * 10 * 16
+    assert [warps(n, scan=True) for n in (1, full, full + 1, 10 ** 7)] == [16, 16, 8, 8]
+    for n in (1, full, 10 ** 7):
+        assert [warps(n, t) for t in (1, 3, 7, 8, 15, 16, 32)] == [2, 6, 14, 16, 16, 16, 16]

@@ -470,6 +470,23 @@ inline bool pair_pays(const PairLists &p, const PairUse &u) {
   const int most = !p.general ? 9 : !u.fma ? 12 : u.uneven ? 44 : 14;
   return groups <= most * static_cast<int64_t>(u.sm_count);
 }
+// Resident warps per SM of the two-lane kernel, 16 particles each: the tuning
+// counts warps of the one-lane kernel, so twice as many, at most the 16 that the
+// registers allow.  A dynamic-aperture scan that nobody tuned gets 8 when it has
+// more than 10 per SM: most of its particles are lost in the first turns, and
+// lanes that refill from a longer queue stay fuller, while two warps per sub-
+// partition still fill most of the FP64 pipe.  FODO ring with errors, strict, 24
+// turns (ms with 8, 16, and on the one-lane kernel): 21 % survive, 24,000
+// particles 30, 37, 47, 30,000 34, 54, 53, 49,152 35, 68, 72.  If nearly all
+// survive the queue is a second round, which up to 10 per SM would cost more than
+// the refill can gain: 20,000 53, 39, 47, 24,000 54, 41, 50, 30,000 62, 57, 58,
+// 36,864 63, 65, 65, 49,152 92, 87, 85.
+inline int pair_warps_per_sm(int64_t n, int sm_count, int tuning, bool untuned_scan) {
+  const int64_t groups = (n + 15) / 16;
+  return untuned_scan && groups > 10 * static_cast<int64_t>(sm_count) ? 8
+                                                                      : std::min(16, 2 * tuning);
+}
+
 // Time slices (Slices in pair.cuh) for a two-lane launch of equal turns with
 // more groups of 16 particles than 8 warps per SM: as many warps as fill every
 // sub-partition evenly (a multiple of 4 per SM) and leave groups in hand.  Below

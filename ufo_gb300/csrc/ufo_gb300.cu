@@ -988,19 +988,6 @@ unsigned long long spread_multiplier(int64_t n_particles) {
   return m;
 }
 
-// Resident warps per SM of the two-lane kernel, 16 particles each: the tuning
-// counts warps of the one-lane kernel, so twice as many, at most the 16 that the
-// registers allow.  A dynamic-aperture scan that nobody tuned gets 8: most of its
-// particles are lost in the first turns, and lanes that refill from a longer
-// queue stay fuller, while two warps per sub-partition still fill most of the
-// FP64 pipe (FODO ring with errors, 49,152 particles, ms with 16 and with 8: 128
-// turns FMA, 15 % survive 48.8 and 31.1, 31 % 60.5 and 34.4, 46 % 60.6 and 57.9,
-// 66 % 61.6 and 62.2; 32 turns strict, 17 % 71.7 and 45.2, 72 % 132 and 117;
-// 196,608 particles and 12,288 within 6 % either way).
-int pair_warps_per_sm(int mode, int warps_per_sm, bool tuned) {
-  return mode == UFO_MODE_SA && !tuned ? 8 : std::min(16, 2 * warps_per_sm);
-}
-
 int64_t pair_warps(int64_t n, int sm_count, int pair_per_sm) {
   return std::min<int64_t>((n + 15) / 16, static_cast<int64_t>(sm_count) * pair_per_sm);
 }
@@ -1210,7 +1197,8 @@ Route plan_route(const ufo_ctx *ctx, const ufo_prog *prog, ufo::TrackArgs &a,
   Route r;
   r.warps_per_sm = ctx->warps_per_sm;
   if (!use_pair(ctx, prog, a.n, a.mode, a.flags, a.pturns != nullptr)) return r;
-  const int whole = pair_warps_per_sm(a.mode, ctx->warps_per_sm, ctx->tuned);
+  const bool scan = a.mode == UFO_MODE_SA && !ctx->tuned;
+  const int whole = ufo::pair_warps_per_sm(a.n, ctx->sm_count, ctx->warps_per_sm, scan);
   int warps = whole;
   ufo::Slices slices = plan_slices(ctx, a, warps);
   if (prog->cache_fields) {
