@@ -29,14 +29,14 @@ int pair_lists(const int32_t *ops, int n_ops, const double *table, int64_t strid
 
 // Whether a launch of n particles of such lists takes the two-lane kernel.
 int pair_use(int n_ops, int wide, int thick, int general, int64_t n, int sm_count, int fma,
-             int uneven, int scan) {
+             int uneven, int scan, int64_t row_bytes) {
   ufo::PairLists p;
   p.n_ops = n_ops;
   p.wide[0] = p.wide[1] = wide;
   p.thick = thick != 0;
   p.general = general != 0;
   p.fma_ready = true;
-  return ufo::pair_pays(p, {n, sm_count, fma != 0, uneven != 0, scan != 0});
+  return ufo::pair_pays(p, {n, sm_count, fma != 0, uneven != 0, scan != 0, row_bytes});
 }
 
 int pair_resident(int64_t n, int sm_count, int tuning, int scan) {

@@ -143,9 +143,10 @@ def test_ops_without_constants_read_none(host):
             assert sum((h & 0xff) == PV_OBSERVE for h in lst[:, 0]) == (kind == OP_OBSERVE)
 
 
-def use(host, n, ops=200, wide=0, thick=False, general=False, fma=False, uneven=False, scan=False):
+def use(host, n, ops=200, wide=0, thick=False, general=False, fma=False, uneven=False, scan=False,
+        row=1000):
     return bool(host.pair_use(ops, wide, int(thick), int(general), ctypes.c_int64(n), 152, int(fma),
-                              int(uneven), int(scan)))
+                              int(uneven), int(scan), ctypes.c_int64(row)))
 
 
 @pytest.mark.parametrize('fma', [False, True])
@@ -187,3 +188,12 @@ def test_scans_refill_from_a_queue_only_where_it_is_long(host):
     assert [warps(n, scan=True) for n in (1, full, full + 1, 10 ** 7)] == [16, 16, 8, 8]
     for n in (1, full, 10 ** 7):
         assert [warps(n, t) for t in (1, 3, 7, 8, 15, 16, 32)] == [2, 6, 14, 16, 16, 16, 16]
+
+
+def test_fused_launches_of_general_magnets_end_where_their_rows_leave_l1(host):
+    for row, most in ((0, 13), (65_536, 13), (65_537, 11), (10 ** 9, 11)):
+        n = 152 * most * 16
+        assert use(host, n, general=True, fma=True, row=row)
+        assert not use(host, n + 1, general=True, fma=True, row=row)
+        assert use(host, 152 * 12 * 16, general=True, row=row)
+        assert not use(host, 152 * 12 * 16 + 1, general=True, row=row)

@@ -412,14 +412,19 @@ inline bool decode_pair(const int32_t *ops, int n_ops, const double *row0,
 //   1,355 -> 318, 65,536 particles 4,481 -> 1,765.
 //   A ring with general error kicks on most magnets (a coefficient enters one
 //   lane's sum, so half its products are idle) gains up to 12 warps per SM:
-//   light-source ring with errors 1,000 particles 15,590 -> 8,480, 30,000 even.
-//  FMA: up to 9 warps per SM, 14 where most kicks are general.  The sextupole
-//   form and the composed linear elements cost the two-lane code more
-//   instructions (6 for 5, 8 for 5 per 32 particles), so the one-lane kernel
-//   wins once its pipe is full: light-source ring 333 particles 652 -> 345,
-//   20,000 (8.2 warps per SM) 699 -> 615, 24,000 (9.9) 705 -> 770; ring with
-//   errors on every magnet 1,000 346 -> 192, 33,000 (13.6) 442 -> 439, 38,900
-//   (16) 477 -> 516.
+//   light-source ring with errors 1,000 particles 15,590 -> 8,480, 20,500 to
+//   24,000 18,770 -> 19,230 (a third warp on some sub-partitions), 29,184 20,240
+//   -> 19,310, 30,000 even.
+//  FMA: up to 9 warps per SM; where most kicks are general 13, or 11 if a row of
+//   constants passes 64 KB, which the two-lane kernel's warps, twice as many, read
+//   every turn.  The sextupole form and the composed linear elements cost the
+//   two-lane code more instructions (6 for 5, 8 for 5 per 32 particles), so the
+//   one-lane kernel wins once its pipe is full: light-source ring 333 particles
+//   652 -> 345, 20,000 (8.2 warps per SM) 699 -> 615, 21,888 755 -> 772, 24,000
+//   (9.9) 705 -> 770; FODO ring with errors on every magnet 1,000 346 -> 192,
+//   31,616 (13) 435 -> 412, 34,000 (14) 435 -> 443; light-source ring with errors
+//   (161 KB) 27,000 (11.1) 3,960 -> 3,740, 29,184 (12) 3,960 -> 4,250, 33,000
+//   4,240 -> 4,370.
 //  Dynamic-aperture scans of such a ring that nobody tuned: always.  Where few
 //  survive the refill of twice as many, half-size warps wins (196,608 particles,
 //  128 turns, ms: 15 % survive 87.5 -> 64.9); where most do it costs up to 5 %
@@ -447,6 +452,7 @@ struct PairUse {
   int64_t n;
   int sm_count;
   bool fma, uneven, untuned_scan;
+  int64_t row_bytes;  // constants of one seed
 };
 
 // the least ops per op without a two-lane form; 0: none may be
@@ -467,7 +473,7 @@ inline bool pair_pays(const PairLists &p, const PairUse &u) {
   if (wide && (!per_wide || p.n_ops < per_wide * wide)) return false;
   if (!u.fma && !p.general) return true;
   if (p.general && (u.untuned_scan || (u.uneven && !u.fma))) return true;
-  const int most = !p.general ? 9 : !u.fma ? 12 : u.uneven ? 44 : 14;
+  const int most = !p.general ? 9 : !u.fma ? 12 : u.uneven ? 44 : u.row_bytes <= 65536 ? 13 : 11;
   return groups <= most * static_cast<int64_t>(u.sm_count);
 }
 // Resident warps per SM of the two-lane kernel, 16 particles each: the tuning

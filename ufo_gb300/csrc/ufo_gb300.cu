@@ -1104,7 +1104,8 @@ bool use_pair(const ufo_ctx *ctx, const ufo_prog *prog, int64_t n, int mode, int
               bool uneven) {
   if (!prog->pair_ops || (flags & (UFO_TRACK_PLAIN | UFO_TRACK_COMPACT))) return false;
   const bool scan = mode == UFO_MODE_SA && !ctx->tuned;
-  return ufo::pair_pays(prog->lists, {n, ctx->sm_count, (flags & UFO_TRACK_FMA) != 0, uneven, scan});
+  return ufo::pair_pays(prog->lists, {n, ctx->sm_count, (flags & UFO_TRACK_FMA) != 0, uneven, scan,
+                                      prog->stride * static_cast<int64_t>(sizeof(double))});
 }
 
 constexpr size_t CACHE_MOST = size_t{4} << 30;
