@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(32, 16)
 // and the simplex goes through the same values.  A shrink (four more trials)
 // and an expansion of an unkept reflection (equal residuals) take a second turn.
 // Measured, 200 steps, whole calls: 12 orbits of the thick 768-element ring
-// 735 ms -> 74 ms.
+// 735 ms -> 67 ms.
 struct OrbitShared {
   double sx[4][5][4], y[4][5], psum[4][4];  // per orbit of the warp
 };
