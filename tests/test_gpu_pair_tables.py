@@ -201,3 +201,23 @@ def test_one_row_apart_is_seen_in_small_and_large_tables(rows, what):
     assert np.array_equal(check(program(apart)), second)
     dp.set_table(table)
     assert np.array_equal(check(dp), first)
+
+
+def test_a_cache_of_many_entries_grows_with_the_launches():
+    """A ring of magnets that share no entry: one entry set per magnet and lane, so
+    the cache starts small and grows with the launches, past what is kept."""
+    import ufo_gb300 as u
+    from ufo_gb300 import capi, compiler as C
+    ctx = u.context(0)
+    rng = np.random.default_rng(6)
+    cells = []
+    for i in range(120):
+        k = 1.0 + 0.01 * rng.standard_normal(2)
+        cells += [u.Quadrupole(f'f{i}', length=0.3, k1=k[0]), u.Drift(f'd{i}', length=0.5),
+                  u.Quadrupole(f'g{i}', length=0.3, k1=-k[1]), u.Drift(f'e{i}', length=0.5)]
+    dp = capi.DeviceProgram(ctx, C.compile_line(u.Line('r', cells), 0, where=[]))
+    for n in (40, 300, 2500, 20_000, 70_000, 100_000, 40):
+        c = beam(n, n)
+        out = [capi.track(ctx, dp, c, 2, capi.UFO_MODE_TRACK, f, slots=0)[1:]
+               for f in (0, capi.UFO_TRACK_PLAIN)]
+        assert np.isfinite(out[1][1]).all() and same(*out), n

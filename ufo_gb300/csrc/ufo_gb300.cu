@@ -15,7 +15,7 @@
 // lane granularity instead of work-item granularity.
 //
 // pair.cuh holds the two-lane kernel (a particle's planes on neighbouring lanes),
-// which strict launches and small ones take: use_pair has the rule and its
+// which strict launches and small ones take: pair_pays in pair_list.h has the rule and its
 // measurements.
 #include <cuda_runtime.h>
 
@@ -1136,20 +1136,22 @@ bool is_capturing(cudaStream_t stream) {
 // kernel.
 void ensure_cache(const ufo_prog *prog, int64_t lanes, cudaStream_t stream) {
   if (!prog->cache_fields || prog->cache_lanes >= lanes || is_capturing(stream)) return;
-  // lanes of the largest grid where that is cheap, so that it grows once
+  // lanes of the largest grid where that is cheap, so that it grows once, and
+  // twofold elsewhere
   const size_t per_lane = sizeof(double) * static_cast<size_t>(prog->cache_fields);
   const int64_t most = static_cast<int64_t>(prog->ctx->sm_count) * 16 * 32;
-  if (per_lane * most <= CACHE_MOST / 8) lanes = std::max(lanes, most);
+  const int64_t ahead =
+      per_lane * most <= CACHE_MOST / 8 ? most : std::min(most, 2 * prog->cache_lanes);
+  if (ahead > lanes && prog->cache_bytes + per_lane * ahead <= CACHE_MOST) lanes = ahead;
   const size_t bytes = per_lane * lanes;
   if (bytes > CACHE_MOST) return;
-  if (prog->cache_bytes + bytes > CACHE_MOST) {
-    if (prog->cache_held()) return;
-    free_caches(prog);
-  }
-  // a capture on another stream forbids this thread to allocate, unless it says
-  // that the allocation is none of the capture's
+  const bool full = prog->cache_bytes + bytes > CACHE_MOST;
+  if (full && prog->cache_held()) return;
+  // a capture on another stream forbids this thread to allocate or free, unless
+  // it says that the memory is none of the capture's
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cudaThreadExchangeStreamCaptureMode(&mode);
+  if (full) free_caches(prog);
   double *buf = nullptr;
   cudaError_t e = cudaMalloc(&buf, bytes);
   // zeros: lanes without a particle read finite coefficients
