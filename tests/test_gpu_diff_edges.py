@@ -70,3 +70,25 @@ def test_weak_focusing_leaves_the_vertical_plane_alone(tangent):
     out, _ = eng.forward(z0, np.ones(2), 2, tangent=tangent)
     assert np.array_equal(out[0, :2], out[1, :2]) and out[0, 2] == np.inf
     assert out[0, 3] == out[1, 3] == 2e-4
+
+
+@pytest.mark.parametrize('tangent', [False, True])
+def test_a_teapot_without_slices_is_its_outer_drift_both_ways(tangent):
+    import types
+    from ufo_gb300 import diff
+    D_TEAPOT = 2
+    prog = types.SimpleNamespace(
+        ops=np.array([[D_TEAPOT, 0, 0, 0, 1, -1, 0, 0]], np.int32),
+        tab=np.array([[0.5, 0.1, 0.0, 0.0, 0.0, 0.25, 0.0, 0.0]]), n_seeds=1, tab_stride=8,
+        kicks_per_turn=0, n_params=0)
+    eng = diff.DiffEngine(prog)
+    z0 = np.arange(12.0).reshape(3, 4)
+    out, state = eng.forward(z0, np.ones(3), 1, tangent=tangent)
+    want = z0.copy()
+    want[:, 0::2] += 0.5 * z0[:, 1::2]
+    assert np.array_equal(out[:, :4], want)
+    zbar = np.arange(12.0)[::-1].reshape(3, 4).copy()
+    got, _ = eng.reverse(state, zbar, np.zeros((3, 16)) if tangent else None)
+    want = zbar.copy()
+    want[:, 1::2] += 0.5 * zbar[:, 0::2]
+    assert np.array_equal(got, want)

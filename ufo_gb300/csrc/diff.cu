@@ -918,6 +918,7 @@ __device__ void turn_reverse_pair(Half &bh, const DiffArgs &a, const double *T0,
           rev_part_pair<4>(bh, a, c, tp, left == N, left == 4, even, j, write, tt, pm, kidx, tape, g0);
         for (; left >= 1; --left)
           rev_part_pair<1>(bh, a, c, tp, left == N, left == 1, even, j, write, tt, pm, kidx, tape, g0);
+        if (tp && N < 1) bh.pu = fma(bh.u, __ldg(c), bh.pu);  // the outer drift alone
         if (pp) *pp = fma(g0 * oo, __ldg(c + 3), p0);
         break;
       }
